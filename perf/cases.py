@@ -3,7 +3,8 @@
 `listed()` names the cases, `draw(rng)` gives further ones of the same ranges, `prepare(case, seed)` makes what a
 program holds before the call, `run(state)` is one pass through the public operators (luxlib_b200) and returns the
 outputs whole, `work(case)` counts the bytes and operations that no implementation can do without, `tolerance(case)`
-says how far another correct implementation of the same precision may be off.
+says how far another correct implementation of the same precision may be off, `exact(case, seed)` is what `run` returns
+in 64-bit arithmetic.
 
 Six kinds of work:
   mlp        two dense layers and the mean-squared error, forward + pullback (small, latency counts)
@@ -375,3 +376,105 @@ def tolerance(case):
         # a pre-activation within rounding of zero may fall on the other side of relu: its cotangent comes or goes whole
         return {"rel": 6e-4, "max": 0.2}
     return {"rel": 1e-5}
+
+
+# ---------------------------------------------------------------------------------------------
+# exact: the same results from plain torch in 64 bits
+# ---------------------------------------------------------------------------------------------
+def _f64(t):
+    """A double copy in row-major memory with the axes reversed: Julia's (W, H, C, N) is torch's (N, C, H, W)."""
+    return t.permute(*reversed(range(t.dim()))).double().contiguous()
+
+
+def _jl(t):
+    t = t.detach()
+    return t.permute(*reversed(range(t.dim()))) if t.dim() > 1 else t
+
+
+_ACT64 = {"identity": lambda t: t, "relu": torch.relu, "tanh": torch.tanh, "sigmoid": torch.sigmoid,
+          "swish": torch.nn.functional.silu, "gelu": lambda t: torch.nn.functional.gelu(t, approximate="tanh")}
+
+
+def _conv64(w, x, dims):
+    """NNlib's convolution flips the filter; torch's does not."""
+    return torch.nn.functional.conv2d(x, w.flip(2, 3), stride=dims.stride, padding=(dims.padding[0], dims.padding[2]))
+
+
+def _norm64(x, mean, var, scale, bias):
+    shape = (1, -1) + (1,) * (x.dim() - 2)
+    return (x - mean) / torch.sqrt(var + 1e-5) * scale.view(shape) + bias.view(shape)
+
+
+def _batch64(x, bn):
+    """Training-mode BatchNorm and its updated running statistics."""
+    over = [0] + list(range(2, x.dim()))
+    n = x.numel() // x.shape[1]
+    mean, var = x.mean(over, keepdim=True), x.var(over, unbiased=False, keepdim=True)
+    y = _norm64(x, mean, var, bn["scale"], bn["bias"])
+    return y, 0.9 * bn["mean"] + 0.1 * mean.flatten(), 0.9 * bn["var"] + 0.1 * var.flatten() * n / (n - 1)
+
+
+def _classify64(st):
+    def layer(act, l, h):
+        bn = {k: v.double() for k, v in l["bn"].items()}
+        shape = (1, -1, 1, 1)
+        return act(_norm64(_conv64(_f64(l["w"]), h, l["dims"]), bn["mean"].view(shape), bn["var"].view(shape), bn["scale"], bn["bias"]))
+
+    same = _ACT64["identity"]
+    h = torch.nn.functional.max_pool2d(layer(torch.relu, st["stem"], _f64(st["x"])), 3, 2, 1)
+    for blk in st["blocks"]:
+        a = layer(torch.relu, blk["b"], layer(torch.relu, blk["a"], h))
+        h = torch.relu(a + (h if blk["skip"] is None else layer(same, blk["skip"], h)))
+    return h.mean((2, 3)) @ _f64(st["Wd"]) + st["bd"].double()
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "resnet18" and case["mode"] == "train":
+        return None                # 62 layers of gradients in 64 bits take too long
+    st = prepare(case, seed)
+    if kind == "resnet18":
+        with torch.no_grad():
+            return _jl(_classify64(st))
+    grad = lambda t: _f64(t).requires_grad_()  # noqa: E731
+    if kind == "mlp":
+        W1, b1, W2, b2, x = (grad(st[k]) for k in ("W1", "b1", "W2", "b2", "x"))
+        y = torch.relu(x @ W1 + b1) @ W2 + b2
+        loss = (y - _f64(st["target"])).square().mean()
+        return [loss.detach().reshape(1)] + [_jl(g) for g in torch.autograd.grad(loss, (W1, b1, W2, b2, x))]
+    if kind == "dense":
+        W, x, b = (grad(st[k]) for k in ("W", "x", "b"))
+        y = _ACT64[case["act"]](x @ W + b)
+        if case["mode"] == "infer":
+            return _jl(y)
+        return [_jl(y)] + [_jl(g) for g in torch.autograd.grad(y, (W, x, b), _f64(st["dy"]))]
+    if kind == "conv_bn" or (kind == "norm" and case["op"] == "batchnorm"):
+        src = st["bn"] if kind == "conv_bn" else st
+        bn = {k: src[k].double() for k in ("scale", "bias", "mean", "var")}
+        bn["scale"].requires_grad_(), bn["bias"].requires_grad_()
+        x = grad(st["x"])
+        inputs = [x, bn["scale"], bn["bias"]]
+        if kind == "conv_bn":
+            w = grad(st["w"])
+            inputs.insert(0, w)
+            y, mean, var = _batch64(_conv64(w, x, st["dims"]), bn)
+            y = torch.relu(y)
+        else:
+            y, mean, var = _batch64(x, bn)
+        return [_jl(y), mean.detach(), var.detach()] + [_jl(g) for g in torch.autograd.grad(y, inputs, _f64(st["dy"]))]
+    if kind == "norm":
+        x, scale, bias = grad(st["x"]), st["scale"].double().requires_grad_(), st["bias"].double().requires_grad_()
+        if case["op"] == "layernorm":
+            y = torch.nn.functional.layer_norm(x, x.shape[1:], scale, bias, 1e-5)
+        else:
+            y = torch.nn.functional.group_norm(x, case["groups"], scale, bias, 1e-5)
+        return [_jl(y)] + [_jl(g) for g in torch.autograd.grad(y, (x, scale, bias), _f64(st["dy"]))]
+    q, k, v = (grad(st[n]) for n in "qkv")                       # (batch, tokens, heads, features)
+    rep = case["H"] // case["Hkv"]
+    k2, v2 = (t.repeat_interleave(rep, 2) for t in (k, v))
+    logits = torch.einsum("bshd,blhd->bhls", k2, q) / math.sqrt(case["D"])
+    if case["causal"]:
+        logits = logits.masked_fill(torch.ones(case["L"], case["S"], device="cuda").triu(1).bool(), -math.inf)
+    w = torch.softmax(logits, -1)
+    y = torch.einsum("bshd,bhls->blhd", v2, w)
+    return [_jl(y), _jl(w)] + [_jl(g) for g in torch.autograd.grad(y, (q, k, v), _f64(st["dx"]))]
