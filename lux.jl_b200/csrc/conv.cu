@@ -37,11 +37,16 @@ int32_t make_geom(const lb2_conv_desc* d, ConvGeom* g) {
 }
 
 // Which kernels serve a geometry: 1 = tensor-core path on the WHCN bytes (conv_tc*.cu), 2 = general bf16 tensor-core
-// path on channel-innermost copies (conv_cw.cu), 0 = CUDA-core direct kernels.
+// path on channel-innermost copies (conv_cw.cu), 3 = the same for Float32 (conv_cw_f32.cu), 0 = CUDA-core direct kernels.
 int conv_route(const ConvGeom& g, int32_t dtype) {
   if (conv_tc_supported(g, dtype)) return 1;
   if (conv_cw_supported(g, dtype)) return 2;
+  if (dtype == LB2_F32 && conv_cwf_supported(g)) return 3;
   return 0;
+}
+size_t route_fwd_bytes(int route, const ConvGeom& g, int32_t dtype) {
+  return route == 1 ? conv_tc_fwd_workspace_bytes(g, dtype) : route == 2 ? conv_cw_fwd_workspace_bytes(g)
+       : route == 3 ? conv_cwf_fwd_workspace_bytes(g) : 0;
 }
 
 int64_t y_numel(const ConvGeom& g) { return (int64_t)g.out[0] * g.out[1] * g.out[2] * g.cout * g.batch; }
@@ -58,7 +63,8 @@ ConvBwdLayout conv_bwd_layout(const ConvGeom& g, int32_t dtype, int32_t act) {
   l.g_bytes = act == LB2_ACT_IDENTITY ? 0 : align_up((size_t)n * dtype_size(dtype), 1024);
   l.red_bytes = align_up(act_bwd_workspace_bytes(y_spatial(g), g.cout, g.batch), 1024);
   const int route = conv_route(g, dtype);
-  l.tc_bytes = route == 1 ? conv_tc_bwd_workspace_bytes(g, dtype) : (route == 2 ? conv_cw_bwd_workspace_bytes(g) : 0);
+  l.tc_bytes = route == 1 ? conv_tc_bwd_workspace_bytes(g, dtype) : route == 2 ? conv_cw_bwd_workspace_bytes(g)
+             : route == 3 ? conv_cwf_bwd_workspace_bytes(g) : 0;
   return l;
 }
 
@@ -78,8 +84,7 @@ int32_t lb2_conv_output_size(const lb2_conv_desc* d, int32_t* out) {
 size_t lb2_conv_fwd_workspace_bytes(const lb2_conv_desc* d, int32_t dtype) {
   ConvGeom g;
   if (!valid_dtype(dtype) || make_geom(d, &g) != LB2_OK || y_numel(g) == 0) return 0;
-  const int route = conv_route(g, dtype);
-  return route == 1 ? conv_tc_fwd_workspace_bytes(g, dtype) : (route == 2 ? conv_cw_fwd_workspace_bytes(g) : 0);
+  return route_fwd_bytes(conv_route(g, dtype), g, dtype);
 }
 
 int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const void* b, const lb2_conv_desc* d,
@@ -102,10 +107,11 @@ int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const 
   if (route == 1 && !(aligned_to(x, 16) && aligned_to(y, 16) && aligned_to(preact, 16)))
     route = (conv_cw_supported(g, dtype) && conv_cw_fwd_workspace_bytes(g) <= workspace_bytes) ? 2 : 0;
   if (route != 0) {
-    const size_t need = route == 1 ? conv_tc_fwd_workspace_bytes(g, dtype) : conv_cw_fwd_workspace_bytes(g);
+    const size_t need = route_fwd_bytes(route, g, dtype);
     LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", need);
     LB2_REQUIRE(aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");
     if (route == 1) return conv_tc_fwd(y, preact, x, w, b, g, dtype, act, workspace, static_cast<cudaStream_t>(stream));
+    if (route == 3) return conv_cwf_fwd(y, preact, x, w, b, g, act, workspace, static_cast<cudaStream_t>(stream));
     return conv_cw_fwd(y, preact, x, w, b, g, act, workspace, static_cast<cudaStream_t>(stream));
   }
   return conv_fwd_direct(y, preact, x, w, b, g, dtype, act, static_cast<cudaStream_t>(stream));
@@ -114,7 +120,7 @@ int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const 
 int32_t lb2_conv_fwd_leaves_x_copy(const lb2_conv_desc* d, int32_t dtype) {
   ConvGeom g;
   if (!valid_dtype(dtype) || make_geom(d, &g) != LB2_OK || y_numel(g) == 0) return 0;
-  return conv_route(g, dtype) == 2 ? 1 : 0;
+  return conv_route(g, dtype) >= 2 ? 1 : 0;
 }
 
 // The epilogue sums cost about a thousand instructions per warp and tile; they disappear behind the tile's MMAs only
@@ -214,10 +220,11 @@ int32_t lb2_conv_bwd(void* dw, void* dx, void* db, const void* dy, const void* o
     if (rc != LB2_OK) return rc;
   }
   const bool x_is_copy = (flags & LB2_FLAG_X_COPY_GIVEN) != 0;
-  LB2_REQUIRE(!x_is_copy || (route == 2 && aligned_to(x, 256)), LB2_BAD_ARG,
+  LB2_REQUIRE(!x_is_copy || (route >= 2 && aligned_to(x, 256)), LB2_BAD_ARG,
               "LB2_FLAG_X_COPY_GIVEN: this geometry does not run on the path that leaves a copy of x (or the pointer is not a workspace start)");
   void* tc_ws = ws + lay.g_bytes + lay.red_bytes;
   if (route == 2) return conv_cw_bwd(dw, (dx && nx > 0) ? dx : nullptr, x, gptr, w, g, tc_ws, st, x_is_copy);
+  if (route == 3) return conv_cwf_bwd(dw, (dx && nx > 0) ? dx : nullptr, x, gptr, w, g, tc_ws, st, x_is_copy);
   // TMA needs 16-byte aligned bases for everything it loads (g, x) or stores (dx); other views go to the direct kernels
   const bool tc = route == 1 && aligned_to(gptr, 16) && aligned_to(x, 16) && aligned_to(dx, 16);
   if (tc && dtype == LB2_F32) {   // both gradients share one set of shifted copies of g

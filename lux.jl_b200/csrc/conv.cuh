@@ -41,6 +41,32 @@ int32_t conv_cw_fwd(void* y, void* preact, const void* x, const void* w, const v
 int32_t conv_cw_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws,
                     cudaStream_t st, bool x_is_copy = false);
 
+// General Float32 tensor-core path on channel-innermost hi/lo copies (conv_cw_f32.cu), same geometries.
+bool conv_cwf_supported(const ConvGeom& g);
+size_t conv_cwf_fwd_workspace_bytes(const ConvGeom& g);
+size_t conv_cwf_bwd_workspace_bytes(const ConvGeom& g);
+int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const void* bias, const ConvGeom& g, int32_t act,
+                     void* ws, cudaStream_t st);
+int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws,
+                     cudaStream_t st, bool x_is_copy = false);
+
+// Box of at most `most` positions (BW columns x BH rows x BI images) that covers an OW x OH x NI grid in the fewest boxes;
+// among equals the widest (contiguous stores). Rows are cut into equal pieces of at least 8 columns.
+inline void conv_position_box(int OW, int OH, int NI, int most, int* BW, int* BH, int* BI) {
+  int64_t best = 0;
+  for (int k = 1; k <= OW; ++k) {
+    const int bw = (OW + k - 1) / k;
+    if (bw > most) continue;
+    if (best != 0 && bw < 8) break;
+    const int rows = most / bw;
+    for (int bh = rows < OH ? rows : OH; bh >= 1; --bh) {
+      const int bi = rows / bh < NI ? rows / bh : NI;
+      const int64_t n = (int64_t)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((NI + bi - 1) / bi);
+      if (best == 0 || n < best) { best = n; *BW = bw; *BH = bh; *BI = bi; }
+    }
+  }
+}
+
 bool conv_tc_f32_supported(const ConvGeom& g);
 size_t conv_tc_f32_fwd_workspace_bytes(const ConvGeom& g);
 size_t conv_tc_f32_bwd_workspace_bytes(const ConvGeom& g);

@@ -1064,3 +1064,48 @@ def test_conv_fwd_sums_entry_point_on_every_route(dt, case):
     parity_report.record("sum y", dt, err1, 1e-5, judged="against the sum of magnitudes when the sum cancels")
     assert err2 <= 1e-5 and err1 <= 1e-5, (err1, err2)
     del y_st
+
+
+F32_GENERAL_CONV_CASES = [
+    # spatial, k, cin, cout, stride, pad, dilation, flip, batch — edges of the Float32 channel-innermost path
+    ((15, 13), (3, 3), 33, 65, 1, 1, 1, False, 3),             # one channel past a chunk / a column tile
+    ((10, 6), (3, 3), 31, 129, (2, 1), 1, 1, True, 2),         # two 128-wide column tiles
+    ((7, 7), (3, 3), 512, 96, 1, 1, 1, False, 1),              # few tiles: split along the contraction
+    ((13, 11), (1, 1), 96, 40, 3, 0, 1, False, 4),             # split data gradient with classes no tap reaches
+    ((14, 14), (5, 5), 256, 32, 1, 2, 1, False, 1),            # 200 k-blocks
+    ((21, 17), (8, 3), 4, 24, 2, (4, 3, 1, 1), 1, False, 2),   # kW * cin = 32: taps folded into one chunk
+    ((21, 17), (3, 3), 11, 24, 2, 1, 2, False, 2),             # kW * cin = 33: not folded; dilation with stride
+    ((130, 3), (3, 3), 8, 16, 1, (0, 2, 1, 0), 1, False, 2),   # rows longer than a tile
+    ((1, 1), (1, 1), 5, 3, 1, 0, 1, False, 1),
+    ((26, 30), (7, 7), 3, 64, 2, 3, 1, False, 9),
+]
+
+
+@pytest.mark.parametrize("act", ["identity", "gelu"])
+@pytest.mark.parametrize("offset", [0, 1])                     # 1: bases that are aligned to the element only
+@pytest.mark.parametrize("case", F32_GENERAL_CONV_CASES)
+def test_fused_conv_f32_general_path(case, offset, act):
+    # 2e-6: three tf32 products drop lo * lo (2^-22 of a product), k-blocks are added in fp32 (at most 400 of them,
+    # random signs); ten times under the contract's 1e-5 for the direct kernels' sequential sums
+    sp, k, cin, cout, stride, pad, dil, flip, batch = case
+    rng = np.random.default_rng(61)
+    x = rng.standard_normal(sp + (cin, batch)).astype(np.float32)
+    w = O.kaiming_normal(rng, k + (cin, cout)).astype(np.float32)
+    b = rng.uniform(-0.1, 0.1, cout).astype(np.float32)
+
+    def place(a):
+        t = dev(a, "f32")
+        if not offset:
+            return t
+        buf = torch.empty(t.numel() + 1, device="cuda")
+        out = torch.as_strided(buf, t.shape, t.stride(), 1)
+        out.copy_(t)
+        return out
+    ocd = O.ConvDims.make(2, stride, pad, dil, 1, flip)
+    y_ref, pb_ref = O.fused_conv_rrule(act, w.astype(np.float64), x.astype(np.float64), b.astype(np.float64), ocd)
+    y, pb = L.rrule_fused_conv(act, place(w), place(x), place(b), L.ConvDims.make(2, stride, pad, dil, 1, flip))
+    check(y, y_ref, "f32", "y", tol=2e-6)
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    for name, got, want in zip(("dw", "dx", "db"), pb(place(delta)), pb_ref(delta.astype(np.float64))):
+        check(got, want, "f32", name, tol=2e-6)
+    assert L._cabi.load().lb2_poll_device_status(None) == 0
