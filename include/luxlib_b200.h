@@ -313,6 +313,26 @@ LB2_API int32_t lb2_attention_softmax_fwd(void* y, const void* logits, const voi
 LB2_API int32_t lb2_attention_softmax_bwd(void* dlogits, void* dbias, const void* dy, const void* y, double scale,
                                           int64_t S, int64_t L, int64_t HB, int32_t dtype, void* stream);
 
+/* scaled_dot_product_attention (lib/LuxLib/src/impl/attention.jl:5-131) and its pullback over all heads and samples at once,
+ * on the tensor cores: q (head_dim, heads, queries, batch), k (head_dim, kv_heads, keys, batch), v (value_dim, kv_heads,
+ * keys, batch) -> x (value_dim, heads, queries, batch), w (keys, queries, heads, batch). Consecutive heads / kv_heads query
+ * heads share a key head. bias, mask, causal, scale as in lb2_attention_softmax_fwd. lb2_attention_is_fused: 1 when the
+ * extents are served (positive, head_dim and value_dim rows a multiple of 16 bytes); arrays must be 16-byte aligned.
+ * Backward: dbias (keys, queries, heads, batch) may be NULL. */
+typedef struct lb2_attention_dims {
+  int64_t head_dim, value_dim, heads, kv_heads, queries, keys, batch;
+} lb2_attention_dims;
+LB2_API int32_t lb2_attention_is_fused(const lb2_attention_dims* dims, int32_t dtype);
+LB2_API size_t lb2_attention_fwd_workspace_bytes(const lb2_attention_dims* dims, int32_t dtype);
+LB2_API int32_t lb2_attention_fwd(void* x, void* w, const void* q, const void* k, const void* v, const void* bias,
+                                  int64_t bias_batch_stride, const uint8_t* mask, int64_t mask_batch_stride, int32_t causal,
+                                  double scale, const lb2_attention_dims* dims, int32_t dtype, void* workspace,
+                                  size_t workspace_bytes, void* stream);
+LB2_API size_t lb2_attention_bwd_workspace_bytes(const lb2_attention_dims* dims, int32_t dtype);
+LB2_API int32_t lb2_attention_bwd(void* dq, void* dk, void* dv, void* dbias, const void* dx, const void* w, const void* q,
+                                  const void* k, const void* v, int32_t causal, double scale, const lb2_attention_dims* dims,
+                                  int32_t dtype, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- Scale layer ------------------------------------------------------------------------------- */
 /* y = act.(x .* weight .+ bias) (src/layers/basic.jl:452-461; the {False} method has no bias: bias = NULL) with
  * weight / bias of the layer's dims and x of shape (dims..., batch...): a (D, B) column-major view, D = prod(dims).

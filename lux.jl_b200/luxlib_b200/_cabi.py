@@ -41,6 +41,12 @@ class PoolDesc(C.Structure):
 POOL_MAX, POOL_MEAN = 0, 1
 
 
+class AttentionDims(C.Structure):
+    """lb2_attention_dims"""
+    _fields_ = [(n, C.c_int64) for n in ("head_dim", "value_dim", "heads", "kv_heads", "queries", "keys", "batch")]
+
+
+
 class OptLeaf(C.Structure):
     """lb2_opt_leaf"""
     _fields_ = [("param", C.c_void_p), ("grad", C.c_void_p), ("state1", C.c_void_p), ("state2", C.c_void_p),
@@ -96,6 +102,11 @@ PROTOTYPES = {
                                   C.c_uint32, _p, _sz, _p]),
     "lb2_attention_softmax_fwd": (_i32, [_p, _p, _p, _i64, _p, _i64, _i32, C.c_double, _i64, _i64, _i64, _i32, _p]),
     "lb2_attention_softmax_bwd": (_i32, [_p, _p, _p, _p, C.c_double, _i64, _i64, _i64, _i32, _p]),
+    "lb2_attention_is_fused": (_i32, [C.POINTER(AttentionDims), _i32]),
+    "lb2_attention_fwd_workspace_bytes": (_sz, [C.POINTER(AttentionDims), _i32]),
+    "lb2_attention_fwd": (_i32, [_p, _p, _p, _p, _p, _p, _i64, _p, _i64, _i32, _dbl, C.POINTER(AttentionDims), _i32, _p, _sz, _p]),
+    "lb2_attention_bwd_workspace_bytes": (_sz, [C.POINTER(AttentionDims), _i32]),
+    "lb2_attention_bwd": (_i32, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _i32, _dbl, C.POINTER(AttentionDims), _i32, _p, _sz, _p]),
     "lb2_conv_fwd_sums_is_fused": (_i32, [_p, _i32]),
     "lb2_conv_fwd_sums_workspace_bytes": (_sz, [_p, _i32]),
     "lb2_conv_fwd_sums": (_i32, [_p, _fp, _p, _p, _p, _i32, C.c_uint32, _p, _sz, _p]),

@@ -601,6 +601,48 @@ def rrule_batched_matmul(x, y, *, flags: int = 0):
     return z, pullback
 
 
+def _attention_fwd_by_product(lib, out, w, Q, Kx, V, bias_c, bias_bs, mask_c, mask_bs, causal, sc, dims, dt, flags):
+    """Attention forward as one batched product per (sample, key head): any extents, any alignment."""
+    D, E, H, Hkv, Lq, S, Bn = (getattr(dims, f[0]) for f in dims._fields_)
+    gs, es, device = H // Hkv, Q.element_size(), Q.device
+    logits = torch.empty_like(w)
+    for b in range(Bn):      # logits[:, :, h, b] = k[:, g, :, b]' * q[:, h, :, b] for the gs heads h of group g: k repeated
+        for g in range(Hkv):
+            _bmm(lib, logits.data_ptr() + ((g * gs + H * b) * S * Lq) * es, Kx.data_ptr() + (g * D + b * D * Hkv * S) * es,
+                 Q.data_ptr() + (g * gs * D + b * D * H * Lq) * es, S, Lq, D, gs, D * Hkv, D * H, S, 0, D, S * Lq, 1, 0, dt, device, flags=flags)
+    _cabi.check(lib.lb2_attention_softmax_fwd(ptr(w), ptr(logits), ptr(bias_c), bias_bs, ptr(mask_c), mask_bs, causal, sc, S, Lq, H * Bn, dt,
+                                              current_stream(device)))
+    for b in range(Bn):      # x[:, h, :, b] = v[:, g, :, b] * w[:, :, h, b]
+        for g in range(Hkv):
+            _bmm(lib, out.data_ptr() + (g * gs * E + b * E * H * Lq) * es, V.data_ptr() + (g * E + b * E * Hkv * S) * es,
+                 w.data_ptr() + ((g * gs + H * b) * S * Lq) * es, E, Lq, S, gs, E * Hkv, S, E * H, 0, S * Lq, E, 0, 0, dt, device, flags=flags)
+
+
+def _attention_bwd_by_product(lib, dq, dk, dv, db, G, w, Q, Kx, V, sc, dims, dt, flags):
+    """The pullback in the same form; the heads of a group add into the same dk / dv one after the other, in order."""
+    D, E, H, Hkv, Lq, S, Bn = (getattr(dims, f[0]) for f in dims._fields_)
+    gs, es, device = H // Hkv, Q.element_size(), Q.device
+    dw, dl = torch.empty_like(w), torch.empty_like(w)
+    for b in range(Bn):      # dw[:, :, h, b] = v[:, g, :, b]' * dx[:, h, :, b]
+        for g in range(Hkv):
+            _bmm(lib, dw.data_ptr() + ((g * gs + H * b) * S * Lq) * es, V.data_ptr() + (g * E + b * E * Hkv * S) * es,
+                 G.data_ptr() + (g * gs * E + b * E * H * Lq) * es, S, Lq, E, gs, E * Hkv, E * H, S, 0, E, S * Lq, 1, 0, dt, device, flags=flags)
+    _cabi.check(lib.lb2_attention_softmax_bwd(ptr(dl), ptr(db), ptr(dw), ptr(w), sc, S, Lq, H * Bn, dt, current_stream(device)))
+    for b in range(Bn):
+        # dq[:, h, :, b] = k[:, g, :, b] * dl[:, :, h, b]; dv[:, g, :, b] += dx[:, h, :, b] * w[:, :, h, b]'; dk likewise
+        for g in range(Hkv):
+            _bmm(lib, dq.data_ptr() + (g * gs * D + b * D * H * Lq) * es, Kx.data_ptr() + (g * D + b * D * Hkv * S) * es,
+                 dl.data_ptr() + ((g * gs + H * b) * S * Lq) * es, D, Lq, S, gs, D * Hkv, S, D * H, 0, S * Lq, D, 0, 0, dt, device, flags=flags)
+            for j in range(gs):
+                h = g * gs + j
+                _bmm(lib, dv.data_ptr() + (g * E + b * E * Hkv * S) * es, G.data_ptr() + (h * E + b * E * H * Lq) * es,
+                     w.data_ptr() + ((h + H * b) * S * Lq) * es, E, S, Lq, 1, E * H, S, E * Hkv, 0, 0, E * S, 0, 1, dt, device,
+                     accumulate=1 if j else 0, flags=flags)
+                _bmm(lib, dk.data_ptr() + (g * D + b * D * Hkv * S) * es, Q.data_ptr() + (h * D + b * D * H * Lq) * es,
+                     dl.data_ptr() + ((h + H * b) * S * Lq) * es, D, S, Lq, 1, D * H, S, D * Hkv, 0, 0, D * S, 0, 1, dt, device,
+                     accumulate=1 if j else 0, flags=flags)
+
+
 def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_causal=None, bias=None, flags: int = 0):
     """LuxLib.scaled_dot_product_attention (lib/LuxLib/src/api/attention.jl, impl/attention.jl:5-118) for the default
     dimension roles head_dim = 1, token_dim = 3: q (D, H, L, B...), k (D, Hkv, S, B...), v (E, Hkv, S, B...) ->
@@ -625,24 +667,16 @@ def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_cau
         raise AssertionError("`v` and `k` must have the same number of tokens and heads")
     if H % Hkv != 0:
         raise AssertionError("num_heads must be divisible by num_kv_groups")
-    gs = H // Hkv
     batch_shape = tuple(Q.shape[3:])
     Bn = math.prod(batch_shape)
     sc = 1.0 / (float(scale) if scale is not None else float(D) ** 0.5)
-    dt, es, device = dtype_code(Q.dtype), Q.element_size(), Q.device
-    logits = jl_empty((S, Lq, H) + batch_shape, Q.dtype, device)
-
-    def per_group(fn):
-        for b in range(Bn):
-            for g in range(Hkv):
-                fn(b, g)
-
-    # logits[:, :, h, b] = k[:, g, :, b]' * q[:, h, :, b] for the gs heads h of group g: one batched call, k repeated
-    def fwd_logits(b, g):
-        _bmm(lib, logits.data_ptr() + ((g * gs + H * b) * S * Lq) * es, Kx.data_ptr() + (g * D + b * D * Hkv * S) * es,
-             Q.data_ptr() + (g * gs * D + b * D * H * Lq) * es, S, Lq, D, gs, D * Hkv, D * H, S, 0, D, S * Lq, 1, 0, dt, device, flags=flags)
-    per_group(fwd_logits)
-
+    dt, device = dtype_code(Q.dtype), Q.device
+    dims = _cabi.AttentionDims(D, E, H, Hkv, Lq, S, Bn)
+    # the tensor-core path reads the arrays through TMA (16-byte bases); the rest runs product by product
+    fused = flags == 0 and lib.lb2_attention_is_fused(C.byref(dims), dt) == 1 and not any(t.data_ptr() % 16 for t in (Q, Kx, V))
+    w = jl_empty((S, Lq, H) + batch_shape, Q.dtype, device)
+    out = jl_empty((E, H, Lq) + batch_shape, Q.dtype, device)
+    causal = 1 if is_causal else 0
     bias_c = mask_c = None
     bias_bs = mask_bs = 0
     if bias is not None:
@@ -661,46 +695,23 @@ def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_cau
             mask_bs = S * Lq
         else:
             raise DimensionMismatch("mask must have the shape (S, L) or (S, L, H, B...)")
-    w = jl_empty(tuple(logits.shape), Q.dtype, device)
-    _cabi.check(lib.lb2_attention_softmax_fwd(ptr(w), ptr(logits), ptr(bias_c), bias_bs, ptr(mask_c), mask_bs, 1 if is_causal else 0, sc,
-                                              S, Lq, H * Bn, dt, current_stream(device)))
-    out = jl_empty((E, H, Lq) + batch_shape, Q.dtype, device)
-
-    # x[:, h, :, b] = v[:, g, :, b] * w[:, :, h, b]
-    def fwd_out(b, g):
-        _bmm(lib, out.data_ptr() + (g * gs * E + b * E * H * Lq) * es, V.data_ptr() + (g * E + b * E * Hkv * S) * es,
-             w.data_ptr() + ((g * gs + H * b) * S * Lq) * es, E, Lq, S, gs, E * Hkv, S, E * H, 0, S * Lq, E, 0, 0, dt, device, flags=flags)
-    per_group(fwd_out)
+    if fused:
+        _, wsp, wsn = _ws(lib.lb2_attention_fwd_workspace_bytes(C.byref(dims), dt), device)
+        _cabi.check(lib.lb2_attention_fwd(ptr(out), ptr(w), ptr(Q), ptr(Kx), ptr(V), ptr(bias_c), bias_bs, ptr(mask_c), mask_bs, causal, sc,
+                                          C.byref(dims), dt, wsp, wsn, current_stream(device)))
+    else:
+        _attention_fwd_by_product(lib, out, w, Q, Kx, V, bias_c, bias_bs, mask_c, mask_bs, causal, sc, dims, dt, flags)
 
     def pullback(dx):
         G = as_colmajor(dx.to(Q.dtype))
-        dw = jl_empty(tuple(w.shape), Q.dtype, device)
         dq, dk, dv = (jl_empty(tuple(t.shape), Q.dtype, device) for t in (Q, Kx, V))
-
-        # dw[:, :, h, b] = v[:, g, :, b]' * dx[:, h, :, b]
-        def bwd_dw(b, g):
-            _bmm(lib, dw.data_ptr() + ((g * gs + H * b) * S * Lq) * es, V.data_ptr() + (g * E + b * E * Hkv * S) * es,
-                 G.data_ptr() + (g * gs * E + b * E * H * Lq) * es, S, Lq, E, gs, E * Hkv, E * H, S, 0, E, S * Lq, 1, 0, dt, device, flags=flags)
-        per_group(bwd_dw)
-        dl = jl_empty(tuple(w.shape), Q.dtype, device)
         db = jl_empty(tuple(w.shape), Q.dtype, device) if bias_c is not None else None
-        _cabi.check(lib.lb2_attention_softmax_bwd(ptr(dl), ptr(db), ptr(dw), ptr(w), sc, S, Lq, H * Bn, dt, current_stream(device)))
-
-        # per head (the heads of a group add into the same dk / dv, so they run one after the other, in order):
-        # dv[:, g, :, b] += dx[:, h, :, b] * w[:, :, h, b]';  dk[:, g, :, b] += q[:, h, :, b] * dl[:, :, h, b]'
-        # dq[:, h, :, b] = k[:, g, :, b] * dl[:, :, h, b]
-        def bwd_rest(b, g):
-            _bmm(lib, dq.data_ptr() + (g * gs * D + b * D * H * Lq) * es, Kx.data_ptr() + (g * D + b * D * Hkv * S) * es,
-                 dl.data_ptr() + ((g * gs + H * b) * S * Lq) * es, D, Lq, S, gs, D * Hkv, S, D * H, 0, S * Lq, D, 0, 0, dt, device, flags=flags)
-            for j in range(gs):
-                h = g * gs + j
-                _bmm(lib, dv.data_ptr() + (g * E + b * E * Hkv * S) * es, G.data_ptr() + (h * E + b * E * H * Lq) * es,
-                     w.data_ptr() + ((h + H * b) * S * Lq) * es, E, S, Lq, 1, E * H, S, E * Hkv, 0, 0, E * S, 0, 1, dt, device,
-                     accumulate=1 if j else 0, flags=flags)
-                _bmm(lib, dk.data_ptr() + (g * D + b * D * Hkv * S) * es, Q.data_ptr() + (h * D + b * D * H * Lq) * es,
-                     dl.data_ptr() + ((h + H * b) * S * Lq) * es, D, S, Lq, 1, D * H, S, D * Hkv, 0, 0, D * S, 0, 1, dt, device,
-                     accumulate=1 if j else 0, flags=flags)
-        per_group(bwd_rest)
+        if fused and G.data_ptr() % 16 == 0:
+            _, wsp, wsn = _ws(lib.lb2_attention_bwd_workspace_bytes(C.byref(dims), dt), device)
+            _cabi.check(lib.lb2_attention_bwd(ptr(dq), ptr(dk), ptr(dv), ptr(db), ptr(G), ptr(w), ptr(Q), ptr(Kx), ptr(V), causal, sc,
+                                              C.byref(dims), dt, wsp, wsn, current_stream(device)))
+        else:
+            _attention_bwd_by_product(lib, dq, dk, dv, db, G, w, Q, Kx, V, sc, dims, dt, flags)
         if db is not None and bias_bs == 0:
             # a bias shared by all heads and samples: its gradient is the sum over them — the bias-gradient reduction on
             # the (1, S*L, H*B) view

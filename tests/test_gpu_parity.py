@@ -1109,3 +1109,40 @@ def test_fused_conv_f32_general_path(case, offset, act):
     for name, got, want in zip(("dw", "dx", "db"), pb(place(delta)), pb_ref(delta.astype(np.float64))):
         check(got, want, "f32", name, tol=2e-6)
     assert L._cabi.load().lb2_poll_device_status(None) == 0
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("variant", ["plain", "causal", "mask+bias"])
+@pytest.mark.parametrize("dims", [
+    # D, H, Hkv, L, S, E, B — edges of the tensor-core attention products
+    (80, 4, 2, 129, 127, 80, 2),       # one row past a tile, keys not a multiple of 8, two k-blocks of features
+    (32, 3, 1, 257, 64, 48, 1),        # more queries than keys, three heads share one key head
+    (64, 2, 2, 20, 300, 128, 3),       # more keys than queries: keys no query sees under a causal mask
+    (16, 1, 1, 9, 1100, 16, 1),        # rows longer than the registers hold
+    (128, 2, 1, 130, 130, 8, 1),
+])
+def test_attention_tensor_core_path(dt, variant, dims):
+    D, H, Hkv, Lq, S, E, B = dims
+    d = L._cabi.AttentionDims(D, E, H, Hkv, Lq, S, B)
+    assert L._cabi.load().lb2_attention_is_fused(d, 1 if dt == "bf16" else 0) == 1
+    rng = np.random.default_rng(62)
+    q, k, v, dx = (prep(rng.standard_normal(s), dt) for s in ((D, H, Lq, B), (D, Hkv, S, B), (E, Hkv, S, B), (E, H, Lq, B)))
+    mask = bias = None
+    if variant == "mask+bias":
+        mask = rng.random((S, Lq)) > 0.3
+        mask[0, :] = True
+        bias = prep(rng.standard_normal((S, Lq)) * 0.5, dt)
+    f64 = lambda a: None if a is None else a.astype(np.float64)
+    causal = True if variant == "causal" else None
+    (x_ref, w_ref), pb_ref = O.attention_rrule(f64(q), f64(k), f64(v), mask=mask, is_causal=causal, bias=f64(bias))
+    (x, w), pb = L.rrule_scaled_dot_product_attention(
+        dev(q, dt), dev(k, dt), dev(v, dt), is_causal=causal, bias=dev(bias, dt),
+        mask=None if mask is None else L.from_numpy(mask.astype(np.uint8), "cuda", torch.uint8))
+    check(w, w_ref, dt, "weights")
+    check(x, x_ref, dt, "x")
+    if causal:
+        assert np.all(L.to_numpy(w)[np.arange(S)[:, None] > np.arange(Lq)[None, :]] == 0)
+    for name, got, want in zip(("dq", "dk", "dv", "dbias"), pb(dev(dx, dt)), pb_ref(f64(dx))):
+        if name != "dbias" or bias is not None:
+            check(got, want, dt, name)
+    assert L._cabi.load().lb2_poll_device_status(None) == 0
