@@ -6,6 +6,8 @@
 // contracted index is contiguous (element (i,k) at k + i*ld). Julia's W*x is A = W (MN-major),
 // B = x (K-major); W'*g is both K-major; g*x' is both MN-major.
 #pragma once
+#include <cuda.h>
+
 #include "common.cuh"
 
 namespace lb2 {
@@ -46,6 +48,26 @@ int32_t gemm_dispatch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64_
                       int32_t dtype, uint32_t flags, const GemmEpilogue& epi, void* ws, size_t ws_bytes,
                       cudaStream_t st);
 
+// How one operand tile is fetched by TMA and described to the MMA.
+struct GemmTmaPlan {
+  int32_t boxes;        // TMA boxes per k-block
+  int32_t box_bytes;    // bytes each box lands in shared memory
+  int32_t mn_step;      // MN-major: elements of the MN extent covered by one box; K-major: unused
+  int32_t mn_major;     // 1: coordinates are {mn, k}; 0: {k, mn}
+  uint32_t desc_hi;     // upper 32 bits of the UMMA smem descriptor (SBO, version, swizzle)
+  uint32_t desc_lbo;    // LBO field already shifted into bits [16,30) of the lower word
+  uint32_t k_advance;   // descriptor start-address increment (bytes >> 4) per MMA k-step
+};
+// 2-D map over an operand. K-major: dims {K, MN}; MN-major: dims {MN, K}. Box = 128-byte rows.
+bool gemm_tma_map(CUtensorMap* map, const GemmOperand& op, int64_t mn, int64_t kc, int elem_bytes, int tile_mn, int bk, GemmTmaPlan* plan,
+                  bool tf32);
+
+// Few output tiles: the contraction split over the CTAs of a cluster (gemm_cluster.cu).
+bool gemm_cluster_wanted(int64_t Mm, int64_t Nn, int64_t Kc, int32_t dtype);
+int32_t gemm_cluster_launch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64_t Mm, int64_t Nn, int64_t Kc, int32_t dtype,
+                            const GemmEpilogue& epi, cudaStream_t st);
+
 extern thread_local int32_t g_last_gemm_plan[8];   // see gemm_tc.cu
+void record_gemm_plan(int kernel, int tile_m, int tile_n, int tiles, int workers, int full_slots, int total_slots);
 
 }  // namespace lb2

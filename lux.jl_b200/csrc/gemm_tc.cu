@@ -34,19 +34,8 @@ namespace lb2 {
 // ----------------------------------------------------------------------------------------------
 // kernel
 // ----------------------------------------------------------------------------------------------
-// How one operand tile is fetched and described (filled in on the host).
-struct OperandPlan {
-  int32_t boxes;        // TMA boxes per k-block
-  int32_t box_bytes;    // bytes each box lands in shared memory
-  int32_t mn_step;      // MN-major: elements of the MN extent covered by one box; K-major: unused
-  int32_t mn_major;     // 1: coordinates are {mn, k}; 0: {k, mn}
-  uint32_t desc_hi;     // upper 32 bits of the UMMA smem descriptor (SBO, version, swizzle)
-  uint32_t desc_lbo;    // LBO field already shifted into bits [16,30) of the lower word
-  uint32_t k_advance;   // descriptor start-address increment (bytes >> 4) per MMA k-step
-};
-
 struct TcParams {
-  OperandPlan a, b;
+  GemmTmaPlan a, b;
   int64_t Mm, Nn, Kc;
   int32_t bk;           // elements of K per k-block (64 bf16 / 32 tf32)
   int32_t tiles_m, tiles_n, num_kb;
@@ -661,7 +650,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // host side
 // ----------------------------------------------------------------------------------------------
 // What the calling thread's last tensor-core GEMM launch looked like (read by lb2_last_gemm_plan; tests use it to
-// assert which kernel and which tile schedule a shape takes): kernel (1 single-CTA, 2 CTA pair), tile_m, tile_n,
+// assert which kernel and which tile schedule a shape takes): kernel (1 single-CTA, 2 CTA pair, 3 cluster), tile_m, tile_n,
 // tiles, workers (CTAs or CTA pairs), full_slots, total_slots.
 thread_local int32_t g_last_gemm_plan[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 void record_gemm_plan(int kernel, int tile_m, int tile_n, int tiles, int workers, int full_slots, int total_slots) {
@@ -685,9 +674,8 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// 2-D map over an operand. K-major: dims {K, MN}; MN-major: dims {MN, K}. Box = 128-byte rows.
-static bool make_operand_map(CUtensorMap* map, const GemmOperand& op, int64_t mn, int64_t kc, int elem_bytes,
-                             int tile_mn, int bk, OperandPlan* plan, bool tf32) {
+bool gemm_tma_map(CUtensorMap* map, const GemmOperand& op, int64_t mn, int64_t kc, int elem_bytes, int tile_mn, int bk, GemmTmaPlan* plan,
+                  bool tf32) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
   const int row_elems = 128 / elem_bytes;  // elements in a 128-byte row
@@ -907,7 +895,7 @@ int32_t gemm_tc_launch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64
   TcParams p{};
   CUtensorMap mA, mB, mAl, mBl;
   if (!split) {
-    if (!make_operand_map(&mA, A, Mm, Kc, es, kBM, bk, &p.a, tf32) || !make_operand_map(&mB, B, Nn, Kc, es, bn, bk, &p.b, tf32))
+    if (!gemm_tma_map(&mA, A, Mm, Kc, es, kBM, bk, &p.a, tf32) || !gemm_tma_map(&mB, B, Nn, Kc, es, bn, bk, &p.b, tf32))
       return fail(LB2_LAUNCH_FAIL, "gemm_tc: cuTensorMapEncodeTiled failed");
     mAl = mA; mBl = mB;
   } else {
@@ -927,9 +915,9 @@ int32_t gemm_tc_launch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64
     Ah.ptr = a_hi; Al.ptr = a_lo; Bh.ptr = b_hi; Bl.ptr = b_lo;
     Ah.ld = Al.ld = packed_ld(a_rows);
     Bh.ld = Bl.ld = packed_ld(b_rows);
-    OperandPlan dummy;
-    if (!make_operand_map(&mA, Ah, Mm, Kc, es, kBM, bk, &p.a, tf32) || !make_operand_map(&mAl, Al, Mm, Kc, es, kBM, bk, &dummy, tf32) ||
-        !make_operand_map(&mB, Bh, Nn, Kc, es, bn, bk, &p.b, tf32) || !make_operand_map(&mBl, Bl, Nn, Kc, es, bn, bk, &dummy, tf32))
+    GemmTmaPlan dummy;
+    if (!gemm_tma_map(&mA, Ah, Mm, Kc, es, kBM, bk, &p.a, tf32) || !gemm_tma_map(&mAl, Al, Mm, Kc, es, kBM, bk, &dummy, tf32) ||
+        !gemm_tma_map(&mB, Bh, Nn, Kc, es, bn, bk, &p.b, tf32) || !gemm_tma_map(&mBl, Bl, Nn, Kc, es, bn, bk, &dummy, tf32))
       return fail(LB2_LAUNCH_FAIL, "gemm_tc: cuTensorMapEncodeTiled failed (split operands)");
   }
   p.Mm = Mm; p.Nn = Nn; p.Kc = Kc;
@@ -981,17 +969,63 @@ int32_t gemm_tc_launch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64
 // ----------------------------------------------------------------------------------------------
 // dispatch between the tensor-core and CUDA-core kernels
 // ----------------------------------------------------------------------------------------------
+constexpr int64_t kTcMinWork = (int64_t)64 * 64 * 64;   // below it the CUDA-core kernel is latency-bound either way
+
 static bool use_tc(const void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64_t Mm, int64_t Nn, int64_t Kc,
                    int32_t dtype, uint32_t flags) {
   if (flags & LB2_FLAG_FORCE_SIMT) return false;
-  if (Mm * Nn * Kc < (int64_t)64 * 64 * 64) return false;  // latency-bound either way; skip descriptor encoding
+  if (Mm * Nn * Kc < kTcMinWork) return false;
   return gemm_tc_supported(D, ldd, A, B, Mm, Nn, Kc, dtype, (flags & LB2_FLAG_TF32_1X) ? 0 : 1);
+}
+
+// bf16 operands that break the TMA rules (base or leading dimension not a multiple of 16 bytes: odd layer widths) are copied
+// to packed columns of a multiple of 8 elements first: one bandwidth pass instead of a CUDA-core product (3001 x 5000 x 2003,
+// forward: 2.29 ms -> 0.10 ms; 1001 x 1 x 3000: 307 -> 14.5 us).
+__global__ void __launch_bounds__(256) pack_bf16_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in, int64_t rows, int64_t cols,
+                                                        int64_t ld_in, int64_t ld_out) {
+  const int64_t vecs = ld_out / 8, n = vecs * cols;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = i / vecs, r = (i - c * vecs) * 8;
+    const uint16_t* src = in + c * ld_in + r;
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t lo = r + 2 * k < rows ? __ldg(src + 2 * k) : 0u, hi = r + 2 * k + 1 < rows ? __ldg(src + 2 * k + 1) : 0u;
+      w[k] = lo | (hi << 16);
+    }
+    *reinterpret_cast<uint4*>(out + c * ld_out + r) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+static int64_t packed_ld16(int64_t rows) { return (rows + 7) / 8 * 8; }
+static size_t packed_bytes16(const GemmOperand& op, int64_t mn, int64_t kc) {
+  return align_up((size_t)packed_ld16(operand_rows(op, mn, kc)) * (size_t)operand_cols(op, mn, kc) * 2, 256);
+}
+static bool tma_ready(const GemmOperand& op) { return aligned_to(op.ptr, 16) && (op.ld * 2) % 16 == 0; }
+static int32_t pack_operand(GemmOperand* op, int64_t mn, int64_t kc, uint8_t** ws, cudaStream_t st) {
+  const int64_t rows = operand_rows(*op, mn, kc), cols = operand_cols(*op, mn, kc), ld = packed_ld16(rows);
+  const int64_t blocks = (ld / 8 * cols + 255) / 256, cap = (int64_t)sm_count() * 16;
+  pack_bf16_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(reinterpret_cast<uint16_t*>(*ws), static_cast<const uint16_t*>(op->ptr),
+                                                                           rows, cols, op->ld, ld);
+  LB2_CHECK_LAUNCH("pack_bf16");
+  const size_t bytes = packed_bytes16(*op, mn, kc);
+  op->ptr = *ws;
+  op->ld = ld;
+  *ws += bytes;
+  return LB2_OK;
+}
+
+// a cluster splits the contraction unless the caller asked for a particular kernel or for spare SMs
+static bool use_cluster(int64_t Mm, int64_t Nn, int64_t Kc, int32_t dtype, uint32_t flags) {
+  return flags == 0 && Mm * Nn * Kc >= kTcMinWork && gemm_cluster_wanted(Mm, Nn, Kc, dtype) && encode_fn() != nullptr;
 }
 
 size_t gemm_workspace_bytes(GemmOperand A, GemmOperand B, int64_t Mm, int64_t Nn, int64_t Kc, int32_t dtype,
                             uint32_t flags) {
-  if (dtype != LB2_F32 || (flags & (LB2_FLAG_TF32_1X | LB2_FLAG_FORCE_SIMT))) return 0;
+  if (flags & LB2_FLAG_FORCE_SIMT) return 0;
   if (Mm <= 0 || Nn <= 0 || Kc <= 0) return 0;
+  if (dtype == LB2_BF16)
+    return (operand_rows(A, Mm, Kc) % 8 != 0 ? packed_bytes16(A, Mm, Kc) : 0) + (operand_rows(B, Nn, Kc) % 8 != 0 ? packed_bytes16(B, Nn, Kc) : 0);
+  if ((flags & LB2_FLAG_TF32_1X) || use_cluster(Mm, Nn, Kc, dtype, flags)) return 0;
   return gemm_tc_split_workspace_bytes(A, B, Mm, Nn, Kc);
 }
 
@@ -999,7 +1033,18 @@ int32_t gemm_dispatch(void* D, int64_t ldd, GemmOperand A, GemmOperand B, int64_
                       int32_t dtype, uint32_t flags, const GemmEpilogue& epi, void* ws, size_t ws_bytes,
                       cudaStream_t st) {
   if (Mm == 0 || Nn == 0) return LB2_OK;
+  if (Kc > 0 && dtype == LB2_BF16 && !(flags & LB2_FLAG_FORCE_SIMT) && Mm * Nn * Kc >= kTcMinWork && (!tma_ready(A) || !tma_ready(B))) {
+    // a view whose base or leading dimension alone is unaligned has no room in the workspace and stays on the CUDA cores
+    const size_t need = (tma_ready(A) ? 0 : packed_bytes16(A, Mm, Kc)) + (tma_ready(B) ? 0 : packed_bytes16(B, Nn, Kc));
+    if (ws != nullptr && ws_bytes >= need && aligned_to(ws, 16)) {
+      uint8_t* w = static_cast<uint8_t*>(ws);
+      int32_t rc = tma_ready(A) ? LB2_OK : pack_operand(&A, Mm, Kc, &w, st);
+      if (rc == LB2_OK && !tma_ready(B)) rc = pack_operand(&B, Nn, Kc, &w, st);
+      if (rc != LB2_OK) return rc;
+    }
+  }
   if (Kc > 0 && use_tc(D, ldd, A, B, Mm, Nn, Kc, dtype, flags)) {
+    if (use_cluster(Mm, Nn, Kc, dtype, flags)) return gemm_cluster_launch(D, ldd, A, B, Mm, Nn, Kc, dtype, epi, st);
     const int split3 = (dtype == LB2_F32 && !(flags & LB2_FLAG_TF32_1X)) ? 1 : 0;
     if (split3) {
       const size_t need = gemm_tc_split_workspace_bytes(A, B, Mm, Nn, Kc);

@@ -1146,3 +1146,48 @@ def test_attention_tensor_core_path(dt, variant, dims):
         if name != "dbias" or bias is not None:
             check(got, want, dt, name)
     assert L._cabi.load().lb2_poll_device_status(None) == 0
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("mnk,offset", [
+    ((129, 65, 129), 0),         # one past a tile and a k-block
+    ((128, 64, 8192), 0),        # one tile, eight splits
+    ((1001, 1, 4097), 0),        # a single column; odd leading dimensions (bf16: packed copies)
+    ((257, 130, 515), 1),        # bases aligned to the element only
+    ((96, 40, 2080), 0),         # a tile that neither its rows nor its columns fill, splits of unequal length
+    ((515, 3000, 333), 0),       # odd widths and many tiles
+])
+def test_matmul_few_tiles_and_odd_widths(dt, ta, tb, mnk, offset):
+    M, N, K = mnk
+    rng = np.random.default_rng(63)
+    A, B, C0 = (prep(rng.standard_normal(s), dt) for s in ((K, M) if ta else (M, K), (N, K) if tb else (K, N), (M, N)))
+    want = (A.T if ta else A).astype(np.float64) @ (B.T if tb else B).astype(np.float64)
+
+    def place(a):
+        t = dev(a, dt)
+        if not offset:
+            return t
+        out = torch.as_strided(torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda"), t.shape, t.stride(), 1)
+        out.copy_(t)
+        return out
+    a, b = place(A), place(B)
+    check(L.matmul(a, b, transA=ta, transB=tb), want, dt, "C")
+    c = place(C0)
+    L.matmul(a, b, transA=ta, transB=tb, out=c, accumulate=True)
+    check(c, want + C0, dt, "C += ")
+    assert L._cabi.load().lb2_poll_device_status(None) == 0
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("act", ["gelu", "relu"])
+@pytest.mark.parametrize("mnk", [(250, 8, 4096), (1001, 33, 257), (64, 300, 100)])
+def test_dense_epilogue_of_the_cluster_kernel(dt, act, mnk):
+    M, N, K = mnk
+    rng = np.random.default_rng(64)
+    W, x, b, d = (prep(a, dt) for a in (O.glorot_uniform(rng, (M, K)), rng.standard_normal((K, N)), rng.uniform(-1, 1, M), rng.standard_normal((M, N))))
+    y_ref, pb_ref = O.fused_dense_rrule(act, *(a.astype(np.float64) for a in (W, x, b)))
+    y, pb = L.rrule_fused_dense(act, dev(W, dt), dev(x, dt), dev(b, dt))
+    check(y, y_ref, dt, "y")
+    for name, got, want in zip(("dW", "dx", "db"), pb(dev(d, dt)), pb_ref(d.astype(np.float64))):
+        check(got, want, dt, name)
