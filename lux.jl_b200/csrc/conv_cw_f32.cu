@@ -15,8 +15,8 @@
 // A problem with too few tiles for the SMs is split along the contraction as well: fp32 partials in the layout of the
 // output and one elementwise pass that adds them in order (deterministic) and applies bias and activation.
 //
-// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 96 / 174 us (77 /
-// 85 TFLOP/s); 3x3 512 -> 512 on 7x7: 105 / 215 us. The CUDA-core kernels of conv_direct.cu, which took these geometries
+// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 86 / 158 us (86 /
+// 94 TFLOP/s); 3x3 512 -> 512 on 7x7: 96 / 198 us (with the MMAs issued from a one-lane branch: 96 / 174 and 105 / 215 us). The CUDA-core kernels of conv_direct.cu, which took these geometries
 // before, made a ResNet-18 training step at batch 32 last 333 ms; it now takes 6.7 ms.
 // What bounds it: a 128 x 128 x 32 k-block is 768 tensor-pipe cycles (three tf32 products) against about 1280 cycles of
 // shared-memory traffic (64 KB written by TMA, 96 KB read by the MMAs at 128 B/cycle).
@@ -209,35 +209,38 @@ template <int SLOTS> struct CwfRing {
 };
 template <int BN>
 __device__ __forceinline__ bool cwf_issue_kblock(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_base, uint32_t sA, uint32_t sB, uint32_t desc_hi,
-                                                 uint32_t lbo, uint32_t k_adv, uint32_t idesc, bool first, bool last, unsigned int* status,
-                                                 unsigned int code) {
+                                                 uint32_t lbo, uint32_t k_adv, uint32_t idesc, bool first, bool last, uint64_t* stage_empty,
+                                                 unsigned int* status, unsigned int code) {
   constexpr int SLOTS = CwfCfg<BN>::SLOTS;
   const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | lbo, b32 = ((sB >> 4) & 0x3FFFu) | lbo;
   const uint64_t top = (uint64_t)desc_hi << 32;
   constexpr uint32_t A_LO = CwfCfg<BN>::A_BYTES >> 4, B_LO = CwfCfg<BN>::B_BYTES >> 4;
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
-    if (!mbar_wait(&ring.empty[ring.slot], ring.phase ^ 1u, status, code)) return false;
-    tc_fence_after();
-#pragma unroll
-    for (int ks = 2 * part; ks < 2 * part + 2; ++ks)
-      umma<true>(tmem_base + ring.slot * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, ks != 2 * part ? 1u : 0u);
-    umma_commit(&ring.full[ring.slot]);
-    ring.next();
+    if (!mbar_wait_uniform(&ring.empty[ring.slot], ring.phase ^ 1u, status, code)) return false;
     if (first && part == 0) {
-      if (!mbar_wait(&ring.empty[SLOTS], ring.small_phase ^ 1u, status, code)) return false;
-      tc_fence_after();
+      if (!mbar_wait_uniform(&ring.empty[SLOTS], ring.small_phase ^ 1u, status, code)) return false;
     }
+    tc_fence_after();
+    if (elect_one()) {
 #pragma unroll
-    for (int ks = 2 * part; ks < 2 * part + 2; ++ks) {
-      umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + B_LO + ks * k_adv), idesc, first && ks == 0 ? 0u : 1u);
-      umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + A_LO + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, 1u);
+      for (int ks = 2 * part; ks < 2 * part + 2; ++ks)
+        umma<true>(tmem_base + ring.slot * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, ks != 2 * part ? 1u : 0u);
+      umma_commit(&ring.full[ring.slot]);
+#pragma unroll
+      for (int ks = 2 * part; ks < 2 * part + 2; ++ks) {
+        umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + B_LO + ks * k_adv), idesc, first && ks == 0 ? 0u : 1u);
+        umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + A_LO + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, 1u);
+      }
+      if (part == 1) {
+        umma_commit(stage_empty);
+        if (last) umma_commit(&ring.full[SLOTS]);
+      }
     }
+    __syncwarp();
+    ring.next();
   }
-  if (last) {
-    umma_commit(&ring.full[SLOTS]);
-    ring.small_phase ^= 1u;
-  }
+  if (last) ring.small_phase ^= 1u;
   return true;
 }
 // accumulating side: one item's k-blocks, columns [col, col + BN / 2) of the warp's lane quarter
@@ -384,20 +387,17 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        int tn, tw, th, ti, z;
-        item_coords(item, &tn, &tw, &th, &ti, &z);
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
-          if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiK, kLboK, kAdvK, p.idesc, kb == kb_lo, kb == kb_hi - 1, p.status, 0x2000u)) { ok = false; break; }
-          umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      int tn, tw, th, ti, z;
+      item_coords(item, &tn, &tw, &th, &ti, &z);
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiK, kLboK, kAdvK, p.idesc, kb == kb_lo, kb == kb_hi - 1, &empty[stage], p.status, 0x2000u)) { ok = false; break; }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
@@ -548,19 +548,16 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int z = item / per_split;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
-          if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiMN, kLboMN, kAdvMN, p.idesc, kb == kb_lo, kb == kb_hi - 1, p.status, 0x40000u)) { ok = false; break; }
-          umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int z = item / per_split;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiMN, kLboMN, kAdvMN, p.idesc, kb == kb_lo, kb == kb_hi - 1, &empty[stage], p.status, 0x40000u)) { ok = false; break; }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
