@@ -106,16 +106,16 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        Item t;
-        if (!decode(item, &t)) continue;
-        for (int j = 0; j < p.rep && ok; ++j) {
-          const int hh = t.head * p.rep + j, ha = hh / p.a.head_div, hb = hh / p.b.head_div;
-          for (int kb = t.kb_lo; kb < t.kb_hi; ++kb) {
-            if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      Item t;
+      if (!decode(item, &t)) continue;
+      for (int j = 0; j < p.rep && ok; ++j) {
+        const int hh = t.head * p.rep + j, ha = hh / p.a.head_div, hb = hh / p.b.head_div;
+        for (int kb = t.kb_lo; kb < t.kb_hi; ++kb) {
+          if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1u)) { ok = false; break; }
+          if (elect_one()) {
             mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
             const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * (F32 ? 2 : 1);
             const int k0 = kb * p.bk;
@@ -127,28 +127,29 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               at_load(sB + bx * p.b.box_bytes, &tmB, p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
               if constexpr (F32) at_load(sB + Cfg::B_BYTES + bx * p.b.box_bytes, &tmBl, p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
             }
-            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
+          __syncwarp();
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = true;
-      for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        Item t;
-        if (!decode(item, &t)) continue;
-        const int n_kb = (t.kb_hi - t.kb_lo) * p.rep;
-        for (int kb = 0; kb < n_kb; ++kb) {
-          if (F32 || kb == 0) {
-            if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2u)) { ok = false; break; }
-          }
-          if (!mbar_wait(&full[stage], phase, p.status, 0x4u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_COLS;
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * (F32 ? 2 : 1);
-          const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | p.a.lbo, b32 = ((sB >> 4) & 0x3FFFu) | p.b.lbo;
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      Item t;
+      if (!decode(item, &t)) continue;
+      const int n_kb = (t.kb_hi - t.kb_lo) * p.rep;
+      for (int kb = 0; kb < n_kb; ++kb) {
+        if (F32 || kb == 0) {
+          if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2u)) { ok = false; break; }
+        }
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4u)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_COLS;
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * (F32 ? 2 : 1);
+        const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | p.a.lbo, b32 = ((sB >> 4) & 0x3FFFu) | p.b.lbo;
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(a32 + ks * p.a.k_adv);
@@ -161,12 +162,13 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
           }
           umma_commit(&empty[stage]);
-          if (F32 || kb == n_kb - 1) {
-            umma_commit(&acc_full[acc]);
-            if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (F32 || kb == n_kb - 1) umma_commit(&acc_full[acc]);
         }
+        __syncwarp();
+        if (F32 || kb == n_kb - 1) {
+          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {

@@ -322,39 +322,40 @@ conv_cw_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmW);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int tn, tw, th, ti;
-        tile_coords(tile, &tn, &tw, &th, &ti);
-        const int w0 = tw * p.BW * p.sw, h0 = th * p.BH * p.sh, i0 = ti * p.BI, n0 = tn * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      int tn, tw, th, ti;
+      tile_coords(tile, &tn, &tw, &th, &ti);
+      const int w0 = tw * p.BW * p.sw, h0 = th * p.BH * p.sh, i0 = ti * p.BI, n0 = tn * BN;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], a_bytes + (uint32_t)B_BYTES);
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
           tma_load_4d(sA, &tmX, p.kb_c0[kb], w0 + p.kb_dw[kb], h0 + p.kb_dh[kb], i0, &full[stage]);
           tma_load_2d(sB, &tmW, p.kb_k0[kb], n0, &full[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2000u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2000u)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | (1u << 16);
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | (1u << 16);
+        const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | (1u << 16);
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | (1u << 16);
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint64_t ad = ((uint64_t)kDescHiSw128 << 32) | (uint64_t)(a_lo32 + ks * 2);
@@ -362,11 +363,13 @@ conv_cw_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             umma<false>(d_tmem, ad, bd, p.idesc, (kb | ks) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     // Two warps share each TMEM lane quarter and split the tile's channels. A thread owns one output position and
@@ -542,16 +545,16 @@ conv_cw_wgrad_kernel(const __grid_constant__ CUtensorMap tmG, const __grid_const
 
   // item -> (co tile fastest, group, split)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmG);
-      tma_prefetch_desc(&tmX);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int ct = item % p.co_tiles, grp = (item / p.co_tiles) % p.groups, z = item / per_split;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmG);
+    tma_prefetch_desc(&tmX);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int ct = item % p.co_tiles, grp = (item / p.co_tiles) % p.groups, z = item / per_split;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+        if (elect_one()) {
           const int bw = kb % p.kbw, bh = (kb / p.kbw) % p.kbh, bi = kb / (p.kbw * p.kbh);
           const int a0 = bw * p.KW_, b0 = bh * p.KH_, i0 = bi * p.KI_;
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
@@ -564,30 +567,31 @@ conv_cw_wgrad_kernel(const __grid_constant__ CUtensorMap tmG, const __grid_const
             if (pr >= p.n_pairs) pr = grp * p.pairs_per_group;   // filler column group (its results are never read)
             tma_load_4d(sB + j * (64 * 128), &tmX, p.pr_c0[pr], a0 * p.sw + p.pr_dw[pr], b0 * p.sh + p.pr_dh[pr], i0, &full[stage]);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = true;
-      // both operands MN-major: 64-wide groups of the non-contracted index are 8192 bytes apart (LBO), eight
-      // positions form a 1024-byte swizzle atom (SBO), one MMA step covers 16 positions = 2048 bytes
-      constexpr uint32_t LBO = ((8192u >> 4) & 0x3FFFu) << 16;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int z = item / per_split;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        if (kb_lo >= kb_hi) continue;   // an empty split contributes nothing (the epilogue writes zeros)
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    // both operands MN-major: 64-wide groups of the non-contracted index are 8192 bytes apart (LBO), eight
+    // positions form a 1024-byte swizzle atom (SBO), one MMA step covers 16 positions = 2048 bytes
+    constexpr uint32_t LBO = ((8192u >> 4) & 0x3FFFu) << 16;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int z = item / per_split;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      if (kb_lo >= kb_hi) continue;   // an empty split contributes nothing (the epilogue writes zeros)
+      if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | LBO;
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | LBO;
+        const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | LBO;
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | LBO;
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint64_t ad = ((uint64_t)kDescHiSw128 << 32) | (uint64_t)(a_lo32 + ks * (2048u >> 4));
@@ -595,11 +599,13 @@ conv_cw_wgrad_kernel(const __grid_constant__ CUtensorMap tmG, const __grid_const
             umma<false>(d_tmem, ad, bd, p.idesc, (kb > kb_lo || ks != 0) ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;

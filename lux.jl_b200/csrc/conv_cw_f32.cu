@@ -362,18 +362,18 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmWh); tma_prefetch_desc(&tmWl);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        int tn, tw, th, ti, z;
-        item_coords(item, &tn, &tw, &th, &ti, &z);
-        const int w0 = tw * p.BW * p.sw, h0 = th * p.BH * p.sh, i0 = ti * p.BI, n0 = tn * BN;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
-        int tap = kb_lo / p.chunks, ch = kb_lo - tap * p.chunks;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmWh); tma_prefetch_desc(&tmWl);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      int tn, tw, th, ti, z;
+      item_coords(item, &tn, &tw, &th, &ti, &z);
+      const int w0 = tw * p.BW * p.sw, h0 = th * p.BH * p.sh, i0 = ti * p.BI, n0 = tn * BN;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
+      int tap = kb_lo / p.chunks, ch = kb_lo - tap * p.chunks;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], tx);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
           const int w = w0 + p.tap_dw[tap], h = h0 + p.tap_dh[tap], k0 = (p.tap_index[tap] * p.chunks + ch) * 32;
@@ -381,9 +381,10 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
           tma_load_2d(sB, &tmWh, k0, n0, &full[stage]);
           tma_load_4d(sA + Cfg::A_BYTES, &tmXl, ch * 32, w, h, i0, &full[stage]);
           tma_load_2d(sB + Cfg::B_BYTES, &tmWl, k0, n0, &full[stage]);
-          if (++ch == p.chunks) { ch = 0; ++tap; }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++ch == p.chunks) { ch = 0; ++tap; }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
@@ -512,23 +513,23 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
 
   // item -> (m tile fastest, n tile, split)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmGh); tma_prefetch_desc(&tmGl);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / per_split;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        int dw[4], dh[4], c0[4];
+    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmGh); tma_prefetch_desc(&tmGl);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / per_split;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      int dw[4], dh[4], c0[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          int pr = mt * 4 + j;
-          if (pr >= p.n_pairs) pr = mt * 4;              // filler rows (never read by the reduction)
-          const int tap = pr / p.chunks;
-          dw[j] = p.tap_dw[tap]; dh[j] = p.tap_dh[tap]; c0[j] = (pr - tap * p.chunks) * 32;
-        }
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+      for (int j = 0; j < 4; ++j) {
+        int pr = mt * 4 + j;
+        if (pr >= p.n_pairs) pr = mt * 4;              // filler rows (never read by the reduction)
+        const int tap = pr / p.chunks;
+        dw[j] = p.tap_dw[tap]; dh[j] = p.tap_dh[tap]; c0[j] = (pr - tap * p.chunks) * 32;
+      }
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+        if (elect_one()) {
           const int bw = kb % p.kbw, bh = (kb / p.kbw) % p.kbh, bi = kb / (p.kbw * p.kbh);
           const int a0 = bw * p.KW_, b0 = bh * p.KH_, i0 = bi * p.KI_;
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
@@ -543,8 +544,9 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
             tma_load_4d(sB + j * 4096, &tmGh, nt * BN + j * 32, a0, b0, i0, &full[stage]);
             tma_load_4d(sB + Cfg::B_BYTES + j * 4096, &tmGl, nt * BN + j * 32, a0, b0, i0, &full[stage]);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {

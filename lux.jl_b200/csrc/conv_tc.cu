@@ -256,9 +256,9 @@ conv_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+    if (elect_one()) {
       mbar_expect_tx(b_full, (uint32_t)(num_b * B_BYTES));
       // packed filter column block (th*KW + tw)*chunks + chunk  ->  resident slot (th*chunks + chunk)*KW + tw,
       // so that the KW taps of one (kernel row, channel chunk) form ONE K-major operand of KW*64 rows
@@ -266,39 +266,43 @@ conv_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
         for (int tw = 0; tw < KW; ++tw)
           for (int ch = 0; ch < p.chunks; ++ch)
             tma_load_2d(sB0 + ((th * p.chunks + ch) * KW + tw) * B_BYTES, &tmW, ((th * KW + tw) * p.chunks + ch) * 64, n0, b_full);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int t = first; t < tiles_per_n && ok; t += step) {
-        const int s0 = (t % p.tiles_m) * kTileOut - kHalo, img = t / p.tiles_m;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+    }
+    __syncwarp();
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int t = first; t < tiles_per_n && ok; t += step) {
+      const int s0 = (t % p.tiles_m) * kTileOut - kHalo, img = t / p.tiles_m;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], A_BYTES);
           const uint32_t sA = sA0 + stage * A_BYTES;
           const int th = kb / p.chunks, chunk = kb % p.chunks;
           const int c0 = s0 + p.row_shift[th];
           tma_load_4d(sA, &tmX, c0, chunk * 64, img, 0, &full[stage]);
           tma_load_4d(sA + A_BYTES / 2, &tmX, c0 + 64, chunk * 64, img, 0, &full[stage]);
-          if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = mbar_wait(b_full, 0, p.status, 0x2000u);
-      for (int t = first; t < tiles_per_n && ok; t += step) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x4000u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = mbar_wait_uniform(b_full, 0, p.status, 0x2000u);
+    for (int t = first; t < tiles_per_n && ok; t += step) {
+      if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x4000u)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + acc * (KW * BN);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x8000u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + acc * (KW * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x8000u)) { ok = false; break; }
-          tc_fence_after();
-          const int th = kb / p.chunks, chunk = kb % p.chunks;
-          const uint32_t sA = sA0 + stage * A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a_desc_lbo;
-          // one MMA of N = KW*64 per k-step: its column blocks are the per-tap accumulators D_tw
-          const uint32_t sB = sB0 + (uint32_t)((th * p.chunks + chunk) * KW * B_BYTES);
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b_desc_lbo;
+        const int th = kb / p.chunks, chunk = kb % p.chunks;
+        const uint32_t sA = sA0 + stage * A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a_desc_lbo;
+        // one MMA of N = KW*64 per k-step: its column blocks are the per-tap accumulators D_tw
+        const uint32_t sB = sB0 + (uint32_t)((th * p.chunks + chunk) * KW * B_BYTES);
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b_desc_lbo;
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint64_t ad = ((uint64_t)p.a_desc_hi << 32) | (uint64_t)(a_lo32 + ks * p.a_k_advance);
@@ -306,11 +310,13 @@ conv_tc_fwd2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             umma<false>(d0, ad, bd, p.idesc, (kb | ks) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
-          if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     const int grp = (warp - 4) >> 3;                  // epilogue group = TMEM accumulator it drains
@@ -484,18 +490,18 @@ conv_tc_wgrad2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 
   // item -> (group fastest, split); group -> (co tile fastest, chunk, kernel row)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmX0);
-      tma_prefetch_desc(&tmG);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int grp = item % groups, z = item / groups;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        const int ct = grp % p.co_tiles, chunk = (grp / p.co_tiles) % p.chunks, th = grp / (p.co_tiles * p.chunks);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmX0);
+    tma_prefetch_desc(&tmG);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int grp = item % groups, z = item / groups;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      const int ct = grp % p.co_tiles, chunk = (grp / p.co_tiles) % p.chunks, th = grp / (p.co_tiles * p.chunks);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+        if (elect_one()) {
           const int img = kb / p.s_blocks, s0 = (kb % p.s_blocks) * 64;
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
           mbar_expect_tx(&full[stage], (uint32_t)STAGE_BYTES);
@@ -506,26 +512,27 @@ conv_tc_wgrad2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             if (tw == p.center_tw) tma_load_4d(sB + tw * (64 * 128), &tmX0, s0 + p.row_shift[th], chunk * 64, img, 0, &full[stage]);
             else tma_load_4d(sB + tw * (64 * 128), &tmX, s0 + p.row_shift[th], chunk * 64, img, tw, &full[stage]);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int z = item / groups;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int z = item / groups;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.desc_lbo;
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.desc_lbo;
+        const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.desc_lbo;
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.desc_lbo;
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint64_t ad = ((uint64_t)p.desc_hi << 32) | (uint64_t)(a_lo32 + ks * p.k_advance);
@@ -533,11 +540,13 @@ conv_tc_wgrad2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             umma<false>(d_tmem, ad, bd, p.idesc, (kb > kb_lo || ks != 0) ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;   // lane quarter; which half of the BN columns
@@ -699,17 +708,17 @@ conv_tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
 
   // item -> (chunk fastest, split)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmXh);
-      tma_prefetch_desc(&tmG);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int chunk = item % p.chunks, z = item / p.chunks;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmXh);
+    tma_prefetch_desc(&tmG);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int chunk = item % p.chunks, z = item / p.chunks;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+        if (elect_one()) {
           const int img = kb / p.s_blocks, s0 = (kb % p.s_blocks) * 64;
           const uint32_t sA = smem_base + stage * stage_bytes, sB = sA + a_bytes, sH = sB + KW * TILE;
           mbar_expect_tx(&raw_full[stage], (uint32_t)((p.kH + 1) * TILE + 2 * HALO));
@@ -717,27 +726,28 @@ conv_tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
           tma_load_4d(sB + PAD * TILE, &tmX, s0, chunk * 64, img, 0, &raw_full[stage]);
           tma_load_4d(sH, &tmXh, s0 - 8, chunk * 64, img, 0, &raw_full[stage]);
           tma_load_4d(sH + HALO, &tmXh, s0 + 64, chunk * 64, img, 0, &raw_full[stage]);
-          if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc_phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int z = item / p.chunks;
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        if (!mbar_wait(acc_empty, acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int z = item / p.chunks;
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      if (!mbar_wait_uniform(acc_empty, acc_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+      tc_fence_after();
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&raw_full[stage], phase, p.status, 0x80000u) || !mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&raw_full[stage], phase, p.status, 0x80000u) || !mbar_wait(&full[stage], phase, p.status, 0x80000u)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * stage_bytes, sB = sA + a_bytes;
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.desc_lbo;
+        const uint32_t sA = smem_base + stage * stage_bytes, sB = sA + a_bytes;
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.desc_lbo;
+        if (elect_one()) {
           for (int pi = 0; pi < p.pairs; ++pi) {
             const uint32_t a_lo32 = (((sA + pi * 2 * TILE) >> 4) & 0x3FFFu) | p.desc_lbo;
 #pragma unroll
@@ -748,11 +758,13 @@ conv_tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
             }
           }
           umma_commit(&empty[stage]);
-          if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(acc_full);
-        acc_phase ^= 1u;
+        __syncwarp();
+        if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(acc_full);
+      __syncwarp();
+      acc_phase ^= 1u;
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;   // lane quarter; which half of the BN columns

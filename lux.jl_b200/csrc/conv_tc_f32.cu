@@ -208,15 +208,15 @@ conv_tc_f32_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_co
 
   // tile -> (m tile fastest, image, n tile)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmWh); tma_prefetch_desc(&tmWl);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int t = tile % tiles_per_n, n0 = (tile / tiles_per_n) * BN;
-        const int m0 = (t % p.tiles_m) * kF32BM, img = t / p.tiles_m;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmWh); tma_prefetch_desc(&tmWl);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      const int t = tile % tiles_per_n, n0 = (tile / tiles_per_n) * BN;
+      const int m0 = (t % p.tiles_m) * kF32BM, img = t / p.tiles_m;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
           const int c0 = m0 + p.a_shift[kb];
@@ -227,27 +227,29 @@ conv_tc_f32_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_co
           }
           tma_load_2d(sB, &tmWh, kb * 32, n0, &full[stage]);
           tma_load_2d(sB + Cfg::B_BYTES, &tmWl, kb * 32, n0, &full[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x2000u)) { ok = false; break; }
-          if (!mbar_wait(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+    uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x2000u)) { ok = false; break; }
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+        if (elect_one()) {
           issue_split_kblock(tmem_base + ch * Cfg::CHUNK_COLS, BN, sA, sA + Cfg::A_BYTES, sB, p.a_desc_hi, p.a_desc_lbo,
                              p.a_k_advance, p.b_desc_hi, p.b_desc_lbo, p.b_k_advance, p.idesc_wide, p.idesc);
           umma_commit(&empty[stage]);
           umma_commit(&chunk_full[ch]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          if (++ch == Cfg::CHUNKS) { ch = 0; ch_phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        if (++ch == Cfg::CHUNKS) { ch = 0; ch_phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
@@ -369,17 +371,17 @@ conv_tc_f32_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_
 
   // item -> (m tile fastest, n tile, split)
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmGh); tma_prefetch_desc(&tmGl);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / (p.m_tiles * p.tiles_n);
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        const int rg0 = 2 * mt, rg1 = 2 * mt + 1;
-        const bool two = rg1 < p.n_rg;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmGh); tma_prefetch_desc(&tmGl);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / (p.m_tiles * p.tiles_n);
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      const int rg0 = 2 * mt, rg1 = 2 * mt + 1;
+      const bool two = rg1 < p.n_rg;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x20000u)) { ok = false; break; }
+        if (elect_one()) {
           const int img = kb / p.s_blocks, s0 = (kb % p.s_blocks) * 32;
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
           mbar_expect_tx(&full[stage], (uint32_t)(2 * (Cfg::B_BYTES + (two ? Cfg::A_BYTES : Cfg::A_BYTES / 2))));
@@ -391,29 +393,31 @@ conv_tc_f32_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_
           }
           tma_load_4d(sB, &tmGh, s0, nt * BN, img, 0, &full[stage]);
           tma_load_4d(sB + Cfg::B_BYTES, &tmGl, s0, nt * BN, img, 0, &full[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const int z = item / (p.m_tiles * p.tiles_n);
-        const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
-          if (!mbar_wait(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+    uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      const int z = item / (p.m_tiles * p.tiles_n);
+      const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x40000u)) { ok = false; break; }
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+        if (elect_one()) {
           issue_split_kblock(tmem_base + ch * Cfg::CHUNK_COLS, BN, sA, sA + Cfg::A_BYTES, sB, p.desc_hi, p.desc_lbo, p.k_advance,
                              p.desc_hi, p.desc_lbo, p.k_advance, p.idesc_wide, p.idesc);
           umma_commit(&empty[stage]);
           umma_commit(&chunk_full[ch]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          if (++ch == Cfg::CHUNKS) { ch = 0; ch_phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        if (++ch == Cfg::CHUNKS) { ch = 0; ch_phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {

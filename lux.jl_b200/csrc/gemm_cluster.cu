@@ -189,10 +189,10 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == kClWorkers + 1) {
     if constexpr (!F32) {
-      if (lane == 0) {
-        uint32_t stage = 0, phase = 0;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1u)) break;
+      uint32_t stage = 0, phase = 0;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1u)) break;
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES;
           const int k0 = kb * 64;
@@ -200,8 +200,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             tma_load_2d(sA + bx * p.a.box_bytes, &tmA, p.a.mn_major ? m0 + bx * p.a.mn_step : k0, p.a.mn_major ? k0 : m0, &full[stage]);
           for (int bx = 0; bx < p.b.boxes; ++bx)
             tma_load_2d(sB + bx * p.b.box_bytes, &tmB, p.b.mn_major ? n0 + bx * p.b.mn_step : k0, p.b.mn_major ? k0 : n0, &full[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == kClWorkers) {

@@ -131,18 +131,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
-      if constexpr (SPLIT3) { tma_prefetch_desc(&tmA_lo); tma_prefetch_desc(&tmB_lo); }
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int tm, tn;
-        tile_coords(p, tile, &tm, &tn);
-        const int m0 = tm * kBM, n0 = tn * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x1u)) { ok = false; break; }
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    if constexpr (SPLIT3) { tma_prefetch_desc(&tmA_lo); tma_prefetch_desc(&tmB_lo); }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      int tm, tn;
+      tile_coords(p, tile, &tm, &tn);
+      const int m0 = tm * kBM, n0 = tn * BN;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
           const uint32_t sB = sA + Cfg::A_BYTES;
@@ -159,27 +159,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tma_load_2d(sB + bx * p.b.box_bytes, &tmB, c0, c1, &full[stage]);
             if constexpr (SPLIT3) tma_load_2d(sB + Cfg::A_BYTES + Cfg::B_BYTES + bx * p.b.box_bytes, &tmB_lo, c0, c1, &full[stage]);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2u)) { ok = false; break; }
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x2u)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x4u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
-          const uint32_t sB = sA + Cfg::A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a.desc_lbo;
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b.desc_lbo;
-          constexpr uint32_t LO_OFF = (Cfg::A_BYTES + Cfg::B_BYTES) >> 4;
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
+        const uint32_t sB = sA + Cfg::A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a.desc_lbo;
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b.desc_lbo;
+        constexpr uint32_t LO_OFF = (Cfg::A_BYTES + Cfg::B_BYTES) >> 4;
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < kKSteps; ++ks) {
             const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(a_lo32 + ks * p.a.k_advance);
@@ -191,11 +192,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
           }
           umma_commit(&empty[stage]);  // frees the smem stage once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
@@ -313,16 +316,16 @@ gemm_tc_f32acc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmA_lo); tma_prefetch_desc(&tmB_lo);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int tm, tn;
-        tile_coords(p, tile, &tm, &tn);
-        const int m0 = tm * kBM, n0 = tn * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x100u)) { ok = false; break; }
+    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmA_lo); tma_prefetch_desc(&tmB_lo);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      int tm, tn;
+      tile_coords(p, tile, &tm, &tn);
+      const int m0 = tm * kBM, n0 = tn * BN;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x100u)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
           const uint32_t sB = sA + Cfg::A_BYTES;
@@ -340,25 +343,26 @@ gemm_tc_f32acc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             tma_load_2d(sB + bx * p.b.box_bytes, &tmB, c0, c1, &full[stage]);
             tma_load_2d(sB + LO + bx * p.b.box_bytes, &tmB_lo, c0, c1, &full[stage]);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x200u)) { ok = false; break; }
-          if (!mbar_wait(&full[stage], phase, p.status, 0x400u)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d_tmem = tmem_base + ch * BN;
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
-          const uint32_t sB = sA + Cfg::A_BYTES;
-          const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a.desc_lbo;
-          const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b.desc_lbo;
-          constexpr uint32_t LO_OFF = (Cfg::A_BYTES + Cfg::B_BYTES) >> 4;
+    uint32_t stage = 0, phase = 0, ch = 0, ch_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&chunk_empty[ch], ch_phase ^ 1u, p.status, 0x200u)) { ok = false; break; }
+        if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x400u)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + ch * BN;
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
+        const uint32_t sB = sA + Cfg::A_BYTES;
+        const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a.desc_lbo;
+        const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b.desc_lbo;
+        constexpr uint32_t LO_OFF = (Cfg::A_BYTES + Cfg::B_BYTES) >> 4;
+        if (elect_one()) {
           // small terms first, so the large hi*hi products are added last
 #pragma unroll
           for (int ks = 0; ks < kKSteps; ++ks) {
@@ -375,9 +379,10 @@ gemm_tc_f32acc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           }
           umma_commit(&empty[stage]);
           umma_commit(&chunk_full[ch]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          if (++ch == 2) { ch = 0; ch_phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        if (++ch == 2) { ch = 0; ch_phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
@@ -508,22 +513,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer (one per CTA) ----------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int slot = cluster_id; slot < p.total_slots && ok; slot += num_clusters) {
-        int tile, halved, which, tm, tn;
-        pair_slot(p, slot, &tile, &halved, &which);
-        tile_coords(p, tile, &tm, &tn);
-        const int bn_eff = halved ? BN / 2 : BN;                 // columns of this work item
-        const int b_boxes = halved ? p.b.boxes / 2 : p.b.boxes;  // B boxes this CTA loads per k-block
-        const int m0 = tm * (2 * kBM) + (int)rank * kBM;
-        const int n0 = tn * BN + which * (BN / 2) + (int)rank * (bn_eff / 2);
-        const uint32_t stage_tx = 2u * (uint32_t)(Cfg::A_BYTES + b_boxes * p.b.box_bytes);
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, p.status, 0x10u)) { ok = false; break; }
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int slot = cluster_id; slot < p.total_slots && ok; slot += num_clusters) {
+      int tile, halved, which, tm, tn;
+      pair_slot(p, slot, &tile, &halved, &which);
+      tile_coords(p, tile, &tm, &tn);
+      const int bn_eff = halved ? BN / 2 : BN;                 // columns of this work item
+      const int b_boxes = halved ? p.b.boxes / 2 : p.b.boxes;  // B boxes this CTA loads per k-block
+      const int m0 = tm * (2 * kBM) + (int)rank * kBM;
+      const int n0 = tn * BN + which * (BN / 2) + (int)rank * (bn_eff / 2);
+      const uint32_t stage_tx = 2u * (uint32_t)(Cfg::A_BYTES + b_boxes * p.b.box_bytes);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x10u)) { ok = false; break; }
+        if (elect_one()) {
           const uint32_t leader_full = map_to_cta(smem_u32(&full[stage]), 0);
           // The partner's bytes may be counted before this arrive (the transaction count then goes negative for
           // a moment); the phase cannot complete before it, because it is the barrier's only pending arrival.
@@ -541,37 +546,42 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int32_t c1 = p.b.mn_major ? k0 : n0;
             tma_load_2d_pair(sB + bx * p.b.box_bytes, &tmB, c0, c1, leader_full);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       bool ok = true;
       for (int slot = cluster_id; slot < p.total_slots && ok; slot += num_clusters) {
         const uint32_t idesc = slot < p.full_slots ? p.idesc : p.idesc_half;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x20u)) { ok = false; break; }
+        if (!mbar_wait_uniform(&acc_empty[acc], acc_phase ^ 1u, p.status, 0x20u)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, 0x40u)) { ok = false; break; }
+          if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x40u)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
           const uint32_t sB = sA + Cfg::A_BYTES;
           const uint32_t a_lo32 = ((sA >> 4) & 0x3FFFu) | p.a.desc_lbo;
           const uint32_t b_lo32 = ((sB >> 4) & 0x3FFFu) | p.b.desc_lbo;
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < kKSteps; ++ks) {
-            const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(a_lo32 + ks * p.a.k_advance);
-            const uint64_t bd = ((uint64_t)p.b.desc_hi << 32) | (uint64_t)(b_lo32 + ks * p.b.k_advance);
-            umma_pair<TF32>(d_tmem, ad, bd, idesc, (kb | ks) != 0 ? 1u : 0u);
+            for (int ks = 0; ks < kKSteps; ++ks) {
+              const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(a_lo32 + ks * p.a.k_advance);
+              const uint64_t bd = ((uint64_t)p.b.desc_hi << 32) | (uint64_t)(b_lo32 + ks * p.b.k_advance);
+              umma_pair<TF32>(d_tmem, ad, bd, idesc, (kb | ks) != 0 ? 1u : 0u);
+            }
+            umma_commit_pair_both(smem_u32(&empty[stage]));   // frees this stage in both CTAs
           }
-          umma_commit_pair_both(smem_u32(&empty[stage]));   // frees this stage in both CTAs
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit_pair_both(smem_u32(&acc_full[acc]));
+        if (ok && elect_one()) umma_commit_pair_both(smem_u32(&acc_full[acc]));
+        __syncwarp();
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
     }
