@@ -50,9 +50,12 @@ int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const 
 int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws,
                      cudaStream_t st, bool x_is_copy = false);
 
-// Box of at most `most` positions (BW columns x BH rows x BI images) that covers an OW x OH x NI grid in the fewest boxes;
-// among equals the widest (contiguous stores). Rows are cut into equal pieces of at least 8 columns.
-inline void conv_position_box(int OW, int OH, int NI, int most, int* BW, int* BH, int* BI) {
+// Box of at most `most` positions (BW columns x BH rows x BI images) for an OW x OH x NI grid, rows cut into equal pieces of at
+// least 8 columns: the one whose boxes, `per_box` tiles each, take the fewest waves of `wave` tiles (wave = 1: the fewest
+// boxes); among equals the widest and tallest, whose stores are the longest runs. 14 x 14 maps in whole rows fill 98 of 128
+// positions, in 14 x 1 x 9 boxes 126 (3x3 256 -> 256, batch 256, bf16: forward 91 -> 79 us); on 7 x 7 both take two waves and
+// the whole planes are 4 % faster.
+inline void conv_position_box(int OW, int OH, int NI, int most, int64_t per_box, int64_t wave, int* BW, int* BH, int* BI) {
   int64_t best = 0;
   for (int k = 1; k <= OW; ++k) {
     const int bw = (OW + k - 1) / k;
@@ -62,7 +65,8 @@ inline void conv_position_box(int OW, int OH, int NI, int most, int* BW, int* BH
     for (int bh = rows < OH ? rows : OH; bh >= 1; --bh) {
       const int bi = rows / bh < NI ? rows / bh : NI;
       const int64_t n = (int64_t)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((NI + bi - 1) / bi);
-      if (best == 0 || n < best) { best = n; *BW = bw; *BH = bh; *BI = bi; }
+      const int64_t waves = (n * per_box + wave - 1) / wave;
+      if (best == 0 || waves < best) { best = waves; *BW = bw; *BH = bh; *BI = bi; }
     }
   }
 }

@@ -702,7 +702,7 @@ struct CwfGrid {       // tiling of one launch of the forward kernel
 };
 CwfGrid cwf_grid(int OW, int OH, int NI, int n_out) {
   CwfGrid t{};
-  conv_position_box(OW, OH, NI, kFBM, &t.BW, &t.BH, &t.BI);
+  conv_position_box(OW, OH, NI, kFBM, 1, 1, &t.BW, &t.BH, &t.BI);
   t.tw = (OW + t.BW - 1) / t.BW; t.th = (OH + t.BH - 1) / t.BH; t.ti = (NI + t.BI - 1) / t.BI;
   t.tn = (n_out + cwf_bn(n_out) - 1) / cwf_bn(n_out);
   return t;
