@@ -3,6 +3,7 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -49,8 +50,13 @@ int sm_count() {
 __device__ unsigned int g_device_status = 0;
 
 unsigned int* device_status_word() {
-  unsigned int* p = nullptr;
+  static std::atomic<unsigned int*> known[64];   // per device; the module's variable does not move
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  unsigned int* p = known[dev].load(std::memory_order_relaxed);
+  if (p != nullptr) return p;
   if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_device_status) != cudaSuccess) return nullptr;
+  known[dev].store(p, std::memory_order_relaxed);
   return p;
 }
 

@@ -688,7 +688,7 @@ int cwf_splits(int64_t items, int kb, int64_t numel, int most) {
   const int sms = sm_count();
   double best = 0;
   int pick = 1;
-  for (int s = 1; s <= most && s <= kb; ++s) {
+  for (int s = 1; s <= most && s <= kb; s += 1 + s / 16) {
     const double waves = (double)((items * s + sms - 1) / sms);
     const double cost = waves * ((kb + s - 1) / s + 6) + (s > 1 ? 6.0 + (double)s * numel * 8.0 / 2.4e6 : 0.0);
     if (s == 1 || cost < best * 0.97) { best = cost; pick = s; }
@@ -810,6 +810,17 @@ int32_t cwf_finish(const CwfOut& o, int64_t numel, int channels, cudaStream_t st
   return LB2_OK;
 }
 
+// 32 positions per k-block in power-of-two boxes; of those the one that covers the output in the fewest blocks, among equals
+// the widest
+void cwf_wg_box(const ConvGeom& g, int* KW, int* KH, int* KI) {
+  int64_t best = 0;
+  for (int kw = 1; kw <= 32; kw *= 2)
+    for (int kh = 1; kh * kw <= 32; kh *= 2) {
+      const int ki = 32 / (kw * kh);
+      const int64_t n = (int64_t)((g.out[0] + kw - 1) / kw) * ((g.out[1] + kh - 1) / kh) * ((g.batch + ki - 1) / ki);
+      if (best == 0 || n <= best) { best = n; *KW = kw; *KH = kh; *KI = ki; }
+    }
+}
 struct CwfWgPlan {
   int chunks, n_pairs, m_tiles, tiles_n, n_pad, KW_, KH_, KI_, kbw, kbh, kb_total, splits, kb_per_split;
   size_t partial_bytes;
@@ -822,16 +833,9 @@ CwfWgPlan cwf_wg_plan(const ConvGeom& g) {
   const int bn = cwf_bn(g.cout);
   w.tiles_n = (g.cout + bn - 1) / bn;
   w.n_pad = w.tiles_n * bn;
-  // 32 positions per k-block in power-of-two boxes; of those the one that covers the output in the fewest blocks
-  int64_t best = 0;
-  for (int kw = 1; kw <= 32; kw *= 2)
-    for (int kh = 1; kh * kw <= 32; kh *= 2) {
-      const int ki = 32 / (kw * kh);
-      const int64_t n = (int64_t)((g.out[0] + kw - 1) / kw) * ((g.out[1] + kh - 1) / kh) * ((g.batch + ki - 1) / ki);
-      if (best == 0 || n <= best) { best = n; w.KW_ = kw; w.KH_ = kh; w.KI_ = ki; }
-    }
+  cwf_wg_box(g, &w.KW_, &w.KH_, &w.KI_);
   w.kbw = (g.out[0] + w.KW_ - 1) / w.KW_; w.kbh = (g.out[1] + w.KH_ - 1) / w.KH_;
-  w.kb_total = (int)best;
+  w.kb_total = w.kbw * w.kbh * ((g.batch + w.KI_ - 1) / w.KI_);
   const int64_t items = (int64_t)w.m_tiles * w.tiles_n;
   const int splits = cwf_splits(items, w.kb_total, items * 128 * bn, 2 * sm_count());
   w.kb_per_split = (w.kb_total + splits - 1) / splits;
@@ -852,8 +856,6 @@ bool conv_cwf_supported(const ConvGeom& g) {
   if (x_numel(g) >= ((int64_t)1 << 40)) return false;
   const CwfGrid t = cwf_grid(g.out[0], g.out[1], g.batch, g.cout);
   if (t.BW * g.stride[0] > 256 || t.BH * g.stride[1] > 256) return false;
-  const CwfWgPlan wg = cwf_wg_plan(g);
-  if (wg.KW_ * g.stride[0] > 256 || wg.KH_ * g.stride[1] > 256) return false;
   return tensor_map_encoder() != nullptr;
 }
 

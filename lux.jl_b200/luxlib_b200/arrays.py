@@ -17,14 +17,14 @@ def colmajor_strides(shape: Sequence[int]):
     st, acc = [], 1
     for d in shape:
         st.append(acc)
-        acc *= max(int(d), 1)
+        if d > 1:
+            acc *= int(d)
     return tuple(st)
 
 
 def jl_empty(shape: Sequence[int], dtype: torch.dtype, device) -> torch.Tensor:
     """similar(x, T, shape...): uninitialised column-major array."""
-    shape = tuple(int(d) for d in shape)
-    return torch.empty_strided(shape, colmajor_strides(shape), dtype=dtype, device=device)
+    return torch.empty_strided(tuple(shape), colmajor_strides(shape), dtype=dtype, device=device)
 
 
 def jl_zeros(shape, dtype, device) -> torch.Tensor:
@@ -34,9 +34,9 @@ def jl_zeros(shape, dtype, device) -> torch.Tensor:
 
 
 def is_colmajor(t: torch.Tensor) -> bool:
-    if t.numel() == 0:
-        return True
     exp = colmajor_strides(t.shape)
+    if t.stride() == exp or t.numel() == 0:
+        return True
     return all(s == e or d == 1 for s, e, d in zip(t.stride(), exp, t.shape))
 
 
@@ -88,7 +88,13 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+# the stream's handle without a torch.cuda.Stream object around it (2 us per call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def current_stream(device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -97,4 +103,4 @@ def workspace(nbytes: int, device) -> torch.Tensor | None:
     torch allocator."""
     if nbytes <= 0:
         return None
-    return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)

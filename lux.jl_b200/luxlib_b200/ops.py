@@ -11,6 +11,7 @@ Arrays are column-major device arrays (see arrays.py); activations are named by 
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import warnings
 from dataclasses import dataclass
@@ -58,8 +59,10 @@ _warned_mixed = False
 def _promote(*ts):
     """Mixed element types are promoted with a one-time warning (lib/LuxLib/ext/CUDAExt/cublaslt.jl:46-64)."""
     global _warned_mixed
+    dt = ts[0].dtype
+    if all(t is None or t.dtype == dt for t in ts):
+        return ts
     present = [t for t in ts if t is not None]
-    dt = present[0].dtype
     for t in present[1:]:
         dt = torch.promote_types(dt, t.dtype)
     if any(t.dtype != dt for t in present):
@@ -90,6 +93,21 @@ def _ws(nbytes: int, device):
     return w, ptr(w), int(nbytes) if w is not None else 0
 
 
+@functools.lru_cache(maxsize=4096)
+def _query(name: str, device_index, *args):
+    """A pure query of the library (workspace sizes and the like): it depends on the extents and on the device's kind only,
+    so it is asked once per set of arguments."""
+    return getattr(_cabi.load(), name)(*args)
+
+
+def _cast(v, dtype):
+    return v if v is None or v.dtype == dtype else v.to(dtype)
+
+
+def _cotangent(delta, dtype):
+    return as_colmajor(delta if delta.dtype == dtype else delta.to(dtype))
+
+
 # --------------------------------------------------------------------------------------------
 # dense
 # --------------------------------------------------------------------------------------------
@@ -112,7 +130,7 @@ def _dense_fwd(act: str, weight, x, b, want_preact: bool, flags: int = 0):
     dt = dtype_code(W.dtype)
     y = jl_empty((M, N), W.dtype, W.device)
     pre = jl_empty((M, N), W.dtype, W.device) if want_preact else None
-    _, wsp, wsn = _ws(lib.lb2_dense_fwd_workspace_bytes(M, N, K, dt, flags), W.device)
+    _, wsp, wsn = _ws(_query("lb2_dense_fwd_workspace_bytes", W.device.index, M, N, K, dt, flags), W.device)
     _cabi.check(lib.lb2_dense_fwd(ptr(y), ptr(pre), ptr(W), ptr(X), ptr(b), M, N, K, ldw, ldx, max(M, 1), dt,
                                   act_code(act), flags, wsp, wsn, current_stream(W.device)))
     if vec_in:
@@ -146,11 +164,11 @@ def rrule_fused_dense(act: str, weight, x, b=None, *, flags: int = 0):
         hooks). `shadows = (dW, dx, db)` switches to the accumulate contract of the Enzyme rules: the gradients are
         added to those arrays in place and Δ is zeroed."""
         if on_param_grads is not None:
-            d = as_colmajor(delta.reshape(M, N).to(W.dtype))
+            d = _cotangent(delta.reshape(M, N), W.dtype)
             g = jl_empty((M, N), W.dtype, W.device)
             db = jl_empty((M,), W.dtype, W.device) if bb is not None else None
             y2, pre2 = y.reshape(M, N), (None if pre is None else pre.reshape(M, N))
-            _, wsp, wsn = _ws(lib.lb2_bias_act_bwd_workspace_bytes(1, M, N), W.device)
+            _, wsp, wsn = _ws(_query("lb2_bias_act_bwd_workspace_bytes", W.device.index, 1, M, N), W.device)
             _cabi.check(lib.lb2_bias_act_bwd(ptr(g), ptr(db), ptr(d), None if keep_pre else ptr(y2), ptr(pre2), 1, M, N, dt,
                                              code, wsp, wsn, current_stream(W.device)))
             if mark is not None:
@@ -168,7 +186,7 @@ def rrule_fused_dense(act: str, weight, x, b=None, *, flags: int = 0):
             if mark is not None:
                 mark()
             return dW, (dx.reshape(x.shape) if x.dim() == 1 else dx), db
-        d = as_colmajor(delta.reshape(M, N).to(W.dtype))
+        d = _cotangent(delta.reshape(M, N), W.dtype)
         if shadows is not None:
             # Enzyme's reverse pass (lib/LuxLib/src/impl/dense.jl:253-283): the gradients are ADDED to the caller's
             # shadow arrays (mul!(dW, g, x', true, true); db .+= ...) and the output shadow is zeroed afterwards.
@@ -182,7 +200,7 @@ def rrule_fused_dense(act: str, weight, x, b=None, *, flags: int = 0):
             dx = dx2 = jl_empty((K, N), W.dtype, W.device)
             db = jl_empty((M,), W.dtype, W.device) if bb is not None else None
         y2, pre2 = y.reshape(M, N), (None if pre is None else pre.reshape(M, N))
-        _, wsp, wsn = _ws(lib.lb2_dense_bwd_workspace_bytes(M, N, K, dt, code, flags), W.device)
+        _, wsp, wsn = _ws(_query("lb2_dense_bwd_workspace_bytes", W.device.index, M, N, K, dt, code, flags), W.device)
         _cabi.check(lib.lb2_dense_bwd(ptr(dW), ptr(dx2), ptr(db), ptr(d), None if keep_pre else ptr(y2), ptr(pre2),
                                       ptr(W), ptr(X), M, N, K, ldw, ldx, max(M, 1), dt, code, int(shadows is not None),
                                       flags, wsp, wsn, current_stream(W.device)))
@@ -218,7 +236,7 @@ def matmul(A, B, *, transA=False, transB=False, flags: int = 0, out=None, accumu
         Cm, ldc = _matrix_ld(out)
         if Cm is not out:
             raise ArgumentError("out must be column-major with a contiguous first index")
-    _, wsp, wsn = _ws(lib.lb2_matmul_workspace_bytes(M, N, K, dt, flags), A2.device)
+    _, wsp, wsn = _ws(_query("lb2_matmul_workspace_bytes", A2.device.index, M, N, K, dt, flags), A2.device)
     _cabi.check(lib.lb2_matmul(ptr(Cm), ptr(A2), ptr(B2), M, N, K, lda, ldb, ldc, int(transA), int(transB), dt,
                                int(bool(accumulate)), flags, wsp, wsn, current_stream(A2.device)))
     return Cm
@@ -268,10 +286,10 @@ def rrule_bias_activation(act: str, x, bias=None):
     y = bias_activation(act, X, bias)
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         dx = jl_empty(X.shape, X.dtype, X.device)
         db = jl_empty((Cc,), X.dtype, X.device) if bias is not None else None
-        _, wsp, wsn = _ws(lib.lb2_bias_act_bwd_workspace_bytes(S, Cc, B), X.device)
+        _, wsp, wsn = _ws(_query("lb2_bias_act_bwd_workspace_bytes", X.device.index, S, Cc, B), X.device)
         _cabi.check(lib.lb2_bias_act_bwd(ptr(dx), ptr(db), ptr(d), None if keep_pre else ptr(y), ptr(pre), S, Cc, B,
                                          dtype_code(X.dtype), code, wsp, wsn, current_stream(X.device)))
         return dx, db
@@ -298,11 +316,11 @@ def rrule_scale(act: str, weight, x, bias=None):
     _cabi.check(lib.lb2_scale_fwd(ptr(y), ptr(X), ptr(Wt), ptr(Bs), D, B, dt, code, current_stream(X.device)))
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         dx = jl_empty(X.shape, X.dtype, X.device)
         dw = jl_empty(Wt.shape, X.dtype, X.device)
         db = jl_empty(Wt.shape, X.dtype, X.device) if Bs is not None else None
-        _, wsp, wsn = _ws(lib.lb2_scale_bwd_workspace_bytes(D, B), X.device)
+        _, wsp, wsn = _ws(_query("lb2_scale_bwd_workspace_bytes", X.device.index, D, B), X.device)
         _cabi.check(lib.lb2_scale_bwd(ptr(dx), ptr(dw), ptr(db), ptr(d), ptr(X), ptr(Wt), ptr(Bs), D, B, dt, code, wsp, wsn,
                                       current_stream(X.device)))
         return dw, dx, db
@@ -346,7 +364,7 @@ def rrule_add_activation(act: str, x, y):
     z = _add_act(code, X, Y)
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         if code == _cabi.ACT_IDENTITY:
             return d, d
         g = jl_empty(X.shape, X.dtype, X.device)
@@ -383,7 +401,14 @@ class ConvDims:
 
 def _conv_desc_from(wshape, spatial, cin: int, batch: int, cd: ConvDims) -> _cabi.ConvDesc:
     """lb2_conv_desc of the convolution that maps an input of spatial extents `spatial` with `cin` channels through a
-    filter of shape `wshape` = (k..., cin / groups, cout)."""
+    filter of shape `wshape` = (k..., cin / groups, cout). Equal geometries share one descriptor, which nobody writes to."""
+    return _conv_desc_of(tuple(wshape), tuple(spatial), cin, batch, tuple(cd.stride), tuple(cd.padding), tuple(cd.dilation), cd.groups,
+                         bool(cd.flipkernel))
+
+
+@functools.lru_cache(maxsize=1024)
+def _conv_desc_of(wshape, spatial, cin, batch, stride, padding, dilation, groups, flipkernel) -> _cabi.ConvDesc:
+    cd = ConvDims(stride, padding, dilation, groups, flipkernel)
     nd = len(spatial)
     if len(wshape) != nd + 2 or nd < 1 or nd > 3:
         raise DimensionMismatch("weight and x must have the same rank (3 to 5)")
@@ -406,6 +431,32 @@ def _conv_desc_from(wshape, spatial, cin: int, batch: int, cd: ConvDims) -> _cab
     return d
 
 
+class _ConvQuery:
+    """What the library answers about a geometry and element type on a device, asked once each (see `_query`)."""
+
+    def __init__(self, d, dt):
+        self.d, self.dt = d, dt
+        lib, ref = _cabi.load(), C.byref(d)
+        osz = (C.c_int32 * 3)()
+        _cabi.check(lib.lb2_conv_output_size(ref, osz))
+        self.yshape = tuple(osz[i] for i in range(d.ndim)) + (d.cout, d.batch)
+        self.fwd_bytes = lib.lb2_conv_fwd_workspace_bytes(ref, dt)
+        self.leaves_x_copy = lib.lb2_conv_fwd_leaves_x_copy(ref, dt) == 1
+        self.sums_fused = lib.lb2_conv_fwd_sums_is_fused(ref, dt) == 1
+        self.bwd_bytes = functools.lru_cache(maxsize=8)(lambda code: lib.lb2_conv_bwd_workspace_bytes(ref, dt, code))
+
+
+@functools.lru_cache(maxsize=1024)
+def _conv_query_of(device_index, dt, wshape, spatial, cin, batch, stride, padding, dilation, groups, flipkernel):
+    return _ConvQuery(_conv_desc_of(wshape, spatial, cin, batch, stride, padding, dilation, groups, flipkernel), dt)
+
+
+def _conv_query(weight, x, cd: ConvDims, dt: int) -> _ConvQuery:
+    xs = tuple(x.shape)
+    return _conv_query_of(x.device.index, dt, tuple(weight.shape), xs[:-2], xs[-2], xs[-1], tuple(cd.stride), tuple(cd.padding),
+                          tuple(cd.dilation), cd.groups, bool(cd.flipkernel))
+
+
 def _conv_desc(weight, x, cd: ConvDims) -> _cabi.ConvDesc:
     if weight.dim() != x.dim():
         raise DimensionMismatch("weight and x must have the same rank (3 to 5)")
@@ -419,20 +470,18 @@ def _conv_fwd(act, weight, x, b, cd, want_preact, flags=0, want_ws=False):
     if b is not None and b.shape[0] != d.cout:
         raise DimensionMismatch("length(bias) must equal the number of output channels")
     Wt, X = as_colmajor(weight), as_colmajor(x)
-    osz = (C.c_int32 * 3)()
-    _cabi.check(lib.lb2_conv_output_size(C.byref(d), osz))
-    yshape = tuple(osz[i] for i in range(d.ndim)) + (d.cout, d.batch)
-    y = jl_empty(yshape, X.dtype, X.device)
-    pre = jl_empty(yshape, X.dtype, X.device) if want_preact else None
     dt = dtype_code(X.dtype)
-    ws, wsp, wsn = _ws(lib.lb2_conv_fwd_workspace_bytes(C.byref(d), dt), X.device)
+    info = _conv_query(Wt, X, cd, dt)
+    y = jl_empty(info.yshape, X.dtype, X.device)
+    pre = jl_empty(info.yshape, X.dtype, X.device) if want_preact else None
+    ws, wsp, wsn = _ws(info.fwd_bytes, X.device)
     _cabi.check(lib.lb2_conv_fwd(ptr(y), ptr(pre), ptr(X), ptr(Wt), ptr(b), C.byref(d), dt, act_code(act), flags, wsp, wsn,
                                  current_stream(X.device)))
     # the general tensor-core path leaves its channel-innermost copy of x at the start of the workspace; a pullback
     # that keeps the workspace alive hands it back instead of having the copy made again
     keep = ws if (want_ws and ws is not None and not (flags & _cabi.FLAG_FORCE_SIMT) and X.data_ptr() % 16 == 0 and
-                  lib.lb2_conv_fwd_leaves_x_copy(C.byref(d), dt) == 1) else None
-    return y, pre, (Wt, X, b, d, dt, keep)
+                  info.leaves_x_copy) else None
+    return y, pre, (Wt, X, b, info, dt, keep)
 
 
 def fused_conv_bias_activation(act: str, weight, x, b, cdims: ConvDims, *, flags: int = 0):
@@ -445,16 +494,16 @@ def rrule_fused_conv(act: str, weight, x, b, cdims: ConvDims, *, flags: int = 0)
     Pullback Δ -> (∂weight, ∂x, ∂b)."""
     lib = _cabi.load()
     keep_pre = needs_preactivation(act)
-    y, pre, (Wt, X, bb, d, dt, xcopy) = _conv_fwd(act, weight, x, b, cdims, keep_pre, flags, want_ws=True)
-    code = act_code(act)
+    y, pre, (Wt, X, bb, info, dt, xcopy) = _conv_fwd(act, weight, x, b, cdims, keep_pre, flags, want_ws=True)
+    d, code = info.d, act_code(act)
 
     def pullback(delta, need_dx=True):
         """Δ -> (∂weight, ∂x, ∂b); `need_dx=False` (a network's first layer) skips the data gradient and returns None for it."""
-        dl = as_colmajor(delta.to(X.dtype))  # NNlib.colmajor(Δ): impl/conv.jl:263
+        dl = _cotangent(delta, X.dtype)  # NNlib.colmajor(Δ): impl/conv.jl:263
         dw = jl_empty(Wt.shape, X.dtype, X.device)
         dx = jl_empty(X.shape, X.dtype, X.device) if need_dx else None
         db = jl_empty((d.cout,), X.dtype, X.device) if bb is not None else None
-        _, wsp, wsn = _ws(lib.lb2_conv_bwd_workspace_bytes(C.byref(d), dt, code), X.device)
+        _, wsp, wsn = _ws(info.bwd_bytes(code), X.device)
         xarg, xflag = (ptr(xcopy), _cabi.FLAG_X_COPY_GIVEN) if xcopy is not None else (ptr(X), 0)
         _cabi.check(lib.lb2_conv_bwd(ptr(dw), ptr(dx), ptr(db), ptr(dl), None if keep_pre else ptr(y), ptr(pre), xarg,
                                      ptr(Wt), C.byref(d), dt, code, flags | xflag, wsp, wsn, current_stream(X.device)))
@@ -527,7 +576,7 @@ def conv_transpose_bias_activation(act: str, weight, x, b, cdims: ConvDims, outp
 # --------------------------------------------------------------------------------------------
 def _bmm(lib, Cp, Ap, Bp, M, N, K, batch, lda, ldb, ldc, sa, sb, sc, ta, tb, dt, device, accumulate=0, flags=0):
     """One lb2_batched_matmul call on raw pointers (integers)."""
-    _, wsp, wsn = _ws(lib.lb2_batched_matmul_workspace_bytes(M, N, K, dt, flags), device)
+    _, wsp, wsn = _ws(_query("lb2_batched_matmul_workspace_bytes", device.index, M, N, K, dt, flags), device)
     _cabi.check(lib.lb2_batched_matmul(Cp, Ap, Bp, M, N, K, batch, lda, ldb, ldc, sa, sb, sc, int(ta), int(tb), dt, accumulate, flags,
                                        wsp, wsn, current_stream(device)))
 
@@ -716,7 +765,7 @@ def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_cau
             # a bias shared by all heads and samples: its gradient is the sum over them — the bias-gradient reduction on
             # the (1, S*L, H*B) view
             full, db = db, jl_empty((S, Lq), Q.dtype, device)
-            _, wsp, wsn = _ws(lib.lb2_bias_act_bwd_workspace_bytes(1, S * Lq, H * Bn), device)
+            _, wsp, wsn = _ws(_query("lb2_bias_act_bwd_workspace_bytes", device.index, 1, S * Lq, H * Bn), device)
             _cabi.check(lib.lb2_bias_act_bwd(None, ptr(db), ptr(full), None, None, 1, S * Lq, H * Bn, dt, act_code("identity"), wsp, wsn,
                                              current_stream(device)))
         return dq, dk, dv, db
@@ -771,7 +820,7 @@ def _batchnorm_fwd(x, scale, bias, rmean, rvar, training, act, momentum, epsilon
     dev = X.device
     y = jl_empty(X.shape, X.dtype, dev)
     code = act_code(act)
-    cast = lambda v: None if v is None else v.to(X.dtype)
+    cast = lambda v: _cast(v, X.dtype)
     scale_c, bias_c, rmean_c, rvar_c = cast(scale), cast(bias), cast(rmean), cast(rvar)
     if training or rmean is None:
         save_mean = torch.empty(Cc, dtype=torch.float32, device=dev)
@@ -779,7 +828,7 @@ def _batchnorm_fwd(x, scale, bias, rmean, rvar, training, act, momentum, epsilon
         update = training and rmean is not None
         new_rm = torch.empty_like(rmean_c) if update else None
         new_rv = torch.empty_like(rvar_c) if update else None
-        _, wsp, wsn = _ws(lib.lb2_batchnorm_workspace_bytes(S, Cc, B), dev)
+        _, wsp, wsn = _ws(_query("lb2_batchnorm_workspace_bytes", dev.index, S, Cc, B), dev)
         _cabi.check(lib.lb2_batchnorm_fwd_train(ptr(y), ptr(save_mean), ptr(save_inv), ptr(new_rm), ptr(new_rv), ptr(X),
                                                 ptr(scale_c), ptr(bias_c), ptr(rmean_c) if update else None,
                                                 ptr(rvar_c) if update else None, S, Cc, B, float(momentum), eps, dt,
@@ -803,11 +852,11 @@ def rrule_batchnorm(x, scale, bias, running_mean, running_var, training: bool, a
         x, scale, bias, running_mean, running_var, training, act, momentum, epsilon)
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         dx = jl_empty(X.shape, X.dtype, X.device)
         dg = torch.empty(Cc, dtype=X.dtype, device=X.device) if sc is not None else None
         db = torch.empty(Cc, dtype=X.dtype, device=X.device) if sc is not None else None
-        _, wsp, wsn = _ws(lib.lb2_batchnorm_workspace_bytes(S, Cc, B), X.device)
+        _, wsp, wsn = _ws(_query("lb2_batchnorm_workspace_bytes", X.device.index, S, Cc, B), X.device)
         if batch_stats:
             _cabi.check(lib.lb2_batchnorm_bwd(ptr(dx), ptr(dg), ptr(db), ptr(d), ptr(X), ptr(sc), ptr(bi), ptr(save_mean),
                                               ptr(save_inv), S, Cc, B, dt, code, wsp, wsn, current_stream(X.device)))
@@ -836,14 +885,13 @@ def rrule_conv_batchnorm(act: str, weight, x, cdims: ConvDims, scale, bias, runn
         raise ArgumentError("running_mean and running_var must both be given or both be nothing")
     d = _conv_desc(weight, x, cdims)
     Wt, X = as_colmajor(weight), as_colmajor(x)
-    osz = (C.c_int32 * 3)()
-    _cabi.check(lib.lb2_conv_output_size(C.byref(d), osz))
-    ushape = tuple(osz[i] for i in range(d.ndim)) + (d.cout, d.batch)
+    dt, dev = dtype_code(X.dtype), X.device
+    info = _conv_query(Wt, X, cdims, dt)
+    ushape = info.yshape
     for v, name in ((scale, "scale"), (bias, "bias"), (running_mean, "running_mean"), (running_var, "running_var")):
         if v is not None and v.shape[0] != d.cout:
             raise DimensionMismatch(f"length({name}) must equal the number of channels {d.cout}")
-    dt, dev = dtype_code(X.dtype), X.device
-    if (flags & _cabi.FLAG_FORCE_SIMT) or lib.lb2_conv_fwd_sums_is_fused(C.byref(d), dt) != 1:
+    if (flags & _cabi.FLAG_FORCE_SIMT) or not info.sums_fused:
         # short contractions and the paths without the epilogue sums: the plain pair is the faster form
         u, pb_conv = rrule_fused_conv("identity", weight, x, None, cdims, flags=flags)
         y, stats, pb_bn = rrule_batchnorm(u, scale, bias, running_mean, running_var, True, act, momentum, epsilon)
@@ -859,34 +907,34 @@ def rrule_conv_batchnorm(act: str, weight, x, cdims: ConvDims, scale, bias, runn
     ws, wsp, wsn = _ws(lib.lb2_conv_fwd_sums_workspace_bytes(C.byref(d), dt), dev)
     _cabi.check(lib.lb2_conv_fwd_sums(ptr(u), ptr(sums), ptr(X), ptr(Wt), C.byref(d), dt, flags, wsp, wsn, current_stream(dev)))
     xcopy = ws if (ws is not None and not (flags & _cabi.FLAG_FORCE_SIMT) and X.data_ptr() % 16 == 0 and
-                   lib.lb2_conv_fwd_leaves_x_copy(C.byref(d), dt) == 1) else None
+                   info.leaves_x_copy) else None
     S, Cc, B = _scb(u)
     eps = default_epsilon(X.dtype) if epsilon is None else float(epsilon)
     code = act_code(act)
-    cast = lambda v: None if v is None else v.to(X.dtype)
+    cast = lambda v: _cast(v, X.dtype)
     sc, bi, rm, rv = cast(scale), cast(bias), cast(running_mean), cast(running_var)
     y = jl_empty(ushape, X.dtype, dev)
     save_mean = torch.empty(Cc, dtype=torch.float32, device=dev)
     save_inv = torch.empty(Cc, dtype=torch.float32, device=dev)
     new_rm = torch.empty_like(rm) if rm is not None else None
     new_rv = torch.empty_like(rv) if rv is not None else None
-    _, w2, n2 = _ws(lib.lb2_batchnorm_workspace_bytes(S, Cc, B), dev)
+    _, w2, n2 = _ws(_query("lb2_batchnorm_workspace_bytes", dev.index, S, Cc, B), dev)
     _cabi.check(lib.lb2_batchnorm_fwd_train_sums(ptr(y), ptr(save_mean), ptr(save_inv), ptr(new_rm), ptr(new_rv), ptr(u), ptr(sc), ptr(bi),
                                                  ptr(rm), ptr(rv), ptr(sums), S, Cc, B, float(momentum), eps, dt, code, w2, n2,
                                                  current_stream(dev)))
     ident = act_code("identity")
 
     def pullback(delta, need_dx=True):
-        dl = as_colmajor(delta.to(X.dtype))
+        dl = _cotangent(delta, X.dtype)
         du = jl_empty(ushape, X.dtype, dev)
         dg = torch.empty(Cc, dtype=X.dtype, device=dev) if sc is not None else None
         db = torch.empty(Cc, dtype=X.dtype, device=dev) if sc is not None else None
-        _, w3, n3 = _ws(lib.lb2_batchnorm_workspace_bytes(S, Cc, B), dev)
+        _, w3, n3 = _ws(_query("lb2_batchnorm_workspace_bytes", dev.index, S, Cc, B), dev)
         _cabi.check(lib.lb2_batchnorm_bwd(ptr(du), ptr(dg), ptr(db), ptr(dl), ptr(u), ptr(sc), ptr(bi), ptr(save_mean), ptr(save_inv),
                                           S, Cc, B, dt, code, w3, n3, current_stream(dev)))
         dw = jl_empty(Wt.shape, X.dtype, dev)
         dx = jl_empty(X.shape, X.dtype, dev) if need_dx else None
-        _, w4, n4 = _ws(lib.lb2_conv_bwd_workspace_bytes(C.byref(d), dt, ident), dev)
+        _, w4, n4 = _ws(info.bwd_bytes(ident), dev)
         xarg, xflag = (ptr(xcopy), _cabi.FLAG_X_COPY_GIVEN) if xcopy is not None else (ptr(X), 0)
         _cabi.check(lib.lb2_conv_bwd(ptr(dw), ptr(dx), None, ptr(du), None, None, xarg, ptr(Wt), C.byref(d), dt, ident, flags | xflag,
                                      w4, n4, current_stream(dev)))
@@ -961,7 +1009,7 @@ def _pool(kind: int, x, pd: PoolDims):
     _cabi.check(lib.lb2_pool_fwd(ptr(y), ptr(X), C.byref(d), kind, dt, current_stream(X.device)))
 
     def pullback(delta):
-        dy = as_colmajor(delta.to(X.dtype))
+        dy = _cotangent(delta, X.dtype)
         if tuple(dy.shape) != tuple(y.shape):
             raise DimensionMismatch("the cotangent must have the shape of the pooled output")
         dx = jl_empty(X.shape, X.dtype, X.device)
@@ -1067,11 +1115,11 @@ def rrule_groupnorm(x, scale, bias, groups: int, act: str = "identity", epsilon:
     y, (X, sc, bi, sm, si, S, Cc, B, dt, code) = _groupnorm_fwd(x, scale, bias, groups, act, epsilon)
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         dx = jl_empty(X.shape, X.dtype, X.device)
         dg = torch.empty(Cc, dtype=X.dtype, device=X.device) if sc is not None else None
         db = torch.empty(Cc, dtype=X.dtype, device=X.device) if sc is not None else None
-        _, wsp, wsn = _ws(lib.lb2_groupnorm_bwd_workspace_bytes(S, Cc, groups, B), X.device)
+        _, wsp, wsn = _ws(_query("lb2_groupnorm_bwd_workspace_bytes", X.device.index, S, Cc, groups, B), X.device)
         _cabi.check(lib.lb2_groupnorm_bwd(ptr(dx), ptr(dg), ptr(db), ptr(d), ptr(X), ptr(sc), ptr(bi), ptr(sm), ptr(si), S,
                                           Cc, groups, B, dt, code, wsp, wsn, current_stream(X.device)))
         return dx, dg, db
@@ -1140,11 +1188,11 @@ def rrule_layernorm(x, scale=None, bias=None, act: str = "identity", dims=None, 
     y, (X, sc, bi, sm, si, D, R, dt, code) = _layernorm_fwd(x, scale, bias, act, dims, epsilon)
 
     def pullback(delta):
-        d = as_colmajor(delta.to(X.dtype))
+        d = _cotangent(delta, X.dtype)
         dx = jl_empty(X.shape, X.dtype, X.device)
         dg = jl_empty(sc.shape, X.dtype, X.device) if sc is not None else None
         db = jl_empty(sc.shape, X.dtype, X.device) if sc is not None else None
-        _, wsp, wsn = _ws(lib.lb2_layernorm_bwd_workspace_bytes(D, R), X.device)
+        _, wsp, wsn = _ws(_query("lb2_layernorm_bwd_workspace_bytes", X.device.index, D, R), X.device)
         _cabi.check(lib.lb2_layernorm_bwd(ptr(dx), ptr(dg), ptr(db), ptr(d), ptr(X), ptr(sc), ptr(bi), ptr(sm), ptr(si), D, R,
                                           dt, code, wsp, wsn, current_stream(X.device)))
         return dx, dg, db
@@ -1167,7 +1215,7 @@ def rrule_mse_loss(yhat, y):
     n = Yh.numel()
     loss = torch.empty(1, dtype=torch.float32, device=Yh.device)
     d = jl_empty(Yh.shape, Yh.dtype, Yh.device)
-    _, wsp, wsn = _ws(lib.lb2_mse_loss_workspace_bytes(n), Yh.device)
+    _, wsp, wsn = _ws(_query("lb2_mse_loss_workspace_bytes", Yh.device.index, n), Yh.device)
     _cabi.check(lib.lb2_mse_loss(ptr(loss), ptr(d), ptr(Yh), ptr(Y), n, dtype_code(Yh.dtype), wsp, wsn, current_stream(Yh.device)))
 
     def pullback(delta=None):
@@ -1192,7 +1240,7 @@ def rrule_cross_entropy_loss(yhat, y, *, logits: bool = False, label_smoothing=N
     eps = float(epsilon) if epsilon is not None else float(torch.finfo(Yh.dtype).eps)
     loss = torch.empty(1, dtype=torch.float32, device=Yh.device)
     d = jl_empty(Yh.shape, Yh.dtype, Yh.device)
-    _, wsp, wsn = _ws(lib.lb2_cross_entropy_workspace_bytes(K, B), Yh.device)
+    _, wsp, wsn = _ws(_query("lb2_cross_entropy_workspace_bytes", Yh.device.index, K, B), Yh.device)
     _cabi.check(lib.lb2_cross_entropy(ptr(loss), ptr(d), ptr(Yh), ptr(Y), K, B, 1 if logits else 0, float(label_smoothing or 0.0), eps,
                                       dtype_code(Yh.dtype), wsp, wsn, current_stream(Yh.device)))
 
