@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) cw_transpose_kernel(uint16_t* __restrict_
 // hq = q when only the kW taps are folded (FR = 1, d = 0), hq = sh*q - pad_h + d when FR = sh kernel rows are folded
 // too. Channels padded with zeros to Cp. A block stages the FR * C input rows of up to kFoldPos positions (with their
 // padding) in shared memory, coalesced, and writes the positions' channels as one run of 16-byte vectors; bound by the write
-// (7x7/2 stem, 224 x 224 x 3 x 256: 316 MB; a gather from global memory per vector took 359 us).
+// (7x7/2 stem, 224 x 224 x 3 x 256: 316 MB; 161 us; a gather from global memory per vector took 359 us).
 constexpr int kFoldPos = 128;
 inline int cw_fold_width(int kW, int s, int dil) { return (kFoldPos - 1) * s + (kW - 1) * dil + 1; }
 __global__ void __launch_bounds__(256) cw_transpose_fold_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in,

@@ -587,41 +587,44 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
   }
 }
 
-// dw[kw, kh, ci, co] = sum over splits (ascending inside each of four slices, the slices in order) of
-// partial[z][(tap * chunks + ci / 32) * 32 + ci % 32][co]. A block takes 4 input channels x 32 output channels x all taps:
-// lanes read 32 consecutive co, the sums are turned in shared memory and written as runs of 4 * taps elements of dw.
+// partial[0] = sum over splits (ascending) of partial[z]: a thread per four elements
+__global__ void __launch_bounds__(256) cwf_sum_splits_kernel(float4* __restrict__ partial, int64_t n4, int splits) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
+    float4 s = partial[i];
+#pragma unroll 8
+    for (int z = 1; z < splits; ++z) {
+      const float4 v = __ldcs(partial + z * n4 + i);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    partial[i] = s;
+  }
+}
+// dw[kw, kh, ci, co] = partial[(tap * chunks + ci / 32) * 32 + ci % 32][co]. A block takes 4 input channels x 32 output
+// channels x all taps: lanes read 32 consecutive co, the block turns them in shared memory and writes runs of 4 * taps elements
+// of dw. (Summing the splits here as well left all but 2 to 64 blocks of the GPU idle for small filters: 136 us for a stem's
+// 74 splits, 52 us for 512 x 512 x 3 x 3.)
 struct CwfReduce {
-  int kW, kH, cin, cout, flip, fold, chunks, rows, n_pad, splits;
+  int kW, kH, cin, cout, flip, fold, chunks, n_pad;
 };
-__global__ void __launch_bounds__(1024) cwf_wgrad_reduce_kernel(float* __restrict__ dw, const float* __restrict__ partial, const CwfReduce g) {
-  extern __shared__ float cwf_part[];                  // [4 slices][4 channels][taps][33]
+__global__ void __launch_bounds__(256) cwf_wgrad_store_kernel(float* __restrict__ dw, const float* __restrict__ partial, const CwfReduce g) {
+  extern __shared__ float cwf_part[];                  // [4 channels][taps][33]
   const int taps = g.kW * g.kH;
   const int cgroups = (g.cin + 3) / 4;
   const int ci0 = (blockIdx.x % cgroups) * 4, co0 = (blockIdx.x / cgroups) * 32;
-  const int lane = threadIdx.x & 31, slice = (threadIdx.x >> 5) & 3, rl = threadIdx.x >> 7;
-  const int64_t split_stride = (int64_t)g.rows * g.n_pad;
-  for (int rt = rl; rt < 4 * taps; rt += 8) {
-    const int c = rt / taps, t = rt - c * taps, ci = ci0 + c;   // t in dw's (kh, kw) order
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int rt = threadIdx.x >> 5; rt < 4 * taps; rt += 8) {
+    const int c = rt / taps, t = rt - c * taps, ci = min(ci0 + c, g.cin - 1);   // t in dw's (kh, kw) order
     const int kw = t % g.kW, kh = t / g.kW;
     const int tw = g.flip ? kw : g.kW - 1 - kw, th = g.flip ? kh : g.kH - 1 - kh;
     const int row = g.fold ? th * 32 + tw * g.cin + ci : ((th * g.kW + tw) * g.chunks + ci / 32) * 32 + (ci & 31);
-    float s = 0.f;
-    if (ci < g.cin) {
-      const float* src = partial + (int64_t)row * g.n_pad + co0 + lane;   // n_pad is a multiple of 64
-#pragma unroll 4
-      for (int z = slice; z < g.splits; z += 4) s += __ldcs(src + z * split_stride);
-    }
-    cwf_part[(slice * 4 * taps + rt) * 33 + lane] = s;
+    cwf_part[rt * 33 + lane] = partial[(int64_t)row * g.n_pad + co0 + lane];    // n_pad is a multiple of 64
   }
   __syncthreads();
   const int run = min(4, g.cin - ci0) * taps;
-  for (int e = threadIdx.x; e < 32 * run; e += 1024) {
+  for (int e = threadIdx.x; e < 32 * run; e += 256) {
     const int co = e / run, k = e - co * run;
-    if (co0 + co >= g.cout) continue;
-    float s = 0.f;
-#pragma unroll
-    for (int y = 0; y < 4; ++y) s += cwf_part[(y * 4 * taps + k) * 33 + co];
-    dw[((int64_t)(co0 + co) * g.cin + ci0) * taps + k] = s;
+    if (co0 + co < g.cout) dw[((int64_t)(co0 + co) * g.cin + ci0) * taps + k] = cwf_part[k * 33 + co];
   }
 }
 
@@ -852,7 +855,6 @@ bool conv_cwf_supported(const ConvGeom& g) {
   if (g.stride[0] > 4 || g.stride[1] > 4) return false;               // box extent = positions x stride must stay <= 256
   if (g.k[0] * g.k[1] > kFMaxTaps) return false;
   if (g.k[0] * g.dil[0] > 120 || g.k[1] * g.dil[1] > 120) return false;
-  if (4 * 4 * g.k[0] * g.k[1] * 33 * 4 > 200 * 1024) return false;    // shared memory of the filter-gradient reduction
   if (x_numel(g) >= ((int64_t)1 << 40)) return false;
   const CwfGrid t = cwf_grid(g.out[0], g.out[1], g.batch, g.cout);
   if (t.BW * g.stride[0] > 256 || t.BH * g.stride[1] > 256) return false;
@@ -950,11 +952,16 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     };
     rc = bn == 64 ? launch(conv_cwf_wgrad_kernel<64>, CwfCfg<64>::SMEM_BYTES) : launch(conv_cwf_wgrad_kernel<128>, CwfCfg<128>::SMEM_BYTES);
     if (rc != LB2_OK) return rc;
-    const CwfReduce rd{g.k[0], g.k[1], g.cin, g.cout, g.flip, fold, pl.chunks, pl.m_tiles * 128, pl.n_pad, pl.splits};
-    const int smem = 4 * 4 * g.k[0] * g.k[1] * 33 * 4;
-    cudaError_t e = cudaFuncSetAttribute(cwf_wgrad_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (pl.splits > 1) {
+      const int64_t n4 = (int64_t)pl.m_tiles * 128 * pl.n_pad / 4;
+      cwf_sum_splits_kernel<<<cwf_flat_grid(n4), 256, 0, st>>>(reinterpret_cast<float4*>(q.partial), n4, pl.splits);
+      LB2_CHECK_LAUNCH("conv_cw_f32 filter-gradient split sum");
+    }
+    const CwfReduce rd{g.k[0], g.k[1], g.cin, g.cout, g.flip, fold, pl.chunks, pl.n_pad};
+    const int smem = 4 * g.k[0] * g.k[1] * 33 * 4;
+    cudaError_t e = cudaFuncSetAttribute(cwf_wgrad_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    cwf_wgrad_reduce_kernel<<<(unsigned)(((g.cin + 3) / 4) * ((g.cout + 31) / 32)), 1024, smem, st>>>((float*)dw, q.partial, rd);
+    cwf_wgrad_store_kernel<<<(unsigned)(((g.cin + 3) / 4) * ((g.cout + 31) / 32)), 256, smem, st>>>((float*)dw, q.partial, rd);
     LB2_CHECK_LAUNCH("conv_cw_f32 filter-gradient reduction");
   }
 
