@@ -1,5 +1,5 @@
 // Direct (CUDA-core) convolution: the catch-all for every ConvDims the implicit-GEMM tensor-core
-// path does not take (1-D / 3-D, dilation, groups, odd strides, unaligned widths). Forward, data
+// paths do not take (1-D / 3-D, groups, strides above 4, very large kernels). Forward, data
 // gradient and filter gradient, each with fp32 accumulation in a fixed order (deterministic).
 // Layout: x (in..., Cin, N), w (k..., Cin/groups, Cout), y (out..., Cout, N), column-major;
 // true convolution (kernel flipped) unless flipkernel is set — NNlib semantics as used by
