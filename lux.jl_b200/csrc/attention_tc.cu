@@ -12,7 +12,7 @@
 // bf16: kind::f16, one accumulator per tile, two in flight. Float32: hi/lo tf32 operands, three products per k-block,
 // k-blocks added in fp32 registers (the tensor core truncates when it accumulates).
 //
-// Measured, forward + pullback through the operator, 8 heads x 8 samples, 512 x 512, 64 features, causal, bf16: 136 us (one
+// Measured, forward + pullback through the operator, 8 heads x 8 samples, 512 x 512, 64 features, causal, bf16: 130 us (one
 // tensor-core GEMM launch per head, sample and product before: 4.1 ms); Float32 4 x 4, 771 x 771: 300 us (3.07 ms).
 // What bounds it: a contraction over a head's 64 features is one k-block, so the products move the S x L weights and little
 // else; the passes over the weights (in L2 for the usual sizes) are the cost.
@@ -36,6 +36,7 @@ struct AtParams {
   int32_t bk, tiles_m, tiles_n, heads, rep, batch, num_kb;
   int32_t M, N;                      // N rounded up to the vector the rows of D are padded to
   int32_t causal;                    // which of the enum's rules applies to this product
+  int32_t wide;                      // rows of D start on 32-byte boundaries: whole sectors per store
   uint32_t idesc, idesc_wide;
   void* D;
   int64_t ldd, head_stride, batch_stride;
@@ -55,6 +56,12 @@ __device__ __forceinline__ void at_load(uint32_t dst, const CUtensorMap* map, co
   const int inner = o.mn_major ? mn : k, outer = o.mn_major ? k : mn;
   if (o.head_first) tma_load_4d(dst, map, inner, head, outer, img, bar);
   else tma_load_4d(dst, map, inner, outer, head, img, bar);
+}
+
+__device__ __forceinline__ void at_store32(void* p, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
 }
 
 template <int BN, bool F32>
@@ -213,6 +220,23 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!ok) break;
       if (m < p.M) {
+        if (p.wide && n0 + COLS <= p.N) {
+#pragma unroll
+          for (int j = 0; j < COLS; j += 2 * VEC) {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              if constexpr (F32) {
+                w[i] = __float_as_uint(sum[j + i]);
+              } else {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(sum[j + 2 * i], sum[j + 2 * i + 1]);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+              }
+            }
+            at_store32(d + j, w);
+          }
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < COLS; j += VEC) {
           if (n0 + j < p.N) {
@@ -337,13 +361,18 @@ __global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, T
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   // a row with every key masked: m = -inf and every difference below is NaN, as in the reference
+  const float off = expf(-INFINITY - m);                       // weight of a key past lim, before the division: 0 (or NaN)
   if constexpr (NV > 0) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
+    for (int i = 0; i < NV; ++i) {
+      if ((i * 32 + lane) * 4 < lim) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if ((i * 32 + lane) * 4 + k < S) { r[i][k] = expf(r[i][k] - m); se += r[i][k]; }
+        for (int k = 0; k < 4; ++k)
+          if ((i * 32 + lane) * 4 + k < S) { r[i][k] = expf(r[i][k] - m); se += r[i][k]; }
+      } else {
+        r[i][0] = r[i][1] = r[i][2] = r[i][3] = off;
       }
+    }
   } else {
     for (int s = lane * 4; s < lim; s += 128) {
       float v[4];
@@ -376,7 +405,7 @@ __global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, T
       float v[4] = {0.f, 0.f, 0.f, 0.f};
       if (s < lim) value4(s, v);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = s < lim && s + k < S ? expf(v[k] - m) * inv : (s + k < S ? expf(-INFINITY - m) * inv : 0.f);
+      for (int k = 0; k < 4; ++k) v[k] = s < lim && s + k < S ? expf(v[k] - m) * inv : (s + k < S ? off * inv : 0.f);
       put(s, v);
     }
   }
@@ -530,6 +559,7 @@ int32_t at_gemm(const AtProduct& g, int64_t batch, int32_t dtype, cudaStream_t s
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((g.a_mn ? 1u : 0u) << 15) | ((g.b_mn ? 1u : 0u) << 16) | ((uint32_t)(bn >> 3) << 17) |
             ((uint32_t)(kAtBM >> 4) << 24);
   p.idesc_wide = (p.idesc & ~(0x3Fu << 17)) | ((uint32_t)((2 * bn) >> 3) << 17);
+  p.wide = aligned_to(g.D, 32) && (g.ldd * es) % 32 == 0 && (g.head_stride * es) % 32 == 0 && (g.batch_stride * es) % 32 == 0;
   p.D = g.D; p.ldd = g.ldd; p.head_stride = g.head_stride; p.batch_stride = g.batch_stride;
   p.status = device_status_word();
   LB2_REQUIRE(p.status != nullptr, LB2_LAUNCH_FAIL, "attention: device status word unavailable");
