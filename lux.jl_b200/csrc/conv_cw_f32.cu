@@ -17,7 +17,7 @@
 //
 // Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 86 / 158 us (86 /
 // 94 TFLOP/s); 3x3 512 -> 512 on 7x7: 96 / 198 us (with the MMAs issued from a one-lane branch: 96 / 174 and 105 / 215 us). The CUDA-core kernels of conv_direct.cu, which took these geometries
-// before, made a ResNet-18 training step at batch 32 last 333 ms; it now takes 6.7 ms.
+// before, made a ResNet-18 training step at batch 32 last 333 ms; it now takes 6.2 ms.
 // What bounds it: a 128 x 128 x 32 k-block is 768 tensor-pipe cycles (three tf32 products) against about 1280 cycles of
 // shared-memory traffic (64 KB written by TMA, 96 KB read by the MMAs at 128 B/cycle).
 #include "conv.cuh"
