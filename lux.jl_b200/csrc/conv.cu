@@ -108,6 +108,9 @@ int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const 
     route = (conv_cw_supported(g, dtype) && conv_cw_fwd_workspace_bytes(g) <= workspace_bytes) ? 2 : 0;
   if (route != 0) {
     const size_t need = route_fwd_bytes(route, g, dtype);
+    // without room for the Float32 copies the CUDA-core kernels, which need none, still serve the call
+    if (route == 3 && (workspace == nullptr || workspace_bytes < need))
+      return conv_fwd_direct(y, preact, x, w, b, g, dtype, act, static_cast<cudaStream_t>(stream));
     LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", need);
     LB2_REQUIRE(aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");
     if (route == 1) return conv_tc_fwd(y, preact, x, w, b, g, dtype, act, workspace, static_cast<cudaStream_t>(stream));
@@ -201,13 +204,18 @@ int32_t lb2_conv_bwd(void* dw, void* dx, void* db, const void* dy, const void* o
                   aligned_to(preact, es) && aligned_to(x, es) && aligned_to(w, es),
               LB2_BAD_ALIGN, "pointer not aligned to the element size");
   const ConvBwdLayout lay = conv_bwd_layout(g, dtype, act);
-  LB2_REQUIRE(workspace != nullptr && workspace_bytes >= lay.total(), LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", lay.total());
+  int route = (flags & LB2_FLAG_FORCE_SIMT) ? 0 : (lay.tc_bytes > 0 ? conv_route(g, dtype) : 0);
+  size_t need = lay.total();
+  if (route == 3 && !(flags & LB2_FLAG_X_COPY_GIVEN) && workspace_bytes < need) {   // as in the forward call
+    route = 0;
+    need = lay.g_bytes + lay.red_bytes;
+  }
+  LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", lay.total());
   LB2_REQUIRE(aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   float* red = reinterpret_cast<float*>(ws + lay.g_bytes);
   const int64_t S = y_spatial(g);
   const void* gptr = dy;
-  const int route = (flags & LB2_FLAG_FORCE_SIMT) ? 0 : (lay.tc_bytes > 0 ? conv_route(g, dtype) : 0);
   // identity activation on the bf16 fast case: the filter-gradient kernel adds up dy on the side, no pass of its own
   const bool db_by_wgrad = act == LB2_ACT_IDENTITY && db && dw && route == 1 && dtype == LB2_BF16 && aligned_to(dy, 16) &&
                            aligned_to(x, 16) && aligned_to(dx, 16) && conv_tc_wgrad_makes_db(g, dtype);

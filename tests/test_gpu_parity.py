@@ -1191,3 +1191,28 @@ def test_dense_epilogue_of_the_cluster_kernel(dt, act, mnk):
     check(y, y_ref, dt, "y")
     for name, got, want in zip(("dW", "dx", "db"), pb(dev(d, dt)), pb_ref(d.astype(np.float64))):
         check(got, want, dt, name)
+
+
+def test_f32_conv_without_room_for_its_copies():
+    # the Float32 general path needs scratch that the CUDA-core kernels did not: a call without it is still served
+    import ctypes as C
+    from luxlib_b200 import ops as _ops
+    rng = np.random.default_rng(65)
+    x, w = rng.standard_normal((9, 7, 6, 3)).astype(np.float32), rng.standard_normal((3, 3, 6, 5)).astype(np.float32)
+    ocd, lcd = O.ConvDims.make(2, 2, 1, 1, 1, False), L.ConvDims.make(2, 2, 1)
+    y_ref, pb_ref = O.fused_conv_rrule("identity", w.astype(np.float64), x.astype(np.float64), None, ocd)
+    lib, X, W = L._cabi.load(), dev(x, "f32"), dev(w, "f32")
+    d = _ops._conv_desc(W, X, lcd)
+    y = L.jl_empty(y_ref.shape, X.dtype, X.device)
+    assert lib.lb2_conv_fwd_workspace_bytes(C.byref(d), 0) > 0
+    assert lib.lb2_conv_fwd(y.data_ptr(), None, X.data_ptr(), W.data_ptr(), None, C.byref(d), 0, 0, 0, None, 0, None) == 0
+    check(y, y_ref, "f32", "y")
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    dw_ref, dx_ref, _ = pb_ref(delta.astype(np.float64))
+    G, dw, dx = dev(delta, "f32"), L.jl_empty(w.shape, X.dtype, X.device), L.jl_empty(x.shape, X.dtype, X.device)
+    ws = torch.empty(1 << 12, dtype=torch.uint8, device="cuda")          # room for the column sums only
+    assert lib.lb2_conv_bwd_workspace_bytes(C.byref(d), 0, 0) > ws.numel()
+    assert lib.lb2_conv_bwd(dw.data_ptr(), dx.data_ptr(), None, G.data_ptr(), None, None, X.data_ptr(), W.data_ptr(), C.byref(d), 0, 0, 0,
+                            ws.data_ptr(), ws.numel(), None) == 0
+    check(dw, dw_ref, "f32", "dw")
+    check(dx, dx_ref, "f32", "dx")
