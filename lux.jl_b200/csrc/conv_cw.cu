@@ -876,6 +876,9 @@ int32_t cw_launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, CwFwdParams&
   // A filter of one column tile that fits 96 KB stays in shared memory: its tiles would otherwise be fetched again for every
   // 128 positions (the folded stem's four: a third of what the kernel takes in, 506 us per 256 images of 224 x 224).
   constexpr int A_BYTES = kCwBM * 128, B_BYTES = BN * 128;
+  // A filter of one column tile that fits 96 KB stays in shared memory; in the ring its tiles are fetched again for every 128
+  // positions, a third of what a folded stem's kernel takes in (256 images of 224 x 224: 506 us, resident 449 us). Above
+  // 96 KB too few A tiles would be left in flight.
   const bool resident = p.tiles_n == 1 && p.num_kb * B_BYTES <= 96 * 1024 && p.sums_partial == nullptr;
   const int fixed = resident ? p.num_kb * B_BYTES : 0, stage_bytes = resident ? A_BYTES : A_BYTES + B_BYTES;
   p.stages = (200 * 1024 - fixed) / stage_bytes > 8 ? 8 : (200 * 1024 - fixed) / stage_bytes;
