@@ -1,27 +1,29 @@
-// General tensor-core convolution for Float32 storage on sm_100a: the channel-innermost implicit GEMM of conv_cw.cu with
-// the fp32-accurate products of conv_tc_f32.cu, for any 2-D stride / padding / dilation / kernel size / channel counts
-// with groups == 1.
+// General tensor-core convolution for Float32 storage on sm_100a: the channel-innermost implicit GEMM of conv_cw.cu on three
+// bf16 parts per operand, for any 2-D padding / dilation / kernel size / channel counts with groups == 1 and strides up to 4
+// whose position boxes fit a TMA box (conv_cwf_supported).
 //
-// Accuracy. Every operand is split on the way in, hi = tf32(x), lo = x - hi; a k-block (32 contracted elements) forms
-// hi*hi, hi*lo and lo*hi. The tensor core truncates when it adds into TMEM, so the hi*hi products are
-// taken out after every two k-steps and eight warps add them round-to-nearest into fp32 registers.
+// Accuracy: products and partial sums as in parts.cuh, x1*w1 taken out of TMEM after every k-block of 32. The filter gradient, a
+// sum over all positions, goes to memory in segments of kSegment k-blocks, so that no register adds up more than that many, and
+// its splits are added with a compensated sum.
 //
-//   layout       x (and dy) are rewritten channel-innermost, hi and lo (one pass: read 4 bytes, write 8 per element); a tap
+//   layout       x (and dy) are rewritten channel-innermost, three parts (one pass: read 4 bytes, write 6 per element); a tap
 //                shift, the padding and the stride are then start coordinates / box parameters of a 4-D TMA map
 //   forward      M = 128 output positions (a w x h x image box), N = 64 / 128 output channels, both operands K-major
 //   data grad.   the same kernel on the copy of dy with the filter transposed; stride s: s*s classes of input positions
 //   filter grad. rows = four (tap, 32-channel chunk) boxes of x, columns = 64 / 128 output channels of dy, contraction over
-//                32-position boxes; both operands MN-major (32-byte-atom swizzle), split over CTAs, fixed-order reduction
+//                32-position boxes; both operands MN-major, split over CTAs, fixed-order reduction
 // A problem with too few tiles for the SMs is split along the contraction as well: fp32 partials in the layout of the
 // output and one elementwise pass that adds them in order (deterministic) and applies bias and activation.
 //
-// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 86 / 158 us (86 /
-// 94 TFLOP/s); 3x3 512 -> 512 on 7x7: 96 / 198 us (with the MMAs issued from a one-lane branch: 96 / 174 and 105 / 215 us). The CUDA-core kernels of conv_direct.cu, which took these geometries
-// before, made a ResNet-18 training step at batch 32 last 333 ms; it now takes 6.2 ms.
-// What bounds it: a 128 x 128 x 32 k-block is 768 tensor-pipe cycles (three tf32 products) against about 1280 cycles of
-// shared-memory traffic (64 KB written by TMA, 96 KB read by the MMAs at 128 B/cycle).
+// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 84 / 155 us (89 /
+// 95 TFLOP/s); 3x3 512 -> 512 on 7x7: 95 / 171 us. Two tf32 parts took 90 / 154 and 99 / 168 us and were less accurate than
+// fp32 sums in the filter gradient. The CUDA-core kernels of conv_direct.cu, which took these geometries before, made a
+// ResNet-18 training step at batch 32 last 333 ms; it now takes 6.2 ms. Error against 64 bits (2-norm, normal data): 5e-8 to
+// 1.6e-7, the CUDA-core kernels' 6e-8 to 1.1e-6.
+// What bounds it: a 128 x 128 x 32 k-block is 768 tensor-pipe cycles (12 MMAs) against about 1150 cycles of shared-memory
+// traffic (48 KB written by TMA, 96 KB read by the MMAs at 128 B/cycle).
 #include "conv.cuh"
-#include "tc_ptx.cuh"
+#include "parts.cuh"
 
 namespace lb2 {
 
@@ -32,21 +34,13 @@ constexpr int kFBM = 128;
 constexpr int kFMaxTaps = 128;
 constexpr int kFMaxSplits = 16;
 
-__device__ __forceinline__ void split_hi_lo(float v, float& hi, float& lo) {
-  uint32_t h;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-  hi = __uint_as_float(h);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v - hi));   // the tensor core would cut the low bits off
-  lo = __uint_as_float(h);
-}
-
 // ----------------------------------------------------------------------------------------------
 // layout passes
 // ----------------------------------------------------------------------------------------------
-// hi/lo[n][s][c] (c contiguous, Cp channels, zero beyond C)  <-  in[n][c][s]: 32 channels x 64 positions per tile through
+// parts[n][s][c] (c contiguous, Cp channels, zero beyond C)  <-  in[n][c][s]: 32 channels x 64 positions per tile through
 // shared memory. V4: 16-byte loads (planes of S % 4 == 0 floats on a 16-byte base); stores are 16 bytes along c.
 template <bool V4>
-__global__ void __launch_bounds__(256) cwf_transpose_kernel(float* __restrict__ hi, float* __restrict__ lo, const float* __restrict__ in,
+__global__ void __launch_bounds__(256) cwf_transpose_kernel(uint16_t* __restrict__ out, int64_t part_stride, const float* __restrict__ in,
                                                             int S, int C, int Cp, int N) {
   __shared__ float tile[32 * 65];
   const int st = (S + 63) / 64, ct = (Cp + 31) / 32;
@@ -75,28 +69,21 @@ __global__ void __launch_bounds__(256) cwf_transpose_kernel(float* __restrict__ 
       }
     }
     __syncthreads();
+    const int j = threadIdx.x / 4, q = (threadIdx.x % 4) * 8;   // one position, eight channels
+    if (s0 + j < S && c0 + q < Cp) {
+      float v[8];
 #pragma unroll
-    for (int v = threadIdx.x; v < 64 * 8; v += 256) {
-      const int j = v / 8, q = (v % 8) * 4;
-      if (s0 + j < S && c0 + q < Cp) {
-        float4 h, l;
-        split_hi_lo(tile[(q + 0) * 65 + j], h.x, l.x);
-        split_hi_lo(tile[(q + 1) * 65 + j], h.y, l.y);
-        split_hi_lo(tile[(q + 2) * 65 + j], h.z, l.z);
-        split_hi_lo(tile[(q + 3) * 65 + j], h.w, l.w);
-        const int64_t o = ((int64_t)n * S + s0 + j) * Cp + c0 + q;
-        *reinterpret_cast<float4*>(hi + o) = h;
-        *reinterpret_cast<float4*>(lo + o) = l;
-      }
+      for (int k = 0; k < 8; ++k) v[k] = tile[(q + k) * 65 + j];
+      store_parts8(out + ((int64_t)n * S + s0 + j) * Cp + c0 + q, part_stride, v);
     }
   }
 }
 
-// Small channel counts, the kW taps folded into the channel index: hi/lo[n][h][ow][tw*C + c] = in[n][c][h][ow*s + tw*dil - pad]
-// (0 outside), padded to Cp. One thread per four channels of the copy.
-__global__ void __launch_bounds__(256) cwf_fold_kernel(float* __restrict__ hi, float* __restrict__ lo, const float* __restrict__ in,
+// Small channel counts, the kW taps folded into the channel index: parts[n][h][ow][tw*C + c] = in[n][c][h][ow*s + tw*dil - pad]
+// (0 outside), padded to Cp. One thread per eight channels of the copy.
+__global__ void __launch_bounds__(256) cwf_fold_kernel(uint16_t* __restrict__ out, int64_t part_stride, const float* __restrict__ in,
                                                        int W, int H, int C, int Cp, int N, int OW, int kW, int s, int dil, int pad) {
-  const int groups = Cp / 4;
+  const int groups = Cp / 8;
   const int64_t total = (int64_t)N * H * OW * groups;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = i;
@@ -105,28 +92,25 @@ __global__ void __launch_bounds__(256) cwf_fold_kernel(float* __restrict__ hi, f
     const int h = (int)(r % H);
     const int n = (int)(r / H);
     const float* plane0 = in + (int64_t)n * C * H * W;
-    int tw = (qg * 4) / C, c = (qg * 4) % C;
-    float eh[4], el[4];
+    int tw = (qg * 8) / C, c = (qg * 8) % C;
+    float v[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float v = 0.f;
+    for (int k = 0; k < 8; ++k) {
       const int w = ow * s + tw * dil - pad;
-      if (tw < kW && w >= 0 && w < W) v = __ldg(plane0 + ((int64_t)c * H + h) * W + w);
-      split_hi_lo(v, eh[k], el[k]);
+      v[k] = tw < kW && w >= 0 && w < W ? __ldg(plane0 + ((int64_t)c * H + h) * W + w) : 0.f;
       if (++c == C) { c = 0; ++tw; }
     }
-    *reinterpret_cast<float4*>(hi + i * 4) = make_float4(eh[0], eh[1], eh[2], eh[3]);
-    *reinterpret_cast<float4*>(lo + i * 4) = make_float4(el[0], el[1], el[2], el[3]);
+    store_parts8(out + i * 8, part_stride, v);
   }
 }
 
-// Packed filter Wp[row][tap][chunk][32], hi and lo. Forward: row = co, contracted channel = ci. Data gradient (transpose):
+// Packed filter Wp[row][tap][chunk][32], three parts. Forward: row = co, contracted channel = ci. Data gradient (transpose):
 // row = ci, contracted = co. tap = th*kW + tw in tap positions (filter index = flip ? t : K-1-t per dim); fold: tap = th and
 // the contracted index of a tap is (tw, ci).
 struct CwfPack {
   int kW, kH, cin, cout, flip, transpose, fold, chunks, n_rows, k_total;
 };
-__global__ void __launch_bounds__(256) cwf_pack_flat_kernel(float* __restrict__ wh, float* __restrict__ wl, const float* __restrict__ w,
+__global__ void __launch_bounds__(256) cwf_pack_flat_kernel(uint16_t* __restrict__ out, int64_t part_stride, const float* __restrict__ w,
                                                             const CwfPack g) {
   const int64_t total = (int64_t)g.n_rows * g.k_total;
   const int kc = g.transpose ? g.cout : g.cin, nc = g.transpose ? g.cin : g.cout;
@@ -150,12 +134,13 @@ __global__ void __launch_bounds__(256) cwf_pack_flat_kernel(float* __restrict__ 
       const int ci = g.transpose ? row : c, co = g.transpose ? c : row;
       v = w[((int64_t)(co * g.cin + ci) * g.kH + kh) * g.kW + kw];
     }
-    split_hi_lo(v, wh[i], wl[i]);
+    const Parts q = split_parts(v);
+    out[i] = q.a; out[i + part_stride] = q.b; out[i + 2 * part_stride] = q.c;
   }
 }
 // The same for unfolded filters: a block turns 8 packed rows x 32 contracted channels x all taps through shared memory, so
-// that the filter is read in runs of its own order and the packed rows are written in runs of 128 bytes.
-__global__ void __launch_bounds__(256) cwf_pack_tile_kernel(float* __restrict__ wh, float* __restrict__ wl, const float* __restrict__ w,
+// that the filter is read in runs of its own order and the packed rows are written in runs of 64 bytes.
+__global__ void __launch_bounds__(256) cwf_pack_tile_kernel(uint16_t* __restrict__ out, int64_t part_stride, const float* __restrict__ w,
                                                             const CwfPack g) {
   extern __shared__ float cwf_tile[];                 // [8 rows][32 channels][taps] in the order it is read
   const int taps = g.kW * g.kH;
@@ -178,7 +163,8 @@ __global__ void __launch_bounds__(256) cwf_pack_tile_kernel(float* __restrict__ 
     const int tw = tap % g.kW, th = tap / g.kW;
     const int kw = g.flip ? tw : g.kW - 1 - tw, kh = g.flip ? th : g.kH - 1 - th;
     const int64_t o = (int64_t)(row0 + r) * g.k_total + (tap * g.chunks + chunk) * 32 + c;
-    split_hi_lo(cwf_tile[(r * 32 + c) * taps + kh * g.kW + kw], wh[o], wl[o]);
+    const Parts q = split_parts(cwf_tile[(r * 32 + c) * taps + kh * g.kW + kw]);
+    out[o] = q.a; out[o + part_stride] = q.b; out[o + 2 * part_stride] = q.c;
   }
 }
 
@@ -186,20 +172,17 @@ __global__ void __launch_bounds__(256) cwf_pack_tile_kernel(float* __restrict__ 
 // kernels
 // ----------------------------------------------------------------------------------------------
 template <int BN> struct CwfCfg {
-  static constexpr int A_BYTES = kFBM * 128;                    // 128 rows x 32 floats, one of hi / lo
-  static constexpr int B_BYTES = BN * 128;
-  static constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES);   // [A_hi | A_lo | B_hi | B_lo]
+  static constexpr int A_BYTES = kFBM * 64;                     // 128 rows x 32 bf16, one part
+  static constexpr int B_BYTES = BN * 64;
+  static constexpr int STAGE_BYTES = 3 * (A_BYTES + B_BYTES);   // [A1 | A2 | A3 | B1 | B2 | B3]
   static constexpr int SLOTS = 512 / BN - 1;                    // TMEM: a ring of BN-column accumulators and one for the small products
   static constexpr int STAGES = (200 * 1024) / STAGE_BYTES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 };
 
-// TMEM between the MMA thread and the accumulating warps. Every accumulation in TMEM truncates: a loss of about 3.5e-8 of
-// the partial sum that always has its sign, so that four k-steps in one accumulator shrink every result by 8.7e-8 (measured,
-// any layer), which the layers of a network add up. So hi*hi has an accumulator for each two k-steps (5.2e-8; a ring of
-// BN-column slots, a k-block's two taken out together, added to each other and then to the fp32 sum), while the small
-// products, 2^-11 of the result, gather in one accumulator for the whole item. One k-step per accumulator (3.5e-8) made a
-// ResNet-18 step a quarter slower.
+// TMEM between the MMA thread and the accumulating warps: x1*w1 has an accumulator for each k-block (a ring of BN-column slots),
+// the small products, 2^-9 of the result, gather in one accumulator for a segment of kSegment k-blocks.
+constexpr int kSegment = 16;
 template <int SLOTS> struct CwfRing {
   uint64_t *full, *empty;             // [SLOTS] of the ring, [SLOTS] = the small products'
   uint32_t slot, phase, small_phase;
@@ -207,69 +190,55 @@ template <int SLOTS> struct CwfRing {
     if (++slot == SLOTS) { slot = 0; phase ^= 1u; }
   }
 };
+// k-block i of `n` of an item
 template <int BN>
 __device__ __forceinline__ bool cwf_issue_kblock(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_base, uint32_t sA, uint32_t sB, uint32_t desc_hi,
-                                                 uint32_t lbo, uint32_t k_adv, uint32_t idesc, bool first, bool last, uint64_t* stage_empty,
+                                                 uint32_t lbo, uint32_t k_adv, uint32_t idesc, int i, int n, uint64_t* stage_empty,
                                                  unsigned int* status, unsigned int code) {
   constexpr int SLOTS = CwfCfg<BN>::SLOTS;
+  const bool first = i % kSegment == 0, last = i % kSegment == kSegment - 1 || i == n - 1;   // of its segment
   const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | lbo, b32 = ((sB >> 4) & 0x3FFFu) | lbo;
   const uint64_t top = (uint64_t)desc_hi << 32;
-  constexpr uint32_t A_LO = CwfCfg<BN>::A_BYTES >> 4, B_LO = CwfCfg<BN>::B_BYTES >> 4;
-#pragma unroll
-  for (int part = 0; part < 2; ++part) {
-    if (!mbar_wait_uniform(&ring.empty[ring.slot], ring.phase ^ 1u, status, code)) return false;
-    if (first && part == 0) {
-      if (!mbar_wait_uniform(&ring.empty[SLOTS], ring.small_phase ^ 1u, status, code)) return false;
-    }
-    tc_fence_after();
-    if (elect_one()) {
-#pragma unroll
-      for (int ks = 2 * part; ks < 2 * part + 2; ++ks)
-        umma<true>(tmem_base + ring.slot * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, ks != 2 * part ? 1u : 0u);
-      umma_commit(&ring.full[ring.slot]);
-#pragma unroll
-      for (int ks = 2 * part; ks < 2 * part + 2; ++ks) {
-        umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + ks * k_adv), top | (uint64_t)(b32 + B_LO + ks * k_adv), idesc, first && ks == 0 ? 0u : 1u);
-        umma<true>(tmem_base + SLOTS * BN, top | (uint64_t)(a32 + A_LO + ks * k_adv), top | (uint64_t)(b32 + ks * k_adv), idesc, 1u);
-      }
-      if (part == 1) {
-        umma_commit(stage_empty);
-        if (last) umma_commit(&ring.full[SLOTS]);
-      }
-    }
-    __syncwarp();
-    ring.next();
+  if (!mbar_wait_uniform(&ring.empty[ring.slot], ring.phase ^ 1u, status, code)) return false;
+  if (first) {
+    if (!mbar_wait_uniform(&ring.empty[SLOTS], ring.small_phase ^ 1u, status, code)) return false;
   }
+  tc_fence_after();
+  if (elect_one()) {
+    parts_issue(tmem_base + ring.slot * BN, tmem_base + SLOTS * BN, top | (uint64_t)a32, top | (uint64_t)b32, CwfCfg<BN>::A_BYTES >> 4,
+                CwfCfg<BN>::B_BYTES >> 4, k_adv, k_adv, idesc, first, &ring.full[ring.slot]);
+    umma_commit(stage_empty);
+    if (last) umma_commit(&ring.full[SLOTS]);
+  }
+  __syncwarp();
+  ring.next();
   if (last) ring.small_phase ^= 1u;
   return true;
 }
-// accumulating side: one item's k-blocks, columns [col, col + BN / 2) of the warp's lane quarter
+// accumulating side: the next `kblocks` (at most a segment) of an item, columns [col, col + BN / 2) of the warp's lane quarter,
+// added to `sum`; `last`: the final ones of the sum
 template <int BN>
-__device__ __forceinline__ bool cwf_accumulate(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_lane, int col, int kblocks, float (&sum)[BN / 2],
-                                               unsigned int* status, unsigned int code) {
+__device__ __forceinline__ bool cwf_accumulate(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_lane, int col, int kblocks, bool last,
+                                               float (&sum)[BN / 2], unsigned int* status, unsigned int code) {
   constexpr int COLS = BN / 2, SLOTS = CwfCfg<BN>::SLOTS;
   const bool lead = (threadIdx.x & 31) == 0;
   for (int i = 0; i < kblocks; ++i) {
-    const uint32_t s0 = ring.slot, p0 = ring.phase;
-    ring.next();
-    const uint32_t s1 = ring.slot, p1 = ring.phase;
-    ring.next();
-    if (!mbar_wait_warp(&ring.full[s0], p0, status, code) || !mbar_wait_warp(&ring.full[s1], p1, status, code)) return false;
+    if (!mbar_wait_warp(&ring.full[ring.slot], ring.phase, status, code)) return false;
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < COLS / 32; ++c) {
-      uint32_t r0[32], r1[32];
-      tmem_ld32(tmem_lane + s0 * BN + col + c * 32, r0);
-      tmem_ld32(tmem_lane + s1 * BN + col + c * 32, r1);
+      uint32_t r[32];
+      tmem_ld32(tmem_lane + ring.slot * BN + col + c * 32, r);
       tmem_ld_wait();
       if (c == COLS / 32 - 1) {
         tc_fence_before();
         __syncwarp();
-        if (lead) { mbar_arrive(&ring.empty[s0]); mbar_arrive(&ring.empty[s1]); }
+        if (lead) mbar_arrive(&ring.empty[ring.slot]);
       }
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+      for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
     }
+    ring.next();
   }
   if (kblocks > 0) {
     if (!mbar_wait_warp(&ring.full[SLOTS], ring.small_phase, status, code)) return false;
@@ -281,7 +250,10 @@ __device__ __forceinline__ bool cwf_accumulate(CwfRing<CwfCfg<BN>::SLOTS>& ring,
       tmem_ld32(tmem_lane + SLOTS * BN + col + c * 32, r);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
+      for (int j = 0; j < 32; ++j) {
+        const float v = __uint_as_float(r[j]);
+        sum[c * 32 + j] = last ? parts_unbias(sum[c * 32 + j], v) : sum[c * 32 + j] + v;
+      }
     }
     tc_fence_before();
     __syncwarp();
@@ -290,13 +262,19 @@ __device__ __forceinline__ bool cwf_accumulate(CwfRing<CwfCfg<BN>::SLOTS>& ring,
   return true;
 }
 
-// K-major operands: 128-byte swizzle, 8-row atoms of 1024 bytes, 32 bytes of K per MMA step
-constexpr uint32_t kDescHiK = (uint32_t)((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
+// K-major operands: 64-byte swizzle, 8-row atoms of 512 bytes, 32 bytes of K per MMA step
+constexpr uint32_t kDescHi = (uint32_t)((512u >> 4) & 0x3FFFu) | (1u << 14) | (4u << 29);
 constexpr uint32_t kLboK = 1u << 16, kAdvK = 2u;
-// MN-major operands: 128-byte swizzle with 32-byte atoms, 4-row atoms of 512 bytes, the next 32 elements one 4096-byte box
-// further, 8 rows of 128 bytes per MMA step
-constexpr uint32_t kDescHiMN = (uint32_t)((512u >> 4) & 0x3FFFu) | (1u << 14) | (1u << 29);
-constexpr uint32_t kLboMN = ((4096u >> 4) & 0x3FFFu) << 16, kAdvMN = (8u * 128u) >> 4;
+// MN-major operands: the same swizzle, atoms of 32 elements x 8 rows, the next 32 elements one 2048-byte box further, 16 rows of
+// 64 bytes per MMA step
+constexpr uint32_t kLboMN = ((2048u >> 4) & 0x3FFFu) << 16, kAdvMN = (16u * 64u) >> 4;
+
+// A channel-innermost array of parts
+struct CwfSource {
+  const uint16_t* ptr;
+  int64_t part_stride;
+  int32_t Cp, W, H;
+};
 
 struct CwfFwdParams {
   int32_t OW, OH, NI;          // grid of output positions; a tile is a BW x BH x BI box of them
@@ -315,12 +293,24 @@ struct CwfFwdParams {
   int32_t act;
   unsigned int* status;
   int16_t tap_dw[kFMaxTaps], tap_dh[kFMaxTaps], tap_index[kFMaxTaps];
+
+  // item -> (channel tile fastest, w tile, h tile, image tile, split)
+  __device__ __forceinline__ void item_coords(int item, int* tn, int* tw, int* th, int* ti, int* z) const {
+    *tn = item % tiles_n; item /= tiles_n;
+    *tw = item % tiles_w; item /= tiles_w;
+    *th = item % tiles_h; item /= tiles_h;
+    *ti = item % tiles_i;
+    *z = item / tiles_i;
+  }
+  __device__ __forceinline__ int64_t out_index(int a, int b, int img, int col) const {
+    return (int64_t)(a * ow_step + ow_off) + (int64_t)FW * (b * oh_step + oh_off) + (int64_t)FW * FH * ((int64_t)n_out * img + col);
+  }
 };
 
 template <int BN, int ACT>
 __global__ void __launch_bounds__(kFThreads, 1)
-conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl,
-                    const __grid_constant__ CUtensorMap tmWh, const __grid_constant__ CUtensorMap tmWl,
+conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
+                    const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmW3,
                     const __grid_constant__ CwfFwdParams p) {
   using Cfg = CwfCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
@@ -336,7 +326,7 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_items = p.tiles_w * p.tiles_h * p.tiles_i * p.tiles_n * p.splits;
   // Rows of an A stage past the box's positions are never written; they only feed accumulator rows that are never stored.
-  const uint32_t tx = (uint32_t)(2 * (p.BW * p.BH * p.BI * 128 + Cfg::B_BYTES));
+  const uint32_t tx = (uint32_t)(3 * (p.BW * p.BH * p.BI * 64 + Cfg::B_BYTES));
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -352,22 +342,14 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // item -> (channel tile fastest, w tile, h tile, image tile, split)
-  auto item_coords = [&](int item, int* tn, int* tw, int* th, int* ti, int* z) {
-    *tn = item % p.tiles_n; item /= p.tiles_n;
-    *tw = item % p.tiles_w; item /= p.tiles_w;
-    *th = item % p.tiles_h; item /= p.tiles_h;
-    *ti = item % p.tiles_i;
-    *z = item / p.tiles_i;
-  };
-
   if (warp == 0) {
-    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmWh); tma_prefetch_desc(&tmWl);
+    tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmX3);
+    tma_prefetch_desc(&tmW1); tma_prefetch_desc(&tmW2); tma_prefetch_desc(&tmW3);
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       int tn, tw, th, ti, z;
-      item_coords(item, &tn, &tw, &th, &ti, &z);
+      p.item_coords(item, &tn, &tw, &th, &ti, &z);
       const int w0 = tw * p.BW * p.sw, h0 = th * p.BH * p.sh, i0 = ti * p.BI, n0 = tn * BN;
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
       int tap = kb_lo / p.chunks, ch = kb_lo - tap * p.chunks;
@@ -375,12 +357,14 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
         if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1000u)) { ok = false; break; }
         if (elect_one()) {
           mbar_expect_tx(&full[stage], tx);
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
           const int w = w0 + p.tap_dw[tap], h = h0 + p.tap_dh[tap], k0 = (p.tap_index[tap] * p.chunks + ch) * 32;
-          tma_load_4d(sA, &tmXh, ch * 32, w, h, i0, &full[stage]);
-          tma_load_2d(sB, &tmWh, k0, n0, &full[stage]);
-          tma_load_4d(sA + Cfg::A_BYTES, &tmXl, ch * 32, w, h, i0, &full[stage]);
-          tma_load_2d(sB + Cfg::B_BYTES, &tmWl, k0, n0, &full[stage]);
+          tma_load_4d(sA, &tmX1, ch * 32, w, h, i0, &full[stage]);
+          tma_load_2d(sB, &tmW1, k0, n0, &full[stage]);
+          tma_load_4d(sA + Cfg::A_BYTES, &tmX2, ch * 32, w, h, i0, &full[stage]);
+          tma_load_2d(sB + Cfg::B_BYTES, &tmW2, k0, n0, &full[stage]);
+          tma_load_4d(sA + 2 * Cfg::A_BYTES, &tmX3, ch * 32, w, h, i0, &full[stage]);
+          tma_load_2d(sB + 2 * Cfg::B_BYTES, &tmW3, k0, n0, &full[stage]);
         }
         __syncwarp();
         if (++ch == p.chunks) { ch = 0; ++tap; }
@@ -392,12 +376,12 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       int tn, tw, th, ti, z;
-      item_coords(item, &tn, &tw, &th, &ti, &z);
+      p.item_coords(item, &tn, &tw, &th, &ti, &z);
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
-        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
-        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiK, kLboK, kAdvK, p.idesc, kb == kb_lo, kb == kb_hi - 1, &empty[stage], p.status, 0x2000u)) { ok = false; break; }
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
+        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHi, kLboK, kAdvK, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x2000u)) { ok = false; break; }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
@@ -408,19 +392,22 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_const
     const int64_t plane = (int64_t)p.FW * p.FH;
     const int pos = q * 32 + lane;
     const int iw = pos % p.BW, ih = (pos / p.BW) % p.BH, ii = pos / (p.BW * p.BH);
-    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       int tn, tw, th, ti, z;
-      item_coords(item, &tn, &tw, &th, &ti, &z);
+      p.item_coords(item, &tn, &tw, &th, &ti, &z);
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
       float sum[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
-      if (!cwf_accumulate<BN>(ring, tmem_base + ((uint32_t)(q * 32) << 16), half * COLS, max(0, kb_hi - kb_lo), sum, p.status, 0x8000u)) break;
+      for (int kb = kb_lo; kb < kb_hi && ok; kb += kSegment)
+        ok = cwf_accumulate<BN>(ring, tmem_base + ((uint32_t)(q * 32) << 16), half * COLS, min(kSegment, kb_hi - kb), kb + kSegment >= kb_hi, sum,
+                                p.status, 0x8000u);
+      if (!ok) break;
       const int a = tw * p.BW + iw, b = th * p.BH + ih, img = ti * p.BI + ii;
       if (ii < p.BI && a < p.OW && b < p.OH && img < p.NI) {
         const int col0 = tn * BN + half * COLS;
-        const int64_t base = (int64_t)(a * p.ow_step + p.ow_off) + (int64_t)p.FW * (b * p.oh_step + p.oh_off) +
-                             plane * ((int64_t)p.n_out * img + col0);
+        const int64_t base = p.out_index(a, b, img, col0);
         if (p.splits > 1) {
           float* d = p.partial + z * p.split_stride + base;
 #pragma unroll
@@ -479,8 +466,8 @@ struct CwfWgParams {
 
 template <int BN>
 __global__ void __launch_bounds__(kFThreads, 1)
-conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl,
-                      const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl,
+conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
+                      const __grid_constant__ CUtensorMap tmG1, const __grid_constant__ CUtensorMap tmG2, const __grid_constant__ CUtensorMap tmG3,
                       const __grid_constant__ CwfWgParams p) {
   using Cfg = CwfCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
@@ -513,7 +500,8 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
 
   // item -> (m tile fastest, n tile, split)
   if (warp == 0) {
-    tma_prefetch_desc(&tmXh); tma_prefetch_desc(&tmXl); tma_prefetch_desc(&tmGh); tma_prefetch_desc(&tmGl);
+    tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmX3);
+    tma_prefetch_desc(&tmG1); tma_prefetch_desc(&tmG2); tma_prefetch_desc(&tmG3);
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
@@ -532,17 +520,21 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
         if (elect_one()) {
           const int bw = kb % p.kbw, bh = (kb / p.kbw) % p.kbh, bi = kb / (p.kbw * p.kbh);
           const int a0 = bw * p.KW_, b0 = bh * p.KH_, i0 = bi * p.KI_;
-          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
+          const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
           mbar_expect_tx(&full[stage], (uint32_t)Cfg::STAGE_BYTES);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            tma_load_4d(sA + j * 4096, &tmXh, c0[j], a0 * p.sw + dw[j], b0 * p.sh + dh[j], i0, &full[stage]);
-            tma_load_4d(sA + Cfg::A_BYTES + j * 4096, &tmXl, c0[j], a0 * p.sw + dw[j], b0 * p.sh + dh[j], i0, &full[stage]);
+            const int w = a0 * p.sw + dw[j], h = b0 * p.sh + dh[j];
+            tma_load_4d(sA + j * 2048, &tmX1, c0[j], w, h, i0, &full[stage]);
+            tma_load_4d(sA + Cfg::A_BYTES + j * 2048, &tmX2, c0[j], w, h, i0, &full[stage]);
+            tma_load_4d(sA + 2 * Cfg::A_BYTES + j * 2048, &tmX3, c0[j], w, h, i0, &full[stage]);
           }
 #pragma unroll
           for (int j = 0; j < BN / 32; ++j) {            // channels past the last and positions past the ends are zero-filled
-            tma_load_4d(sB + j * 4096, &tmGh, nt * BN + j * 32, a0, b0, i0, &full[stage]);
-            tma_load_4d(sB + Cfg::B_BYTES + j * 4096, &tmGl, nt * BN + j * 32, a0, b0, i0, &full[stage]);
+            const int c = nt * BN + j * 32;
+            tma_load_4d(sB + j * 2048, &tmG1, c, a0, b0, i0, &full[stage]);
+            tma_load_4d(sB + Cfg::B_BYTES + j * 2048, &tmG2, c, a0, b0, i0, &full[stage]);
+            tma_load_4d(sB + 2 * Cfg::B_BYTES + j * 2048, &tmG3, c, a0, b0, i0, &full[stage]);
           }
         }
         __syncwarp();
@@ -557,24 +549,35 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
-        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 2 * Cfg::A_BYTES;
-        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHiMN, kLboMN, kAdvMN, p.idesc, kb == kb_lo, kb == kb_hi - 1, &empty[stage], p.status, 0x40000u)) { ok = false; break; }
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
+        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHi, kLboMN, kAdvMN, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x40000u)) { ok = false; break; }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;
     constexpr int COLS = BN / 2;
-    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / per_split;
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
-      float sum[COLS];
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
-      if (!cwf_accumulate<BN>(ring, tmem_base + ((uint32_t)(q * 32) << 16), half * COLS, max(0, kb_hi - kb_lo), sum, p.status, 0x100000u)) break;
       float4* dst = reinterpret_cast<float4*>(p.partial + ((int64_t)z * p.m_tiles * 128 + mt * 128 + q * 32 + lane) * p.n_pad + nt * BN + half * COLS);
+      int kb = kb_lo;
+      do {                                               // an empty split stores zeros
+        float sum[COLS];
 #pragma unroll
-      for (int j = 0; j < COLS / 4; ++j) dst[j] = make_float4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+        for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+        ok = cwf_accumulate<BN>(ring, tmem_base + ((uint32_t)(q * 32) << 16), half * COLS, max(0, min(kSegment, kb_hi - kb)), true, sum, p.status,
+                                0x100000u);
+        if (!ok) break;
+#pragma unroll
+        for (int j = 0; j < COLS / 4; ++j) {
+          float4 v = make_float4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+          if (kb > kb_lo) { const float4 o = dst[j]; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+          dst[j] = v;
+        }
+        kb += kSegment;
+      } while (kb < kb_hi);
     }
   }
 
@@ -587,14 +590,19 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_con
   }
 }
 
-// partial[0] = sum over splits (ascending) of partial[z]: a thread per four elements
+// partial[0] = sum over splits (ascending, compensated: there are hundreds where the filter is small) of partial[z]
+__device__ __forceinline__ void cwf_add(float& s, float& c, float v) {   // Kahan; a sum that is not finite is left as it is
+  const float y = v - c, t = s + y;
+  c = fabsf(t) < INFINITY ? (t - s) - y : 0.f;
+  s = t;
+}
 __global__ void __launch_bounds__(256) cwf_sum_splits_kernel(float4* __restrict__ partial, int64_t n4, int splits) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-    float4 s = partial[i];
+    float4 s = partial[i], c = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int z = 1; z < splits; ++z) {
       const float4 v = __ldcs(partial + z * n4 + i);
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      cwf_add(s.x, c.x, v.x); cwf_add(s.y, c.y, v.y); cwf_add(s.z, c.z, v.z); cwf_add(s.w, c.w, v.w);
     }
     partial[i] = s;
   }
@@ -631,27 +639,27 @@ __global__ void __launch_bounds__(256) cwf_wgrad_store_kernel(float* __restrict_
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
-// 4-D map over a channel-innermost float array (Cp, W, H, N): box = 32 channels x bw x bh x bi positions
-bool cwf_map(CUtensorMap* map, const void* ptr, int Cp, int W, int H, int N, int bw, int bh, int bi, int sw, int sh, bool mn_major) {
+// 4-D map over one part of a channel-innermost array (Cp, W, H, N): box = 32 channels x bw x bh x bi positions
+bool cwf_map(CUtensorMap* map, const void* ptr, int Cp, int W, int H, int N, int bw, int bh, int bi, int sw, int sh) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t dims[4] = {(cuuint64_t)Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-  cuuint64_t strides[3] = {(cuuint64_t)Cp * 4, (cuuint64_t)Cp * W * 4, (cuuint64_t)Cp * W * H * 4};
+  cuuint64_t strides[3] = {(cuuint64_t)Cp * 2, (cuuint64_t)Cp * W * 2, (cuuint64_t)Cp * W * H * 2};
   cuuint32_t box[4] = {32, (cuuint32_t)(bw * sw), (cuuint32_t)(bh * sh), (cuuint32_t)bi};
   cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 bool cwf_map_2d(CUtensorMap* map, const void* ptr, int64_t d0, int64_t d1, int box1) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t dims[2] = {(cuuint64_t)d0, (cuuint64_t)d1};
-  cuuint64_t strides[1] = {(cuuint64_t)d0 * 4};
+  cuuint64_t strides[1] = {(cuuint64_t)d0 * 2};
   cuuint32_t box[2] = {32, (cuuint32_t)box1};
   cuuint32_t estr[2] = {1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 unsigned cwf_flat_grid(int64_t total) {
@@ -666,13 +674,14 @@ int cwf_taps(const ConvGeom& g) { return cwf_fold(g) ? g.k[1] : g.k[0] * g.k[1];
 
 struct CwfCopy {
   int Cp, W, H;
-  size_t one;          // bytes of the hi (or lo) array
-  size_t bytes() const { return 2 * one; }
+  size_t one;          // bytes of one part
+  size_t bytes() const { return 3 * one; }
+  int64_t part_stride() const { return (int64_t)(one / 2); }
 };
 CwfCopy cwf_copy(int C, int W, int H, int N) {
   CwfCopy c{};
-  c.Cp = (C + 3) / 4 * 4; c.W = W; c.H = H;
-  c.one = align_up((size_t)c.Cp * W * H * N * 4, 1024);
+  c.Cp = (C + 7) / 8 * 8; c.W = W; c.H = H;   // TMA strides are multiples of 16 bytes
+  c.one = align_up((size_t)c.Cp * W * H * N * 2, 1024);
   return c;
 }
 CwfCopy cwf_copy_x(const ConvGeom& g) {
@@ -680,8 +689,10 @@ CwfCopy cwf_copy_x(const ConvGeom& g) {
 }
 CwfCopy cwf_copy_y(const ConvGeom& g) { return cwf_copy(g.cout, g.out[0], g.out[1], g.batch); }
 
+CwfSource cwf_source(const void* ptr, const CwfCopy& c) { return CwfSource{static_cast<const uint16_t*>(ptr), c.part_stride(), c.Cp, c.W, c.H}; }
+
 size_t cwf_packed_one(int rows, int taps, int chunks) {
-  return align_up((size_t)((rows + cwf_bn(rows) - 1) / cwf_bn(rows) * cwf_bn(rows)) * taps * chunks * 32 * 4, 1024);
+  return align_up((size_t)((rows + cwf_bn(rows) - 1) / cwf_bn(rows) * cwf_bn(rows)) * taps * chunks * 32 * 2, 1024);
 }
 
 // Split along the contraction: cost in k-blocks (about 0.6 us each) of `items` tiles on the SMs in `s` splits, 6 for a
@@ -724,36 +735,35 @@ int cwf_dgrad_splits(const ConvGeom& g) {
   return cwf_splits(t.tiles(), tw * th * cwf_chunks(g.cout), x_numel(g), kFMaxSplits);
 }
 
-int32_t cwf_transpose(float* hi, float* lo, const float* in, int S, int C, int Cp, int N, cudaStream_t st) {
-  const int64_t blocks = (int64_t)N * ((S + 63) / 64) * ((Cp + 31) / 32);
+int32_t cwf_transpose(void* out, const CwfCopy& c, const float* in, int S, int C, int N, cudaStream_t st) {
+  const int64_t blocks = (int64_t)N * ((S + 63) / 64) * ((c.Cp + 31) / 32);
   const int64_t cap = (int64_t)sm_count() * 8;
   const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
-  if (S % 4 == 0 && aligned_to(in, 16)) cwf_transpose_kernel<true><<<grid, 256, 0, st>>>(hi, lo, in, S, C, Cp, N);
-  else cwf_transpose_kernel<false><<<grid, 256, 0, st>>>(hi, lo, in, S, C, Cp, N);
+  if (S % 4 == 0 && aligned_to(in, 16)) cwf_transpose_kernel<true><<<grid, 256, 0, st>>>((uint16_t*)out, c.part_stride(), in, S, C, c.Cp, N);
+  else cwf_transpose_kernel<false><<<grid, 256, 0, st>>>((uint16_t*)out, c.part_stride(), in, S, C, c.Cp, N);
   LB2_CHECK_LAUNCH("conv_cw_f32 transpose");
   return LB2_OK;
 }
-int32_t cwf_make_copy_x(float* hi, const float* x, const ConvGeom& g, const CwfCopy& c, cudaStream_t st) {
-  float* lo = hi + c.one / 4;
-  if (!cwf_fold(g)) return cwf_transpose(hi, lo, x, g.in[0] * g.in[1], g.cin, c.Cp, g.batch, st);
-  cwf_fold_kernel<<<cwf_flat_grid((int64_t)(c.Cp / 4) * c.W * c.H * g.batch), 256, 0, st>>>(
-      hi, lo, x, g.in[0], g.in[1], g.cin, c.Cp, g.batch, g.out[0], g.k[0], g.stride[0], g.dil[0], g.pad_lo[0]);
+int32_t cwf_make_copy_x(void* out, const float* x, const ConvGeom& g, const CwfCopy& c, cudaStream_t st) {
+  if (!cwf_fold(g)) return cwf_transpose(out, c, x, g.in[0] * g.in[1], g.cin, g.batch, st);
+  cwf_fold_kernel<<<cwf_flat_grid((int64_t)(c.Cp / 8) * c.W * c.H * g.batch), 256, 0, st>>>(
+      (uint16_t*)out, c.part_stride(), x, g.in[0], g.in[1], g.cin, c.Cp, g.batch, g.out[0], g.k[0], g.stride[0], g.dil[0], g.pad_lo[0]);
   LB2_CHECK_LAUNCH("conv_cw_f32 folded copy");
   return LB2_OK;
 }
-int32_t cwf_pack(float* wh, float* wl, const float* w, const CwfPack& pk, cudaStream_t st) {
+int32_t cwf_pack(uint16_t* out, size_t packed_one, const float* w, const CwfPack& pk, cudaStream_t st) {
   const size_t tile = (size_t)pk.kW * pk.kH * 256 * sizeof(float);
   if (!pk.fold && tile <= 48 * 1024)
-    cwf_pack_tile_kernel<<<(unsigned)(pk.n_rows / 8 * pk.chunks), 256, tile, st>>>(wh, wl, w, pk);
+    cwf_pack_tile_kernel<<<(unsigned)(pk.n_rows / 8 * pk.chunks), 256, tile, st>>>(out, (int64_t)(packed_one / 2), w, pk);
   else
-    cwf_pack_flat_kernel<<<cwf_flat_grid((int64_t)pk.n_rows * pk.k_total), 256, 0, st>>>(wh, wl, w, pk);
+    cwf_pack_flat_kernel<<<cwf_flat_grid((int64_t)pk.n_rows * pk.k_total), 256, 0, st>>>(out, (int64_t)(packed_one / 2), w, pk);
   LB2_CHECK_LAUNCH("conv_cw_f32 filter packing");
   return LB2_OK;
 }
 
 uint32_t cwf_idesc(int n, bool mn_major) {
   const uint32_t mj = mn_major ? 1u : 0u;
-  return (1u << 4) | (2u << 7) | (2u << 10) | (mj << 15) | (mj << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kFBM >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mj << 15) | (mj << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kFBM >> 4) << 24);
 }
 
 struct CwfTap { int dw, dh, index; };
@@ -766,8 +776,8 @@ struct CwfOut {         // destination of a forward / data-gradient GEMM
   int splits;
   int64_t split_stride;
 };
-int32_t cwf_run(const CwfOut& o, const float* src, const CwfCopy& c, int NI, int chunks, const float* wp, size_t packed_one, int wp_rows,
-                int wp_cols, const CwfTap* taps, int n_taps, int OW, int OH, int sw, int sh, int n_out, cudaStream_t st) {
+int32_t cwf_run(const CwfOut& o, const CwfSource& src, int NI, int chunks, const uint16_t* wp, size_t packed_one, int wp_rows, int wp_cols,
+                const CwfTap* taps, int n_taps, int OW, int OH, int sw, int sh, int n_out, cudaStream_t st) {
   const int bn = cwf_bn(n_out);
   const CwfGrid t = cwf_grid(OW, OH, NI, n_out);
   CwfFwdParams p{};
@@ -784,10 +794,12 @@ int32_t cwf_run(const CwfOut& o, const float* src, const CwfCopy& c, int NI, int
   for (int i = 0; i < n_taps; ++i) {
     p.tap_dw[i] = (int16_t)taps[i].dw; p.tap_dh[i] = (int16_t)taps[i].dh; p.tap_index[i] = (int16_t)taps[i].index;
   }
-  CUtensorMap mXh, mXl, mWh, mWl;
-  if (!cwf_map(&mXh, src, c.Cp, c.W, c.H, NI, t.BW, t.BH, t.BI, sw, sh, false) ||
-      !cwf_map(&mXl, src + c.one / 4, c.Cp, c.W, c.H, NI, t.BW, t.BH, t.BI, sw, sh, false) ||
-      !cwf_map_2d(&mWh, wp, wp_cols, wp_rows, bn) || !cwf_map_2d(&mWl, wp + packed_one / 4, wp_cols, wp_rows, bn))
+  CUtensorMap mX[3], mW[3];
+  bool encoded = true;
+  for (int i = 0; i < 3; ++i)
+    encoded = encoded && cwf_map(&mX[i], src.ptr + i * src.part_stride, src.Cp, src.W, src.H, NI, t.BW, t.BH, t.BI, sw, sh) &&
+              cwf_map_2d(&mW[i], wp + i * (packed_one / 2), wp_cols, wp_rows, bn);
+  if (!encoded)
     return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cuTensorMapEncodeTiled failed");
   const int64_t items = t.tiles() * o.splits;
   LB2_REQUIRE(items <= 0x7FFFFFFF, LB2_BAD_SHAPE, "conv_cw_f32: too many tiles");
@@ -795,7 +807,7 @@ int32_t cwf_run(const CwfOut& o, const float* src, const CwfCopy& c, int NI, int
   auto launch = [&](auto kernel, int smem) -> int32_t {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    kernel<<<grid, kFThreads, smem, st>>>(mXh, mXl, mWh, mWl, p);
+    kernel<<<grid, kFThreads, smem, st>>>(mX[0], mX[1], mX[2], mW[0], mW[1], mW[2], p);
     LB2_CHECK_LAUNCH("conv_cw_f32");
     return LB2_OK;
   };
@@ -863,24 +875,23 @@ bool conv_cwf_supported(const ConvGeom& g) {
 
 size_t conv_cwf_fwd_workspace_bytes(const ConvGeom& g) {
   const int s = cwf_fwd_splits(g);
-  return cwf_copy_x(g).bytes() + 2 * cwf_packed_one(g.cout, cwf_taps(g), cwf_fold(g) ? 1 : cwf_chunks(g.cin)) +
+  return cwf_copy_x(g).bytes() + 3 * cwf_packed_one(g.cout, cwf_taps(g), cwf_fold(g) ? 1 : cwf_chunks(g.cin)) +
          (s > 1 ? align_up((size_t)s * g.out[0] * g.out[1] * g.cout * g.batch * 4, 1024) : 0);
 }
 
-// leaves the channel-innermost hi | lo copy of x at the start of the workspace
 int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const void* bias, const ConvGeom& g, int32_t act, void* ws_,
                      cudaStream_t st) {
   uint8_t* ws = static_cast<uint8_t*>(ws_);
   const int fold = cwf_fold(g), n_taps = cwf_taps(g);
   const CwfCopy xc = cwf_copy_x(g);
-  int32_t rc = cwf_make_copy_x(reinterpret_cast<float*>(ws), (const float*)x, g, xc, st);
+  int32_t rc = cwf_make_copy_x(ws, (const float*)x, g, xc, st);
   if (rc != LB2_OK) return rc;
   CwfPack pk{g.k[0], g.k[1], g.cin, g.cout, g.flip, 0, fold, fold ? 1 : cwf_chunks(g.cin), 0, 0};
   pk.n_rows = (g.cout + cwf_bn(g.cout) - 1) / cwf_bn(g.cout) * cwf_bn(g.cout);
   pk.k_total = n_taps * pk.chunks * 32;
   const size_t packed = cwf_packed_one(g.cout, n_taps, pk.chunks);
-  float* wp = reinterpret_cast<float*>(ws + xc.bytes());
-  rc = cwf_pack(wp, wp + packed / 4, (const float*)w, pk, st);
+  uint16_t* wp = reinterpret_cast<uint16_t*>(ws + xc.bytes());
+  rc = cwf_pack(wp, packed, (const float*)w, pk, st);
   if (rc != LB2_OK) return rc;
   CwfTap taps[kFMaxTaps];
   for (int t = 0; t < n_taps; ++t)
@@ -888,15 +899,15 @@ int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const 
                    : CwfTap{(t % g.k[0]) * g.dil[0] - g.pad_lo[0], (t / g.k[0]) * g.dil[1] - g.pad_lo[1], t};
   const int64_t numel = (int64_t)g.out[0] * g.out[1] * g.cout * g.batch;
   const CwfOut o{(float*)y, (float*)preact, (const float*)bias, act, g.out[0], g.out[1], 1, 0, 1, 0,
-                 reinterpret_cast<float*>(ws + xc.bytes() + 2 * packed), cwf_fwd_splits(g), numel};
-  rc = cwf_run(o, reinterpret_cast<float*>(ws), xc, g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n_taps, g.out[0], g.out[1],
+                 reinterpret_cast<float*>(ws + xc.bytes() + 3 * packed), cwf_fwd_splits(g), numel};
+  rc = cwf_run(o, cwf_source(ws, xc), g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n_taps, g.out[0], g.out[1],
                fold ? 1 : g.stride[0], g.stride[1], g.cout, st);
   return rc != LB2_OK ? rc : cwf_finish(o, numel, g.cout, st);
 }
 
 size_t conv_cwf_bwd_workspace_bytes(const ConvGeom& g) {
   const int s = cwf_dgrad_splits(g);
-  const size_t dgrad = 2 * cwf_packed_one(g.cin, g.k[0] * g.k[1], cwf_chunks(g.cout)) + (s > 1 ? align_up((size_t)s * x_numel(g) * 4, 1024) : 0);
+  const size_t dgrad = 3 * cwf_packed_one(g.cin, g.k[0] * g.k[1], cwf_chunks(g.cout)) + (s > 1 ? align_up((size_t)s * x_numel(g) * 4, 1024) : 0);
   const size_t wgrad = cwf_copy_x(g).bytes() + cwf_wg_plan(g).partial_bytes;
   return cwf_copy_y(g).bytes() + (dgrad > wgrad ? dgrad : wgrad);
 }
@@ -906,17 +917,17 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
                      bool x_is_copy) {
   uint8_t* ws = static_cast<uint8_t*>(ws_);
   const CwfCopy yc = cwf_copy_y(g);
-  float* gcopy = reinterpret_cast<float*>(ws);
-  int32_t rc = cwf_transpose(gcopy, gcopy + yc.one / 4, (const float*)gy, g.out[0] * g.out[1], g.cout, yc.Cp, g.batch, st);
+  const CwfSource gcopy = cwf_source(ws, yc);
+  int32_t rc = cwf_transpose(ws, yc, (const float*)gy, g.out[0] * g.out[1], g.cout, g.batch, st);
   if (rc != LB2_OK) return rc;
   uint8_t* rest = ws + yc.bytes();
 
   if (dw != nullptr) {
     const int fold = cwf_fold(g), n_taps = cwf_taps(g);
     const CwfCopy xc = cwf_copy_x(g);
-    const float* xcopy = reinterpret_cast<const float*>(x_is_copy ? x : rest);
+    const CwfSource xcopy = cwf_source(x_is_copy ? x : rest, xc);
     if (!x_is_copy) {
-      rc = cwf_make_copy_x(reinterpret_cast<float*>(rest), (const float*)x, g, xc, st);
+      rc = cwf_make_copy_x(rest, (const float*)x, g, xc, st);
       if (rc != LB2_OK) return rc;
     }
     const CwfWgPlan pl = cwf_wg_plan(g);
@@ -934,11 +945,13 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
       q.tap_dw[t] = (int16_t)(fold ? 0 : (t % g.k[0]) * g.dil[0] - g.pad_lo[0]);
       q.tap_dh[t] = (int16_t)((fold ? t : t / g.k[0]) * g.dil[1] - g.pad_lo[1]);
     }
-    CUtensorMap mXh, mXl, mGh, mGl;
-    if (!cwf_map(&mXh, xcopy, xc.Cp, xc.W, xc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, q.sw, q.sh, true) ||
-        !cwf_map(&mXl, xcopy + xc.one / 4, xc.Cp, xc.W, xc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, q.sw, q.sh, true) ||
-        !cwf_map(&mGh, gcopy, yc.Cp, yc.W, yc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, 1, 1, true) ||
-        !cwf_map(&mGl, gcopy + yc.one / 4, yc.Cp, yc.W, yc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, 1, 1, true))
+    CUtensorMap mX[3], mG[3];
+    bool encoded = true;
+    for (int i = 0; i < 3; ++i)
+      encoded = encoded &&
+                cwf_map(&mX[i], xcopy.ptr + i * xcopy.part_stride, xc.Cp, xc.W, xc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, q.sw, q.sh) &&
+                cwf_map(&mG[i], gcopy.ptr + i * gcopy.part_stride, yc.Cp, yc.W, yc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, 1, 1);
+    if (!encoded)
       return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cuTensorMapEncodeTiled failed");
     const int64_t items = (int64_t)pl.m_tiles * pl.tiles_n * pl.splits;
     LB2_REQUIRE(items <= 0x7FFFFFFF, LB2_BAD_SHAPE, "conv_cw_f32: too many tiles");
@@ -946,7 +959,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     auto launch = [&](auto kernel, int smem) -> int32_t {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      kernel<<<grid, kFThreads, smem, st>>>(mXh, mXl, mGh, mGl, q);
+      kernel<<<grid, kFThreads, smem, st>>>(mX[0], mX[1], mX[2], mG[0], mG[1], mG[2], q);
       LB2_CHECK_LAUNCH("conv_cw_f32 filter gradient");
       return LB2_OK;
     };
@@ -972,12 +985,12 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     pk.n_rows = (g.cin + cwf_bn(g.cin) - 1) / cwf_bn(g.cin) * cwf_bn(g.cin);
     pk.k_total = g.k[0] * g.k[1] * pk.chunks * 32;
     const size_t packed = cwf_packed_one(g.cin, g.k[0] * g.k[1], pk.chunks);
-    float* wp = reinterpret_cast<float*>(rest);
-    rc = cwf_pack(wp, wp + packed / 4, (const float*)w, pk, st);
+    uint16_t* wp = reinterpret_cast<uint16_t*>(rest);
+    rc = cwf_pack(wp, packed, (const float*)w, pk, st);
     if (rc != LB2_OK) return rc;
     const int sw = g.stride[0], sh = g.stride[1];
     const int64_t numel = x_numel(g);
-    CwfOut o{(float*)dx, nullptr, nullptr, LB2_ACT_IDENTITY, g.in[0], g.in[1], sw, 0, sh, 0, reinterpret_cast<float*>(rest + 2 * packed),
+    CwfOut o{(float*)dx, nullptr, nullptr, LB2_ACT_IDENTITY, g.in[0], g.in[1], sw, 0, sh, 0, reinterpret_cast<float*>(rest + 3 * packed),
              cwf_dgrad_splits(g), numel};
     auto class_taps = [&](int pw, int ph, CwfTap* taps) {
       int n = 0;
@@ -1006,7 +1019,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
         const int n = class_taps(pw, ph, taps);
         if (n == 0) continue;
         o.ow_off = pw; o.oh_off = ph;
-        rc = cwf_run(o, gcopy, yc, g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n, (g.in[0] - pw + sw - 1) / sw,
+        rc = cwf_run(o, gcopy, g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n, (g.in[0] - pw + sw - 1) / sw,
                      (g.in[1] - ph + sh - 1) / sh, 1, 1, g.cin, st);
         if (rc != LB2_OK) return rc;
       }

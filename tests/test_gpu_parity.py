@@ -1085,8 +1085,8 @@ F32_GENERAL_CONV_CASES = [
 @pytest.mark.parametrize("offset", [0, 1])                     # 1: bases that are aligned to the element only
 @pytest.mark.parametrize("case", F32_GENERAL_CONV_CASES)
 def test_fused_conv_f32_general_path(case, offset, act):
-    # 2e-6: three tf32 products drop lo * lo (2^-22 of a product), k-blocks are added in fp32 (at most 400 of them,
-    # random signs); ten times under the contract's 1e-5 for the direct kernels' sequential sums
+    # 2e-6: the products left out are below 2^-25 of a product, k-blocks are added in fp32 (at most 400 of them, random
+    # signs); ten times under the contract's 1e-5 for the direct kernels' sequential sums
     sp, k, cin, cout, stride, pad, dil, flip, batch = case
     rng = np.random.default_rng(61)
     x = rng.standard_normal(sp + (cin, batch)).astype(np.float32)
@@ -1216,3 +1216,37 @@ def test_f32_conv_without_room_for_its_copies():
                             ws.data_ptr(), ws.numel(), None) == 0
     check(dw, dw_ref, "f32", "dw")
     check(dx, dx_ref, "f32", "dx")
+
+
+def _off(got, want):
+    """Relative 2-norm of got - want, and the share of `want` itself in the difference (a loss that always has its sign)."""
+    d = L.to_numpy(got).astype(np.float64) - want
+    return np.linalg.norm(d) / np.linalg.norm(want), abs(np.vdot(d, want)) / np.vdot(want, want)
+
+
+@pytest.mark.parametrize("case", [
+    ((56, 50), (7, 7), 3, 64, 2, 3, 4),        # folded taps
+    ((14, 14), (3, 3), 128, 96, 1, 1, 16),     # 36 k-blocks in one accumulation, filter gradient in segments
+    ((13, 13), (1, 1), 80, 16, 1, 0, 82),      # hundreds of splits of the filter gradient
+    ((28, 28), (1, 1), 64, 128, 2, 0, 8),
+    ((9, 7), (3, 3), 6, 5, 2, 1, 3),           # a handful of terms
+])
+def test_f32_conv_is_as_close_to_64_bits_as_fp32_sums(case):
+    # The tensor cores stand in for the CUDA-core kernels' fp32 multiply-adds, so they may be no further from the exact result
+    # than those are, and their truncating accumulators may not shrink it: 2^-25 is half the rounding unit of fp32, and the
+    # results' own roundings (thousands, either way) share less than that with the result.
+    sp, k, cin, cout, stride, pad, batch = case
+    rng = np.random.default_rng(66)
+    x, w = rng.standard_normal(sp + (cin, batch)).astype(np.float32), O.kaiming_normal(rng, k + (cin, cout)).astype(np.float32)
+    y_ref, pb_ref = O.fused_conv_rrule("identity", w.astype(np.float64), x.astype(np.float64), None, O.ConvDims.make(2, stride, pad, 1, 1, False))
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    want = (y_ref,) + tuple(pb_ref(delta.astype(np.float64))[:2])
+
+    def outputs(flags):
+        y, pb = L.rrule_fused_conv("identity", dev(w, "f32"), dev(x, "f32"), None, L.ConvDims.make(2, stride, pad), flags=flags)
+        return (y,) + tuple(pb(dev(delta, "f32"))[:2])
+    for name, got, fp32, ref in zip(("y", "dw", "dx"), outputs(0), outputs(L._cabi.FLAG_FORCE_SIMT), want):
+        (err, loss), (fp32_err, _) = _off(got, ref), _off(fp32, ref)
+        parity_report.record(name, "f32", err, fp32_err)
+        assert err <= fp32_err, (name, err, fp32_err)
+        assert loss <= (2.0 ** -25 if ref.size > 4096 else 2.0 ** -24), (name, loss)
