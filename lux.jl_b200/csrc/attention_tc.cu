@@ -9,15 +9,15 @@
 // The arrays are read in place through 4-D TMA maps (feature, head, token, sample); either index of an operand may be the
 // contiguous one (K-major / MN-major shared-memory descriptors), so nothing is transposed. A causal mask skips the tiles
 // and the k-blocks that are zero.
-// bf16: kind::f16, one accumulator per tile, two in flight. Float32: hi/lo tf32 operands, three products per k-block,
-// k-blocks added in fp32 registers (the tensor core truncates when it accumulates).
+// bf16: one accumulator per tile, two in flight. Float32: operands in three bf16 parts (parts.cuh), six products per k-block,
+// k-blocks added in fp32 registers.
 //
 // Measured, forward + pullback through the operator, 8 heads x 8 samples, 512 x 512, 64 features, causal, bf16: 130 us (one
 // tensor-core GEMM launch per head, sample and product before: 4.1 ms); Float32 4 x 4, 771 x 771: 300 us (3.07 ms).
 // What bounds it: a contraction over a head's 64 features is one k-block, so the products move the S x L weights and little
 // else; the passes over the weights (in L2 for the usual sizes) are the cost.
 #include "common.cuh"
-#include "tc_ptx.cuh"
+#include "parts.cuh"
 
 namespace lb2 {
 
@@ -37,19 +37,22 @@ struct AtParams {
   int32_t M, N;                      // N rounded up to the vector the rows of D are padded to
   int32_t causal;                    // which of the enum's rules applies to this product
   int32_t wide;                      // rows of D start on 32-byte boundaries: whole sectors per store
-  uint32_t idesc, idesc_wide;
+  uint32_t idesc;
   void* D;
   int64_t ldd, head_stride, batch_stride;
   unsigned int* status;
 };
 
 template <int BN, bool F32> struct AtCfg {
-  static constexpr int A_BYTES = kAtBM * 128, B_BYTES = BN * 128;
-  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES) * (F32 ? 2 : 1);   // F32: [A_hi | A_lo | B_hi | B_lo]
+  static constexpr int ROW = F32 ? 64 : 128;                                // bytes of a k-block's row: 32 / 64 elements
+  static constexpr int A_BYTES = kAtBM * ROW, B_BYTES = BN * ROW;           // one part
+  static constexpr int PARTS = F32 ? 3 : 1;
+  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES) * PARTS;           // F32: [A1 | A2 | A3 | B1 | B2 | B3]
   static constexpr int STAGES = (200 * 1024) / STAGE_BYTES < 6 ? (200 * 1024) / STAGE_BYTES : 6;
-  static constexpr int ACC_COLS = F32 ? 2 * BN : BN;                        // F32: [hi*hi | hi*lo + lo*hi] of one k-block
+  static constexpr int ACC_COLS = F32 ? 2 * BN : BN;                        // F32: [A1*B1 | the small products] of one k-block
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 };
+struct AtMaps { CUtensorMap m[3]; };   // the parts; bf16: the first only
 
 __device__ __forceinline__ void at_load(uint32_t dst, const CUtensorMap* map, const AtOperand& o, int mn, int k, int head, int img,
                                         uint64_t* bar) {
@@ -66,8 +69,7 @@ __device__ __forceinline__ void at_store32(void* p, const uint32_t (&w)[8]) {
 
 template <int BN, bool F32>
 __global__ void __launch_bounds__(kAtThreads, 1)
-attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAl, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmBl, const __grid_constant__ AtParams p) {
+attn_gemm_kernel(const __grid_constant__ AtMaps tmA, const __grid_constant__ AtMaps tmB, const __grid_constant__ AtParams p) {
   using Cfg = AtCfg<BN, F32>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -124,15 +126,14 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait_uniform(&empty[stage], phase ^ 1u, p.status, 0x1u)) { ok = false; break; }
           if (elect_one()) {
             mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-            const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * (F32 ? 2 : 1);
+            const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * Cfg::PARTS;
             const int k0 = kb * p.bk;
-            for (int bx = 0; bx < p.a.boxes; ++bx) {
-              at_load(sA + bx * p.a.box_bytes, &tmA, p.a, t.m0 + bx * p.a.mn_step, k0, ha, t.img, &full[stage]);
-              if constexpr (F32) at_load(sA + Cfg::A_BYTES + bx * p.a.box_bytes, &tmAl, p.a, t.m0 + bx * p.a.mn_step, k0, ha, t.img, &full[stage]);
-            }
-            for (int bx = 0; bx < p.b.boxes; ++bx) {
-              at_load(sB + bx * p.b.box_bytes, &tmB, p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
-              if constexpr (F32) at_load(sB + Cfg::B_BYTES + bx * p.b.box_bytes, &tmBl, p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
+#pragma unroll
+            for (int part = 0; part < Cfg::PARTS; ++part) {
+              for (int bx = 0; bx < p.a.boxes; ++bx)
+                at_load(sA + part * Cfg::A_BYTES + bx * p.a.box_bytes, &tmA.m[part], p.a, t.m0 + bx * p.a.mn_step, k0, ha, t.img, &full[stage]);
+              for (int bx = 0; bx < p.b.boxes; ++bx)
+                at_load(sB + part * Cfg::B_BYTES + bx * p.b.box_bytes, &tmB.m[part], p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
             }
           }
           __syncwarp();
@@ -154,19 +155,15 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4u)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_COLS;
-        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * (F32 ? 2 : 1);
-        const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | p.a.lbo, b32 = ((sB >> 4) & 0x3FFFu) | p.b.lbo;
+        const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * Cfg::PARTS;
+        const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(((sA >> 4) & 0x3FFFu) | p.a.lbo);
+        const uint64_t bd = ((uint64_t)p.b.desc_hi << 32) | (uint64_t)(((sB >> 4) & 0x3FFFu) | p.b.lbo);
         if (elect_one()) {
+          if constexpr (F32) {
+            parts_issue(d_tmem, d_tmem + BN, ad, bd, Cfg::A_BYTES >> 4, Cfg::B_BYTES >> 4, p.a.k_adv, p.b.k_adv, p.idesc, true, nullptr);
+          } else {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            const uint64_t ad = ((uint64_t)p.a.desc_hi << 32) | (uint64_t)(a32 + ks * p.a.k_adv);
-            const uint64_t bd = ((uint64_t)p.b.desc_hi << 32) | (uint64_t)(b32 + ks * p.b.k_adv);
-            if constexpr (F32) {
-              umma<true>(d_tmem, ad, bd, p.idesc_wide, ks != 0 ? 1u : 0u);                       // A_hi * [B_hi ; B_lo]
-              umma<true>(d_tmem + BN, ad + (Cfg::A_BYTES >> 4), bd, p.idesc, 1u);                // A_lo * B_hi
-            } else {
-              umma<false>(d_tmem, ad, bd, p.idesc, (kb | ks) != 0 ? 1u : 0u);
-            }
+            for (int ks = 0; ks < 4; ++ks) umma<false>(d_tmem, ad + ks * p.a.k_adv, bd + ks * p.b.k_adv, p.idesc, (kb | ks) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
           if (F32 || kb == n_kb - 1) umma_commit(&acc_full[acc]);
@@ -209,7 +206,7 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if constexpr (F32) sum[c * 32 + j] += __uint_as_float(vs[j]) + __uint_as_float(v[j]);
+            if constexpr (F32) sum[c * 32 + j] += parts_unbias(__uint_as_float(v[j]), __uint_as_float(vs[j]));
             else sum[c * 32 + j] = __uint_as_float(v[j]);
           }
         }
@@ -269,12 +266,6 @@ attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // ----------------------------------------------------------------------------------------------
 // softmax passes: a warp per query row, four elements per lane and step
 // ----------------------------------------------------------------------------------------------
-__device__ __forceinline__ void at_split(float v, float& hi, float& lo) {
-  uint32_t h;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-  hi = __uint_as_float(h);
-  lo = v - hi;
-}
 template <typename T> struct At4;
 template <> struct At4<float> {
   static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
@@ -306,22 +297,15 @@ template <typename T> __device__ __forceinline__ void at_store_row(T* row, int s
   for (int i = 0; i < 4; ++i)
     if (s + i < S) row[s + i] = from_f32<T>(v[i]);
 }
-// operand copies of a row for the products that follow: rows padded to Sp; Float32 as hi / lo
-template <typename T> __device__ __forceinline__ void at_store_operand(T* hi, T* lo, int64_t off, const float (&v)[4]) {
-  if constexpr (sizeof(T) == 4) {
-    float h[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) at_split(v[i], h[i], l[i]);
-    At4<float>::store(hi + off, h);
-    At4<float>::store(lo + off, l);
-  } else {
-    At4<T>::store(hi + off, v);
-  }
+// operand copies of a row for the products that follow: rows padded to Sp; Float32 in parts
+template <typename T> __device__ __forceinline__ void at_store_operand(uint16_t* op, int64_t part_stride, int64_t off, const float (&v)[4]) {
+  if constexpr (sizeof(T) == 4) store_parts4(op + off, part_stride, v);
+  else At4<T>::store(reinterpret_cast<T*>(op) + off, v);
 }
 
 // NV > 0: rows of at most NV * 128 keys are kept in registers; NV = 0: longer rows are read again for each pass.
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, T* __restrict__ op, T* __restrict__ op_lo, const T* __restrict__ logits,
+__global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, uint16_t* __restrict__ op, int64_t part_stride, const T* __restrict__ logits,
                                                             const T* __restrict__ bias, int64_t bias_bs, const uint8_t* __restrict__ mask,
                                                             int64_t mask_bs, int causal, float scale, int S, int Sp, int L, int64_t rows) {
   const int lane = threadIdx.x & 31;
@@ -387,7 +371,7 @@ __global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, T
   const int op_lim = causal ? min(Sp, (l / kAtBM + 1) * kAtBM) : Sp;   // what the products read of this row
   auto put = [&](int s, float (&v)[4]) {
     at_store_row(w + row * S, s, S, vec, v);
-    if (op != nullptr && s < op_lim) at_store_operand(op, op_lo, row * Sp + s, v);
+    if (op != nullptr && s < op_lim) at_store_operand<T>(op, part_stride, row * Sp + s, v);
   };
   if constexpr (NV > 0) {
 #pragma unroll
@@ -411,10 +395,10 @@ __global__ void __launch_bounds__(256) attn_rows_fwd_kernel(T* __restrict__ w, T
   }
 }
 
-// dl = scale * w .* (dw - sum_s w dw), written over dw (hi / lo for Float32); dbias = dl / scale; op = operand copy of w
+// dl = scale * w .* (dw - sum_s w dw) as an operand (bf16: written over dw); dbias = dl / scale; op = operand copy of w
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) attn_rows_bwd_kernel(T* __restrict__ dl, T* __restrict__ dl_lo, T* __restrict__ dbias, T* __restrict__ op,
-                                                            T* __restrict__ op_lo, const T* __restrict__ w, int causal, float scale, int S,
+__global__ void __launch_bounds__(256) attn_rows_bwd_kernel(uint16_t* dl, const T* dw, T* __restrict__ dbias, uint16_t* __restrict__ op,
+                                                            int64_t part_stride, const T* __restrict__ w, int causal, float scale, int S,
                                                             int Sp, int L, int64_t rows) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -424,7 +408,7 @@ __global__ void __launch_bounds__(256) attn_rows_bwd_kernel(T* __restrict__ dl, 
   const int op_lim = causal ? min(Sp, (l / kAtBM + 1) * kAtBM) : Sp;
   const bool vec = S % 4 == 0;
   const T* wr = w + row * S;
-  T* g = dl + row * Sp;
+  const T* g = dw + row * Sp;
   float rw[NV > 0 ? NV : 1][4], rg[NV > 0 ? NV : 1][4];
   auto get = [&](int s, float (&a)[4], float (&b)[4]) {
     if (s < lim) {
@@ -461,8 +445,8 @@ __global__ void __launch_bounds__(256) attn_rows_bwd_kernel(T* __restrict__ dl, 
     for (int k = 0; k < 4; ++k) { d[k] = a[k] * (b[k] - dot); e[k] = d[k] * scale; }
     if (dbias != nullptr) at_store_row(dbias + row * S, s, S, vec, d);
     if (s < op_lim) {
-      at_store_operand(dl, dl_lo, row * Sp + s, e);
-      if (op != nullptr) at_store_operand(op, op_lo, row * Sp + s, a);
+      at_store_operand<T>(dl, part_stride, row * Sp + s, e);
+      if (op != nullptr) at_store_operand<T>(op, part_stride, row * Sp + s, a);
     }
   };
   if constexpr (NV > 0) {
@@ -480,57 +464,59 @@ __global__ void __launch_bounds__(256) attn_rows_bwd_kernel(T* __restrict__ dl, 
   }
 }
 
-__global__ void __launch_bounds__(256) attn_split_kernel(float* __restrict__ hi, float* __restrict__ lo, const float* __restrict__ x, int64_t n4) {
+// rows of `features` (a multiple of 4) floats -> three parts, rows padded to `ld`
+__global__ void __launch_bounds__(256) attn_split_kernel(uint16_t* __restrict__ out, int64_t part_stride, const float* __restrict__ x, int64_t n4,
+                                                         int quads, int ld) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-    float v[4], h[4], l[4];
+    const int64_t row = i / quads;
+    float v[4];
     At4<float>::load(x + i * 4, v);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) at_split(v[k], h[k], l[k]);
-    At4<float>::store(hi + i * 4, h);
-    At4<float>::store(lo + i * 4, l);
+    store_parts4(out + row * ld + (i - row * quads) * 4, part_stride, v);
   }
 }
 
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
-// An operand: (feature, head, token, sample) arrays [head_first] or (key, query, head, sample) arrays of weights.
+// An operand: (feature, head, token, sample) arrays [head_first] or (key, query, head, sample) arrays of weights; 2-byte elements
+// (bf16, or a part of a Float32 value; the parts `part_stride` elements apart).
 struct AtArray {
   const void* ptr;
-  const void* lo;                    // Float32: the low parts
+  int64_t part_stride;
   int64_t inner, outer, ld, heads, head_stride, batch_stride;
   bool head_first;
 };
 
-bool at_encode(CUtensorMap* map, const void* ptr, const AtArray& t, int64_t batch, int es, int box_outer, bool atom32) {
+bool at_encode(CUtensorMap* map, const void* ptr, const AtArray& t, int64_t batch, bool f32, int box_outer) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
   const int o = t.head_first ? 2 : 1, h = t.head_first ? 1 : 2;
   cuuint64_t dims[4], strides[3];
-  cuuint32_t box[4] = {(cuuint32_t)(128 / es), 1, 1, 1}, estr[4] = {1, 1, 1, 1};
+  cuuint32_t box[4] = {f32 ? 32u : 64u, 1, 1, 1}, estr[4] = {1, 1, 1, 1};
   dims[0] = (cuuint64_t)t.inner; dims[o] = (cuuint64_t)t.outer; dims[h] = (cuuint64_t)t.heads; dims[3] = (cuuint64_t)batch;
-  strides[o - 1] = (cuuint64_t)(t.ld * es); strides[h - 1] = (cuuint64_t)(t.head_stride * es); strides[2] = (cuuint64_t)(t.batch_stride * es);
+  strides[o - 1] = (cuuint64_t)(t.ld * 2); strides[h - 1] = (cuuint64_t)(t.head_stride * 2); strides[2] = (cuuint64_t)(t.batch_stride * 2);
   box[o] = (cuuint32_t)box_outer;
-  return enc(map, es == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides, box,
-             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             f32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-bool at_operand(CUtensorMap* hi, CUtensorMap* lo, const AtArray& t, bool mn_major, int head_div, int64_t batch, int es, int tile_mn, AtOperand* o) {
-  const int row = 128 / es;          // elements per 128-byte row = k-block depth
-  const bool atom32 = es == 4 && mn_major;
+bool at_operand(AtMaps* maps, const AtArray& t, bool mn_major, int head_div, int64_t batch, bool f32, int tile_mn, AtOperand* o) {
+  const int row = f32 ? 32 : 64, row_bytes = row * 2;   // a k-block's row: its depth, or the elements of the other index in a box
   o->mn_major = mn_major; o->head_first = t.head_first; o->head_div = head_div;
   if (mn_major) {
-    o->boxes = tile_mn / row; o->box_bytes = row * 128; o->mn_step = row;
+    o->boxes = tile_mn / row; o->box_bytes = row * row_bytes; o->mn_step = row;
     o->lbo = ((uint32_t)(o->box_bytes >> 4) & 0x3FFFu) << 16;
-    o->k_adv = (uint32_t)(((es == 4 ? 8 : 16) * 128) >> 4);
+    o->k_adv = (uint32_t)((16 * row_bytes) >> 4);
   } else {
-    o->boxes = 1; o->box_bytes = tile_mn * 128; o->mn_step = 0;
+    o->boxes = 1; o->box_bytes = tile_mn * row_bytes; o->mn_step = 0;
     o->lbo = 1u << 16;
     o->k_adv = 2u;
   }
-  o->desc_hi = (uint32_t)(((atom32 ? 512u : 1024u) >> 4) & 0x3FFFu) | (1u << 14) | ((atom32 ? 1u : 2u) << 29);
-  const int outer_box = mn_major ? row : tile_mn;
-  return at_encode(hi, t.ptr, t, batch, es, outer_box, atom32) && at_encode(lo, es == 4 ? t.lo : t.ptr, t, batch, es, outer_box, atom32);
+  // eight-row swizzle atoms of 128-byte (2) or 64-byte (4) rows
+  o->desc_hi = ((uint32_t)((8 * row_bytes) >> 4) & 0x3FFFu) | (1u << 14) | ((f32 ? 4u : 2u) << 29);
+  for (int i = 0; i < (f32 ? 3 : 1); ++i)
+    if (!at_encode(&maps->m[i], static_cast<const uint16_t*>(t.ptr) + i * t.part_stride, t, batch, f32, mn_major ? row : tile_mn)) return false;
+  return true;
 }
 
 struct AtProduct {
@@ -544,21 +530,20 @@ struct AtProduct {
 };
 int32_t at_gemm(const AtProduct& g, int64_t batch, int32_t dtype, cudaStream_t st) {
   const int es = (int)dtype_size(dtype);
+  const bool f32 = dtype == LB2_F32;
   const int bn = g.N <= 64 ? 64 : 128;
   AtParams p{};
-  CUtensorMap mA, mAl, mB, mBl;
-  if (!at_operand(&mA, &mAl, g.A, g.a_mn, g.a_div, batch, es, kAtBM, &p.a) || !at_operand(&mB, &mBl, g.B, g.b_mn, g.b_div, batch, es, bn, &p.b))
+  AtMaps mA{}, mB{};
+  if (!at_operand(&mA, g.A, g.a_mn, g.a_div, batch, f32, kAtBM, &p.a) || !at_operand(&mB, g.B, g.b_mn, g.b_div, batch, f32, bn, &p.b))
     return fail(LB2_LAUNCH_FAIL, "attention: cuTensorMapEncodeTiled failed");
-  p.bk = 128 / es;
+  p.bk = f32 ? 32 : 64;
   p.M = (int)g.M; p.N = (int)g.n_store;
   p.tiles_m = (int)((g.M + kAtBM - 1) / kAtBM); p.tiles_n = (int)((g.N + bn - 1) / bn);
   p.heads = (int)g.heads; p.rep = (int)g.rep; p.batch = (int)batch;
   p.num_kb = (int)((g.K + p.bk - 1) / p.bk);
   p.causal = g.causal;
-  const uint32_t fmt = es == 4 ? 2u : 1u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((g.a_mn ? 1u : 0u) << 15) | ((g.b_mn ? 1u : 0u) << 16) | ((uint32_t)(bn >> 3) << 17) |
+  p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((g.a_mn ? 1u : 0u) << 15) | ((g.b_mn ? 1u : 0u) << 16) | ((uint32_t)(bn >> 3) << 17) |
             ((uint32_t)(kAtBM >> 4) << 24);
-  p.idesc_wide = (p.idesc & ~(0x3Fu << 17)) | ((uint32_t)((2 * bn) >> 3) << 17);
   p.wide = aligned_to(g.D, 32) && (g.ldd * es) % 32 == 0 && (g.head_stride * es) % 32 == 0 && (g.batch_stride * es) % 32 == 0;
   p.D = g.D; p.ldd = g.ldd; p.head_stride = g.head_stride; p.batch_stride = g.batch_stride;
   p.status = device_status_word();
@@ -568,18 +553,24 @@ int32_t at_gemm(const AtProduct& g, int64_t batch, int32_t dtype, cudaStream_t s
   auto launch = [&](auto kernel, int smem) -> int32_t {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "attention: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    kernel<<<grid, kAtThreads, smem, st>>>(mA, mAl, mB, mBl, p);
+    kernel<<<grid, kAtThreads, smem, st>>>(mA, mB, p);
     LB2_CHECK_LAUNCH("attention product");
     return LB2_OK;
   };
-  if (es == 4) return bn == 64 ? launch(attn_gemm_kernel<64, true>, AtCfg<64, true>::SMEM_BYTES) : launch(attn_gemm_kernel<128, true>, AtCfg<128, true>::SMEM_BYTES);
+  if (f32) return bn == 64 ? launch(attn_gemm_kernel<64, true>, AtCfg<64, true>::SMEM_BYTES) : launch(attn_gemm_kernel<128, true>, AtCfg<128, true>::SMEM_BYTES);
   return bn == 64 ? launch(attn_gemm_kernel<64, false>, AtCfg<64, false>::SMEM_BYTES) : launch(attn_gemm_kernel<128, false>, AtCfg<128, false>::SMEM_BYTES);
 }
 
 int64_t at_pad(int64_t S) { return (S + 7) / 8 * 8; }
 size_t at_bytes(int64_t elems, int es) { return align_up((size_t)elems * es, 1024); }
-// weights need an operand copy of their own: hi / lo for Float32, padded rows where S breaks the 16-byte stride rule
+// weights need an operand copy of their own: parts for Float32, padded rows where S breaks the 16-byte stride rule
 bool at_needs_copy(const lb2_attention_dims& d, int es) { return es == 4 || d.keys % 8 != 0; }
+// an operand copy of n elements: bf16, or the three parts of Float32
+size_t at_operand_bytes(int64_t n, int es) { return at_bytes(n, 2) * (es == 4 ? 3 : 1); }
+int64_t at_part_stride(int64_t n) { return (int64_t)(at_bytes(n, 2) / 2); }
+// Float32 token arrays are copied into parts, rows padded to the 16-byte rule
+int64_t at_token_ld(int64_t features, int es) { return es == 4 ? at_pad(features) : features; }
+size_t at_token_bytes(int64_t features, int64_t rows, int es) { return es == 4 ? at_operand_bytes(at_pad(features) * rows, es) : 0; }
 
 int32_t at_check(const lb2_attention_dims* d, int32_t dtype) {
   LB2_REQUIRE(valid_dtype(dtype), LB2_UNSUPPORTED_DTYPE, "dtype %d not supported", (int)dtype);
@@ -588,26 +579,21 @@ int32_t at_check(const lb2_attention_dims* d, int32_t dtype) {
   return LB2_OK;
 }
 
-// feature-major array (features, heads, tokens, samples)
-AtArray at_tokens(const void* ptr, const void* lo, int64_t features, int64_t heads, int64_t tokens) {
-  return AtArray{ptr, lo, features, tokens, features * heads, heads, features, features * heads * tokens, true};
-}
 // weights (keys padded to ld, queries, heads, samples)
-AtArray at_weights(const void* ptr, const void* lo, int64_t keys, int64_t ld, int64_t queries, int64_t heads) {
-  return AtArray{ptr, lo, keys, queries, ld, heads, ld * queries, ld * queries * heads, false};
+AtArray at_weights(const void* ptr, int64_t part_stride, int64_t keys, int64_t ld, int64_t queries, int64_t heads) {
+  return AtArray{ptr, part_stride, keys, queries, ld, heads, ld * queries, ld * queries * heads, false};
 }
-
-// Float32: hi / lo copies of an array in the workspace; bf16: the array itself
-int32_t at_split_array(const void** hi, const void** lo, const void* x, int64_t n, int es, uint8_t** ws, cudaStream_t st) {
-  *hi = x; *lo = x;
+// feature-major array (features, heads, tokens, samples): bf16 in place, Float32 as a copy in the workspace
+int32_t at_tokens(AtArray* out, const void* x, int64_t features, int64_t heads, int64_t tokens, int64_t batch, int es, uint8_t** ws, cudaStream_t st) {
+  const int64_t ld = at_token_ld(features, es), rows = heads * tokens * batch;
+  *out = AtArray{x, 0, features, tokens, ld * heads, heads, ld, ld * heads * tokens, true};
   if (es == 2) return LB2_OK;
-  float* h = reinterpret_cast<float*>(*ws);
-  float* l = h + at_bytes(n, 4) / 4;
-  *ws += 2 * at_bytes(n, 4);
-  const int64_t blocks = (n / 4 + 255) / 256, cap = (int64_t)sm_count() * 8;
-  attn_split_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(h, l, (const float*)x, n / 4);
+  out->ptr = *ws; out->part_stride = at_part_stride(ld * rows);
+  const int64_t n4 = features / 4 * rows, blocks = (n4 + 255) / 256, cap = (int64_t)sm_count() * 8;
+  attn_split_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(reinterpret_cast<uint16_t*>(*ws), out->part_stride, (const float*)x, n4,
+                                                                            (int)(features / 4), (int)ld);
   LB2_CHECK_LAUNCH("attention split");
-  *hi = h; *lo = l;
+  *ws += at_token_bytes(features, rows, es);
   return LB2_OK;
 }
 
@@ -646,12 +632,9 @@ size_t lb2_attention_fwd_workspace_bytes(const lb2_attention_dims* d, int32_t dt
   if (lb2_attention_is_fused(d, dtype) != 1) return 0;
   const int es = (int)dtype_size(dtype);
   const int64_t w = at_pad(d->keys) * d->queries * d->heads * d->batch;
-  size_t n = at_bytes(w, es);
-  if (at_needs_copy(*d, es)) n += at_bytes(w, es) * (es == 4 ? 2 : 1);
-  if (es == 4)
-    n += 2 * (at_bytes(d->head_dim * d->heads * d->queries * d->batch, 4) + at_bytes(d->head_dim * d->kv_heads * d->keys * d->batch, 4) +
-              at_bytes(d->value_dim * d->kv_heads * d->keys * d->batch, 4));
-  return n;
+  const int64_t qr = d->heads * d->queries * d->batch, kr = d->kv_heads * d->keys * d->batch;
+  return at_bytes(w, es) + (at_needs_copy(*d, es) ? at_operand_bytes(w, es) : 0) + at_token_bytes(d->head_dim, qr, es) +
+         at_token_bytes(d->head_dim, kr, es) + at_token_bytes(d->value_dim, kr, es);
 }
 
 int32_t lb2_attention_fwd(void* x, void* w, const void* q, const void* k, const void* v, const void* bias, int64_t bias_batch_stride,
@@ -673,26 +656,23 @@ int32_t lb2_attention_fwd(void* x, void* w, const void* q, const void* k, const 
   const int es = (int)dtype_size(dtype);
   const int gs = (int)(H / d->kv_heads);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  const size_t wb = at_bytes(Sp * L * H * B, es);
-  void* logits = ws; ws += wb;
-  void *op = nullptr, *op_lo = nullptr;
-  if (at_needs_copy(*d, es)) { op = ws; ws += wb; }
-  if (es == 4) { op_lo = ws; ws += wb; }
-  const void *qh, *ql, *kh, *kl, *vh, *vl;
-  if ((rc = at_split_array(&qh, &ql, q, d->head_dim * H * L * B, es, &ws, st)) != LB2_OK) return rc;
-  if ((rc = at_split_array(&kh, &kl, k, d->head_dim * d->kv_heads * S * B, es, &ws, st)) != LB2_OK) return rc;
-  if ((rc = at_split_array(&vh, &vl, v, d->value_dim * d->kv_heads * S * B, es, &ws, st)) != LB2_OK) return rc;
-  const AtArray Q = at_tokens(qh, ql, d->head_dim, H, L), K = at_tokens(kh, kl, d->head_dim, d->kv_heads, S),
-                V = at_tokens(vh, vl, d->value_dim, d->kv_heads, S);
+  const int64_t wn = Sp * L * H * B, wps = at_part_stride(wn);
+  void* logits = ws; ws += at_bytes(wn, es);
+  uint16_t* op = nullptr;
+  if (at_needs_copy(*d, es)) { op = reinterpret_cast<uint16_t*>(ws); ws += at_operand_bytes(wn, es); }
+  AtArray Q, K, V;
+  if ((rc = at_tokens(&Q, q, d->head_dim, H, L, B, es, &ws, st)) != LB2_OK) return rc;
+  if ((rc = at_tokens(&K, k, d->head_dim, d->kv_heads, S, B, es, &ws, st)) != LB2_OK) return rc;
+  if ((rc = at_tokens(&V, v, d->value_dim, d->kv_heads, S, B, es, &ws, st)) != LB2_OK) return rc;
   rc = at_gemm(AtProduct{Q, K, false, false, 1, gs, L, S, d->head_dim, H, 1, causal ? kCausalTiles : kCausalNone, logits, Sp, Sp, Sp * L, Sp * L * H},
                B, dtype, st);
   if (rc != LB2_OK) return rc;
   LB2_DISPATCH_DTYPE(dtype, {
-    LB2_AT_ROWS(attn_rows_fwd_kernel, T, S, (T*)w, (T*)op, (T*)op_lo, (const T*)logits, (const T*)bias, bias_batch_stride, mask, mask_batch_stride,
+    LB2_AT_ROWS(attn_rows_fwd_kernel, T, S, (T*)w, op, wps, (const T*)logits, (const T*)bias, bias_batch_stride, mask, mask_batch_stride,
                 causal, (float)scale, (int)S, (int)Sp, (int)L, rows);
   });
   LB2_CHECK_LAUNCH("attention softmax");
-  const AtArray W = op != nullptr ? at_weights(op, op_lo, S, Sp, L, H) : at_weights(w, w, S, S, L, H);
+  const AtArray W = op != nullptr ? at_weights(op, wps, S, Sp, L, H) : at_weights(w, 0, S, S, L, H);
   return at_gemm(AtProduct{W, V, false, true, 1, gs, L, d->value_dim, S, H, 1, causal ? kCausalKeys : kCausalNone, x, d->value_dim,
                            d->value_dim * H, d->value_dim, d->value_dim * H * L},
                  B, dtype, st);
@@ -702,12 +682,10 @@ size_t lb2_attention_bwd_workspace_bytes(const lb2_attention_dims* d, int32_t dt
   if (lb2_attention_is_fused(d, dtype) != 1) return 0;
   const int es = (int)dtype_size(dtype);
   const int64_t w = at_pad(d->keys) * d->queries * d->heads * d->batch;
-  size_t n = at_bytes(w, es) * (es == 4 ? 2 : 1);
-  if (at_needs_copy(*d, es)) n += at_bytes(w, es) * (es == 4 ? 2 : 1);
-  if (es == 4)
-    n += 2 * (at_bytes(d->head_dim * d->heads * d->queries * d->batch, 4) + at_bytes(d->value_dim * d->heads * d->queries * d->batch, 4) +
-              at_bytes(d->head_dim * d->kv_heads * d->keys * d->batch, 4) + at_bytes(d->value_dim * d->kv_heads * d->keys * d->batch, 4));
-  return n;
+  const int64_t qr = d->heads * d->queries * d->batch, kr = d->kv_heads * d->keys * d->batch;
+  return at_bytes(w, es) + (es == 4 ? at_operand_bytes(w, es) : 0) + (at_needs_copy(*d, es) ? at_operand_bytes(w, es) : 0) +
+         at_token_bytes(d->head_dim, qr, es) + at_token_bytes(d->value_dim, qr, es) + at_token_bytes(d->head_dim, kr, es) +
+         at_token_bytes(d->value_dim, kr, es);
 }
 
 int32_t lb2_attention_bwd(void* dq, void* dk, void* dv, void* dbias, const void* dx, const void* w, const void* q, const void* k, const void* v,
@@ -728,26 +706,23 @@ int32_t lb2_attention_bwd(void* dq, void* dk, void* dv, void* dbias, const void*
   const int es = (int)dtype_size(dtype);
   const int gs = (int)(H / Hkv);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  const size_t wb = at_bytes(Sp * L * H * B, es);
-  void* dl = ws; ws += wb;               // dw, then dlogits over it
-  void *dl_lo = nullptr, *op = nullptr, *op_lo = nullptr;
-  if (es == 4) { dl_lo = ws; ws += wb; }
-  if (at_needs_copy(*d, es)) { op = ws; ws += wb; }
-  if (es == 4) { op_lo = ws; ws += wb; }
-  const void *qh, *ql, *kh, *kl, *vh, *vl, *gh, *gl;
-  if ((rc = at_split_array(&qh, &ql, q, D * H * L * B, es, &ws, st)) != LB2_OK) return rc;
-  if ((rc = at_split_array(&gh, &gl, dx, E * H * L * B, es, &ws, st)) != LB2_OK) return rc;
-  if ((rc = at_split_array(&kh, &kl, k, D * Hkv * S * B, es, &ws, st)) != LB2_OK) return rc;
-  if ((rc = at_split_array(&vh, &vl, v, E * Hkv * S * B, es, &ws, st)) != LB2_OK) return rc;
-  const AtArray Q = at_tokens(qh, ql, D, H, L), G = at_tokens(gh, gl, E, H, L), K = at_tokens(kh, kl, D, Hkv, S), V = at_tokens(vh, vl, E, Hkv, S);
-  rc = at_gemm(AtProduct{G, V, false, false, 1, gs, L, S, E, H, 1, causal ? kCausalTiles : kCausalNone, dl, Sp, Sp, Sp * L, Sp * L * H}, B, dtype, st);
+  const int64_t wn = Sp * L * H * B, wps = at_part_stride(wn);
+  void* dw = ws; ws += at_bytes(wn, es);
+  uint16_t *dl = static_cast<uint16_t*>(dw), *op = nullptr;       // bf16: dlogits over dw
+  if (es == 4) { dl = reinterpret_cast<uint16_t*>(ws); ws += at_operand_bytes(wn, es); }
+  if (at_needs_copy(*d, es)) { op = reinterpret_cast<uint16_t*>(ws); ws += at_operand_bytes(wn, es); }
+  AtArray Q, G, K, V;
+  if ((rc = at_tokens(&Q, q, D, H, L, B, es, &ws, st)) != LB2_OK) return rc;
+  if ((rc = at_tokens(&G, dx, E, H, L, B, es, &ws, st)) != LB2_OK) return rc;
+  if ((rc = at_tokens(&K, k, D, Hkv, S, B, es, &ws, st)) != LB2_OK) return rc;
+  if ((rc = at_tokens(&V, v, E, Hkv, S, B, es, &ws, st)) != LB2_OK) return rc;
+  rc = at_gemm(AtProduct{G, V, false, false, 1, gs, L, S, E, H, 1, causal ? kCausalTiles : kCausalNone, dw, Sp, Sp, Sp * L, Sp * L * H}, B, dtype, st);
   if (rc != LB2_OK) return rc;
   LB2_DISPATCH_DTYPE(dtype, {
-    LB2_AT_ROWS(attn_rows_bwd_kernel, T, S, (T*)dl, (T*)dl_lo, (T*)dbias, (T*)op, (T*)op_lo, (const T*)w, causal, (float)scale, (int)S, (int)Sp,
-                (int)L, rows);
+    LB2_AT_ROWS(attn_rows_bwd_kernel, T, S, dl, (const T*)dw, (T*)dbias, op, wps, (const T*)w, causal, (float)scale, (int)S, (int)Sp, (int)L, rows);
   });
   LB2_CHECK_LAUNCH("attention softmax backward");
-  const AtArray W = op != nullptr ? at_weights(op, op_lo, S, Sp, L, H) : at_weights(w, w, S, S, L, H), DL = at_weights(dl, dl_lo, S, Sp, L, H);
+  const AtArray W = op != nullptr ? at_weights(op, wps, S, Sp, L, H) : at_weights(w, 0, S, S, L, H), DL = at_weights(dl, wps, S, Sp, L, H);
   rc = at_gemm(AtProduct{DL, K, false, true, 1, gs, L, D, S, H, 1, causal ? kCausalKeys : kCausalNone, dq, D, D * H, D, D * H * L}, B, dtype, st);
   if (rc != LB2_OK) return rc;
   const int cq = causal ? kCausalQueries : kCausalNone;

@@ -1250,3 +1250,25 @@ def test_f32_conv_is_as_close_to_64_bits_as_fp32_sums(case):
         parity_report.record(name, "f32", err, fp32_err)
         assert err <= fp32_err, (name, err, fp32_err)
         assert loss <= (2.0 ** -25 if ref.size > 4096 else 2.0 ** -24), (name, loss)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dims", [(32, 2, 1, 100, 60, 2), (64, 2, 2, 43, 43, 4), (128, 2, 2, 64, 64, 1), (64, 4, 2, 200, 330, 1), (20, 2, 2, 140, 140, 2)])
+def test_f32_attention_is_as_close_to_64_bits_as_fp32_sums(dims, causal):
+    # as for the convolutions; the products of these sizes were fp32 multiply-adds. 2^-23: up to four products and two row
+    # passes follow one another, each allowed its 2^-25
+    D, H, Hkv, Lq, S, B = dims
+    rng = np.random.default_rng(67)
+    q, k, v, dx = (rng.standard_normal(s).astype(np.float32) for s in ((D, H, Lq, B), (D, Hkv, S, B), (D, Hkv, S, B), (D, H, Lq, B)))
+    causal = causal or None
+    (x_ref, w_ref), pb_ref = O.attention_rrule(*(a.astype(np.float64) for a in (q, k, v)), is_causal=causal)
+    want = (x_ref, w_ref) + tuple(pb_ref(dx.astype(np.float64))[:3])
+
+    def outputs(flags):
+        (x, w), pb = L.rrule_scaled_dot_product_attention(dev(q, "f32"), dev(k, "f32"), dev(v, "f32"), is_causal=causal, flags=flags)
+        return (x, w) + tuple(pb(dev(dx, "f32"))[:3])
+    for name, got, fp32, ref in zip(("x", "w", "dq", "dk", "dv"), outputs(0), outputs(L._cabi.FLAG_FORCE_SIMT), want):
+        (err, loss), (fp32_err, _) = _off(got, ref), _off(fp32, ref)
+        parity_report.record(name, "f32", err, fp32_err)
+        assert err <= fp32_err, (name, err, fp32_err)
+        assert loss <= 2.0 ** -23, (name, loss)
