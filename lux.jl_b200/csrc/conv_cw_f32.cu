@@ -6,6 +6,10 @@
 // sum over all positions, goes to memory in segments of kSegment k-blocks, so that no register adds up more than that many, and
 // its splits are added with a compensated sum.
 //
+// Zero-filled positions outside the arrays, which are no terms of the sum, make NaN of an infinity or NaN on the other side:
+// elements that come out as NaN are formed again, term by term, by the warp that stored them (cwf_redo_*). Ordinary data never
+// gets there.
+//
 //   layout       x (and dy) are rewritten channel-innermost, three parts (one pass: read 4 bytes, write 6 per element); a tap
 //                shift, the padding and the stride are then start coordinates / box parameters of a 4-D TMA map
 //   forward      M = 128 output positions (a w x h x image box), N = 64 / 128 output channels, both operands K-major
@@ -269,11 +273,22 @@ constexpr uint32_t kLboK = 1u << 16, kAdvK = 2u;
 // 64 bytes per MMA step
 constexpr uint32_t kLboMN = ((2048u >> 4) & 0x3FFFu) << 16, kAdvMN = (16u * 64u) >> 4;
 
-// A channel-innermost array of parts
+// A channel-innermost array of parts and what of it exists; the taps a folded copy (fold = cin) holds beside one another
 struct CwfSource {
   const uint16_t* ptr;
   int64_t part_stride;
   int32_t Cp, W, H;
+  int32_t fold, fold_step, fold_dil, fold_pad, fold_W;
+  // channel c of position (w, h, img) belongs to the arrays
+  __device__ __forceinline__ bool has(int c, int w, int h) const {
+    if (c >= Cp || w < 0 || w >= W || h < 0 || h >= H) return false;
+    if (fold == 0) return true;
+    const int iw = w * fold_step + (c / fold) * fold_dil - fold_pad;
+    return iw >= 0 && iw < fold_W;
+  }
+  __device__ __forceinline__ float at(int c, int w, int h, int img) const {
+    return join_parts(ptr + (((int64_t)img * H + h) * W + w) * Cp + c, part_stride);
+  }
 };
 
 struct CwfFwdParams {
@@ -292,6 +307,10 @@ struct CwfFwdParams {
   int64_t split_stride;
   int32_t act;
   unsigned int* status;
+  CwfSource src;
+  const uint16_t* wp;          // packed filter
+  int64_t wp_part_stride;
+  int32_t wp_cols;
   int16_t tap_dw[kFMaxTaps], tap_dh[kFMaxTaps], tap_index[kFMaxTaps];
 
   // item -> (channel tile fastest, w tile, h tile, image tile, split)
@@ -306,6 +325,51 @@ struct CwfFwdParams {
     return (int64_t)(a * ow_step + ow_off) + (int64_t)FW * (b * oh_step + oh_off) + (int64_t)FW * FH * ((int64_t)n_out * img + col);
   }
 };
+
+// A warp's elements that came out as NaN once more, as the sum of their terms (positions outside the arrays are none). The lanes
+// share an element's channels. A NaN among the terms stays NaN and ends the sum early.
+template <int BN>
+__device__ __noinline__ void cwf_redo_fwd(const CwfFwdParams& p, int q, int half) {
+  constexpr int COLS = BN / 2;
+  const int lane = threadIdx.x & 31, pos = q * 32 + lane;
+  const int iw = pos % p.BW, ih = (pos / p.BW) % p.BH, ii = pos / (p.BW * p.BH);
+  const int num_items = p.tiles_w * p.tiles_h * p.tiles_i * p.tiles_n * p.splits;
+  for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+    int tn, tw, th, ti, z;
+    p.item_coords(item, &tn, &tw, &th, &ti, &z);
+    const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
+    const int a = tw * p.BW + iw, b = th * p.BH + ih, img = ti * p.BI + ii;
+    const bool live = ii < p.BI && a < p.OW && b < p.OH && img < p.NI;
+    for (int j = 0; j < COLS; ++j) {
+      const int col = tn * BN + half * COLS + j;
+      if (col >= p.n_out) break;
+      const int64_t out = p.out_index(a, b, img, col);
+      float* const dst = p.splits > 1 ? p.partial + z * p.split_stride + out : p.y + out;
+      const float old = live ? *dst : 0.f;
+      for (uint32_t todo = __ballot_sync(0xffffffffu, old != old); todo != 0; todo &= todo - 1) {
+        const int who = __ffs(todo) - 1;
+        const int wa = __shfl_sync(0xffffffffu, a, who) * p.sw, wb = __shfl_sync(0xffffffffu, b, who) * p.sh, wi = __shfl_sync(0xffffffffu, img, who);
+        float sum = 0.f;
+        for (int kb = kb_lo; kb < kb_hi && !__any_sync(0xffffffffu, sum != sum); ++kb) {
+          const int tap = kb / p.chunks, c = (kb - tap * p.chunks) * 32 + lane;
+          const int w = wa + p.tap_dw[tap], h = wb + p.tap_dh[tap];
+          if (p.src.has(c, w, h))
+            sum = fmaf(p.src.at(c, w, h, wi),
+                       join_parts(p.wp + (int64_t)col * p.wp_cols + p.tap_index[tap] * p.chunks * 32 + c, p.wp_part_stride), sum);
+        }
+        sum = warp_sum(sum);
+        if (lane == who) {
+          if (p.splits == 1) {
+            if (p.bias != nullptr) sum += __ldg(p.bias + col);
+            if (p.preact != nullptr) p.preact[out] = sum;
+            sum = act_apply_any<-1, false>(p.act, sum);
+          }
+          *dst = sum;
+        }
+      }
+    }
+  }
+}
 
 template <int BN, int ACT>
 __global__ void __launch_bounds__(kFThreads, 1)
@@ -392,7 +456,7 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
     const int64_t plane = (int64_t)p.FW * p.FH;
     const int pos = q * 32 + lane;
     const int iw = pos % p.BW, ih = (pos / p.BW) % p.BH, ii = pos / (p.BW * p.BH);
-    bool ok = true;
+    bool nan = false, ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       int tn, tw, th, ti, z;
       p.item_coords(item, &tn, &tw, &th, &ti, &z);
@@ -412,7 +476,7 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
           float* d = p.partial + z * p.split_stride + base;
 #pragma unroll
           for (int j = 0; j < COLS; ++j)
-            if (col0 + j < p.n_out) d[j * plane] = sum[j];
+            if (col0 + j < p.n_out) { d[j * plane] = sum[j]; nan |= sum[j] != sum[j]; }
         } else {
           float* yp = p.y + base;
           float* pp = p.preact != nullptr ? p.preact + base : nullptr;
@@ -421,12 +485,15 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
             if (col0 + j < p.n_out) {
               const float v = sum[j] + (p.bias != nullptr ? __ldg(p.bias + col0 + j) : 0.f);
               if (pp != nullptr) pp[j * plane] = v;
-              yp[j * plane] = act_apply_any<ACT, false>(p.act, v);
+              yp[j * plane] = v == v ? act_apply_any<ACT, false>(p.act, v) : v;   // cwf_redo_fwd finds it by its value
+              nan |= v != v;
             }
           }
         }
       }
+      __syncwarp();
     }
+    if (ok && __any_sync(0xffffffffu, nan)) cwf_redo_fwd<BN>(p, q, half);
   }
 
   tc_fence_before();
@@ -457,12 +524,45 @@ struct CwfWgParams {
   int32_t kbw, kbh;                   // k-blocks along w and h
   int32_t sw, sh;
   int32_t m_tiles, tiles_n, splits, kb_total, kb_per_split;
-  int32_t n_pairs, chunks, n_pad;
+  int32_t n_pairs, chunks, n_pad, cout;
   uint32_t idesc;
   float* partial;                     // [splits][m_tiles * 128][n_pad]
   unsigned int* status;
+  CwfSource x, g;
+  int32_t NI;
   int16_t tap_dw[kFMaxTaps], tap_dh[kFMaxTaps];
 };
+
+// As cwf_redo_fwd: the 32 rows of a warp are the channels of one tap and chunk, a lane forms its own elements.
+template <int BN>
+__device__ __noinline__ void cwf_redo_wgrad(const CwfWgParams& p, int q, int half) {
+  constexpr int COLS = BN / 2;
+  const int lane = threadIdx.x & 31, per_split = p.m_tiles * p.tiles_n;
+  for (int item = blockIdx.x; item < per_split * p.splits; item += gridDim.x) {
+    const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / per_split;
+    const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+    const int pr = mt * 4 + q;
+    if (pr >= p.n_pairs) continue;
+    const int tap = pr / p.chunks, c = (pr - tap * p.chunks) * 32 + lane;
+    float* const row = p.partial + ((int64_t)z * p.m_tiles * 128 + mt * 128 + q * 32 + lane) * p.n_pad;
+    for (int j = 0; j < COLS; ++j) {
+      const int col = nt * BN + half * COLS + j;
+      if (col >= p.cout) break;
+      const bool todo = row[col] != row[col];
+      if (!__any_sync(0xffffffffu, todo)) continue;
+      float sum = 0.f;
+      for (int kb = kb_lo; kb < kb_hi && __any_sync(0xffffffffu, todo && sum == sum); ++kb) {
+        const int a0 = (kb % p.kbw) * p.KW_, b0 = (kb / p.kbw) % p.kbh * p.KH_, i0 = kb / (p.kbw * p.kbh) * p.KI_;
+        for (int t = 0; t < 32; ++t) {
+          const int a = a0 + t % p.KW_, b = b0 + t / p.KW_ % p.KH_, img = i0 + t / (p.KW_ * p.KH_);
+          const int w = a * p.sw + p.tap_dw[tap], h = b * p.sh + p.tap_dh[tap];
+          if (a < p.g.W && b < p.g.H && img < p.NI && p.x.has(c, w, h)) sum = fmaf(p.x.at(c, w, h, img), p.g.at(col, a, b, img), sum);
+        }
+      }
+      if (todo) row[col] = sum;
+    }
+  }
+}
 
 template <int BN>
 __global__ void __launch_bounds__(kFThreads, 1)
@@ -557,7 +657,7 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;
     constexpr int COLS = BN / 2;
-    bool ok = true;
+    bool nan = false, ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
       const int mt = item % p.m_tiles, nt = (item / p.m_tiles) % p.tiles_n, z = item / per_split;
       const int kb_lo = z * p.kb_per_split, kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
@@ -575,10 +675,12 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
           float4 v = make_float4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
           if (kb > kb_lo) { const float4 o = dst[j]; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
           dst[j] = v;
+          nan |= v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
         }
         kb += kSegment;
       } while (kb < kb_hi);
     }
+    if (ok && __any_sync(0xffffffffu, nan)) cwf_redo_wgrad<BN>(p, q, half);
   }
 
   tc_fence_before();
@@ -689,7 +791,9 @@ CwfCopy cwf_copy_x(const ConvGeom& g) {
 }
 CwfCopy cwf_copy_y(const ConvGeom& g) { return cwf_copy(g.cout, g.out[0], g.out[1], g.batch); }
 
-CwfSource cwf_source(const void* ptr, const CwfCopy& c) { return CwfSource{static_cast<const uint16_t*>(ptr), c.part_stride(), c.Cp, c.W, c.H}; }
+CwfSource cwf_source(const void* ptr, const CwfCopy& c, const ConvGeom& g, int fold) {
+  return CwfSource{static_cast<const uint16_t*>(ptr), c.part_stride(), c.Cp, c.W, c.H, fold ? g.cin : 0, g.stride[0], g.dil[0], g.pad_lo[0], g.in[0]};
+}
 
 size_t cwf_packed_one(int rows, int taps, int chunks) {
   return align_up((size_t)((rows + cwf_bn(rows) - 1) / cwf_bn(rows) * cwf_bn(rows)) * taps * chunks * 32 * 2, 1024);
@@ -794,11 +898,12 @@ int32_t cwf_run(const CwfOut& o, const CwfSource& src, int NI, int chunks, const
   for (int i = 0; i < n_taps; ++i) {
     p.tap_dw[i] = (int16_t)taps[i].dw; p.tap_dh[i] = (int16_t)taps[i].dh; p.tap_index[i] = (int16_t)taps[i].index;
   }
+  p.src = src; p.wp = wp; p.wp_part_stride = (int64_t)(packed_one / 2); p.wp_cols = wp_cols;
   CUtensorMap mX[3], mW[3];
   bool encoded = true;
   for (int i = 0; i < 3; ++i)
     encoded = encoded && cwf_map(&mX[i], src.ptr + i * src.part_stride, src.Cp, src.W, src.H, NI, t.BW, t.BH, t.BI, sw, sh) &&
-              cwf_map_2d(&mW[i], wp + i * (packed_one / 2), wp_cols, wp_rows, bn);
+              cwf_map_2d(&mW[i], wp + i * p.wp_part_stride, wp_cols, wp_rows, bn);
   if (!encoded)
     return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cuTensorMapEncodeTiled failed");
   const int64_t items = t.tiles() * o.splits;
@@ -900,7 +1005,7 @@ int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const 
   const int64_t numel = (int64_t)g.out[0] * g.out[1] * g.cout * g.batch;
   const CwfOut o{(float*)y, (float*)preact, (const float*)bias, act, g.out[0], g.out[1], 1, 0, 1, 0,
                  reinterpret_cast<float*>(ws + xc.bytes() + 3 * packed), cwf_fwd_splits(g), numel};
-  rc = cwf_run(o, cwf_source(ws, xc), g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n_taps, g.out[0], g.out[1],
+  rc = cwf_run(o, cwf_source(ws, xc, g, fold), g.batch, pk.chunks, wp, packed, pk.n_rows, pk.k_total, taps, n_taps, g.out[0], g.out[1],
                fold ? 1 : g.stride[0], g.stride[1], g.cout, st);
   return rc != LB2_OK ? rc : cwf_finish(o, numel, g.cout, st);
 }
@@ -917,7 +1022,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
                      bool x_is_copy) {
   uint8_t* ws = static_cast<uint8_t*>(ws_);
   const CwfCopy yc = cwf_copy_y(g);
-  const CwfSource gcopy = cwf_source(ws, yc);
+  const CwfSource gcopy = cwf_source(ws, yc, g, 0);
   int32_t rc = cwf_transpose(ws, yc, (const float*)gy, g.out[0] * g.out[1], g.cout, g.batch, st);
   if (rc != LB2_OK) return rc;
   uint8_t* rest = ws + yc.bytes();
@@ -925,7 +1030,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
   if (dw != nullptr) {
     const int fold = cwf_fold(g), n_taps = cwf_taps(g);
     const CwfCopy xc = cwf_copy_x(g);
-    const CwfSource xcopy = cwf_source(x_is_copy ? x : rest, xc);
+    const CwfSource xcopy = cwf_source(x_is_copy ? x : rest, xc, g, fold);
     if (!x_is_copy) {
       rc = cwf_make_copy_x(rest, (const float*)x, g, xc, st);
       if (rc != LB2_OK) return rc;
@@ -936,7 +1041,8 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     q.KW_ = pl.KW_; q.KH_ = pl.KH_; q.KI_ = pl.KI_; q.kbw = pl.kbw; q.kbh = pl.kbh;
     q.sw = fold ? 1 : g.stride[0]; q.sh = g.stride[1];
     q.m_tiles = pl.m_tiles; q.tiles_n = pl.tiles_n; q.splits = pl.splits; q.kb_total = pl.kb_total; q.kb_per_split = pl.kb_per_split;
-    q.n_pairs = pl.n_pairs; q.chunks = pl.chunks; q.n_pad = pl.n_pad;
+    q.n_pairs = pl.n_pairs; q.chunks = pl.chunks; q.n_pad = pl.n_pad; q.cout = g.cout;
+    q.x = xcopy; q.g = gcopy; q.NI = g.batch;
     q.idesc = cwf_idesc(bn, true);
     q.partial = reinterpret_cast<float*>(rest + (x_is_copy ? 0 : xc.bytes()));
     q.status = device_status_word();

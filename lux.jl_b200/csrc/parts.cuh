@@ -17,13 +17,28 @@ struct Parts { uint16_t a, b, c; };
 __device__ __forceinline__ float part_f32(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
 __device__ __forceinline__ uint16_t part_rn(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
 
+// Not-a-number and infinity give what a sum of fp32 products gives. An infinity is (+-1, 0, +-Inf), NaN (1, 0, NaN): the third
+// part meets only the other operand's first, so that an infinite term is formed once, with its own sign (0 * Inf included);
+// where both are infinite the ones carry the sign.
 __device__ __forceinline__ Parts split_parts(float v) {
   Parts p;
+  const uint32_t u = __float_as_uint(v);
+  if ((u & 0x7F800000u) == 0x7F800000u) {
+    const bool nan = (u & 0x007FFFFFu) != 0;
+    p.a = nan ? 0x3F80u : (uint16_t)(((u >> 16) & 0x8000u) | 0x3F80u);
+    p.b = 0;
+    p.c = nan ? 0x7FC0u : (uint16_t)(u >> 16);
+    return p;
+  }
   p.a = part_rn(v);
+  if ((p.a & 0x7FFFu) == 0x7F80u) p.a = (uint16_t)(u >> 16);   // finite, but rounded up to infinity
   const float r = v - part_f32(p.a);
   p.b = part_rn(r);
   p.c = part_rn(r - part_f32(p.b));
   return p;
+}
+__device__ __forceinline__ float join_parts(const uint16_t* p, int64_t part_stride) {
+  return (part_f32(__ldg(p)) + part_f32(__ldg(p + part_stride))) + part_f32(__ldg(p + 2 * part_stride));
 }
 // four values: one 8-byte store per part; eight: one 16-byte store
 __device__ __forceinline__ void pack_parts4(const float* v, uint32_t (&w)[3][2]) {

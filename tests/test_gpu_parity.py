@@ -1272,3 +1272,68 @@ def test_f32_attention_is_as_close_to_64_bits_as_fp32_sums(dims, causal):
         parity_report.record(name, "f32", err, fp32_err)
         assert err <= fp32_err, (name, err, fp32_err)
         assert loss <= 2.0 ** -23, (name, loss)
+
+
+def _same_kind(got, want, what):
+    """The same elements NaN, +Inf and -Inf; the finite ones within the tolerance of the Float32 convolutions above."""
+    g, w = L.to_numpy(got).astype(np.float64), L.to_numpy(want).astype(np.float64)
+    for kind in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(kind(g), kind(w)), (what, kind.__name__, int(kind(g).sum()), int(kind(w).sum()))
+    fin = np.isfinite(w)
+    if fin.any():
+        assert np.linalg.norm(g[fin] - w[fin]) <= 3e-6 * np.linalg.norm(w[fin]), what
+
+
+@pytest.mark.parametrize("act", ["identity", "relu"])
+@pytest.mark.parametrize("planted", ["x", "w", "dy", "x and w", "largest"])
+@pytest.mark.parametrize("case", [
+    ((9, 7), (3, 3), 6, 5, 2, 1, 3),
+    ((14, 14), (3, 3), 40, 70, 1, 1, 2),           # two chunks, the second padded with zeros; positions past the ends of a box
+    ((7, 7), (3, 3), 512, 96, 1, 1, 1),            # split along the contraction
+    ((21, 17), (7, 7), 3, 24, 2, 3, 2),            # folded taps: zeros beside the image inside the copy
+    ((13, 11), (1, 1), 96, 40, 3, 0, 4),           # classes of the data gradient that no tap reaches
+])
+def test_f32_conv_passes_infinities_and_nan_on_as_fp32_sums_do(case, planted, act):
+    # corners, edges and an inner point, so that taps meet them that reach outside; the CUDA-core kernels are the reference
+    sp, k, cin, cout, stride, pad, batch = case
+    rng = np.random.default_rng(68)
+    x, w = rng.standard_normal(sp + (cin, batch)).astype(np.float32), O.kaiming_normal(rng, k + (cin, cout)).astype(np.float32)
+    out = tuple((n + 2 * pad - kk) // stride + 1 for n, kk in zip(sp, k))
+    b, dy = rng.standard_normal(cout).astype(np.float32), rng.standard_normal(out + (cout, batch)).astype(np.float32)
+    if "x" in planted.split():
+        x[0, 0, -1, 0], x[-1, -1, 0, -1] = -np.inf, np.inf
+        if planted == "x":
+            x[sp[0] // 2, 2, 1, 0] = np.nan
+    if "w" in planted.split():
+        w[0, 0, 0, 0], w[-1, -1, 1, 1] = np.inf, -np.inf
+        if planted == "w":
+            w[-1, 0, 2, 2] = np.nan
+    if planted == "dy":
+        dy[0, 0, 0, 0], dy[-1, -1, 1, -1], dy[-1, 0, 2, -1] = np.inf, -np.inf, np.nan
+    if planted == "largest":                       # rounds up to infinity in fewer bits
+        x[0, 0, -1, 0], x[-1, -1, 0, -1] = np.finfo(np.float32).max, -np.finfo(np.float32).max
+        w *= np.float32(1e-3)
+
+    def outputs(flags):
+        y, pb = L.rrule_fused_conv(act, dev(w, "f32"), dev(x, "f32"), dev(b, "f32"), L.ConvDims.make(2, stride, pad), flags=flags)
+        return (y,) + tuple(pb(dev(dy, "f32")))
+    for name, got, want in zip(("y", "dw", "dx", "db"), outputs(0), outputs(L._cabi.FLAG_FORCE_SIMT)):
+        _same_kind(got, want, name)
+    assert L._cabi.load().lb2_poll_device_status(None) == 0
+
+
+@pytest.mark.parametrize("planted", range(4))      # q, k, v, dx
+@pytest.mark.parametrize("dims", [(64, 2, 2, 40, 60, 2), (20, 2, 1, 130, 130, 1)])
+def test_f32_attention_passes_infinities_on_as_fp32_sums_do(dims, planted):
+    # no causal mask: the terms it zeroes are not formed at all outside the diagonal tiles, as the header states
+    D, H, Hkv, Lq, S, B = dims
+    rng = np.random.default_rng(69)
+    a = [rng.standard_normal(s).astype(np.float32) for s in ((D, H, Lq, B), (D, Hkv, S, B), (D, Hkv, S, B), (D, H, Lq, B))]
+    a[planted][1, 0, 3, 0] = np.inf
+    a[planted][:, 0, 5, 0] = -np.inf
+
+    def outputs(flags):
+        (x, w), pb = L.rrule_scaled_dot_product_attention(*(dev(t, "f32") for t in a[:3]), flags=flags)
+        return (x, w) + tuple(pb(dev(a[3], "f32"))[:3])
+    for name, got, want in zip(("x", "w", "dq", "dk", "dv"), outputs(0), outputs(L._cabi.FLAG_FORCE_SIMT)):
+        _same_kind(got, want, name)
