@@ -320,7 +320,7 @@ LB2_API int32_t lb2_attention_softmax_bwd(void* dlogits, void* dbias, const void
  * extents are served (positive, head_dim and value_dim rows a multiple of 16 bytes); arrays must be 16-byte aligned.
  * Backward: dbias (keys, queries, heads, batch) may be NULL. The terms that a causal mask zeroes are formed only inside the
  * 128 x 128 tiles on the diagonal: an infinity or NaN in a position that the mask hides may not reach the results, where the
- * reference's product over all keys (lib/LuxLib/src/impl/attention.jl:103-118) makes NaN of 0 * Inf. */
+ * reference's product over all keys (lib/LuxLib/src/impl/attention.jl:76-118) makes NaN of 0 * Inf. */
 typedef struct lb2_attention_dims {
   int64_t head_dim, value_dim, heads, kv_heads, queries, keys, batch;
 } lb2_attention_dims;
