@@ -41,14 +41,14 @@ int32_t conv_cw_fwd(void* y, void* preact, const void* x, const void* w, const v
 int32_t conv_cw_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws,
                     cudaStream_t st, bool x_is_copy = false);
 
-// General Float32 tensor-core path on channel-innermost hi/lo copies (conv_cw_f32.cu), same geometries.
+// General Float32 tensor-core path on channel-innermost copies in three bf16 parts (conv_cw_f32.cu), same geometries.
 bool conv_cwf_supported(const ConvGeom& g);
 size_t conv_cwf_fwd_workspace_bytes(const ConvGeom& g);
 size_t conv_cwf_bwd_workspace_bytes(const ConvGeom& g);
 int32_t conv_cwf_fwd(void* y, void* preact, const void* x, const void* w, const void* bias, const ConvGeom& g, int32_t act,
                      void* ws, cudaStream_t st);
 int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws,
-                     cudaStream_t st, bool x_is_copy = false);
+                     cudaStream_t st);
 
 // Box of at most `most` positions (BW columns x BH rows x BI images) for an OW x OH x NI grid, rows cut into equal pieces of at
 // least 8 columns: the one whose boxes, `per_box` tiles each, take the fewest waves of `wave` tiles (wave = 1: the fewest

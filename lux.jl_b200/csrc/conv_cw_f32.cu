@@ -1017,9 +1017,8 @@ size_t conv_cwf_bwd_workspace_bytes(const ConvGeom& g) {
   return cwf_copy_y(g).bytes() + (dgrad > wgrad ? dgrad : wgrad);
 }
 
-// both gradients (either output may be null) from one copy of gy; with `x_is_copy`, x points at the copy that conv_cwf_fwd left
-int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws_, cudaStream_t st,
-                     bool x_is_copy) {
+// both gradients (either output may be null) from one copy of gy
+int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const void* w, const ConvGeom& g, void* ws_, cudaStream_t st) {
   uint8_t* ws = static_cast<uint8_t*>(ws_);
   const CwfCopy yc = cwf_copy_y(g);
   const CwfSource gcopy = cwf_source(ws, yc, g, 0);
@@ -1030,11 +1029,9 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
   if (dw != nullptr) {
     const int fold = cwf_fold(g), n_taps = cwf_taps(g);
     const CwfCopy xc = cwf_copy_x(g);
-    const CwfSource xcopy = cwf_source(x_is_copy ? x : rest, xc, g, fold);
-    if (!x_is_copy) {
-      rc = cwf_make_copy_x(rest, (const float*)x, g, xc, st);
-      if (rc != LB2_OK) return rc;
-    }
+    const CwfSource xcopy = cwf_source(rest, xc, g, fold);
+    rc = cwf_make_copy_x(rest, (const float*)x, g, xc, st);
+    if (rc != LB2_OK) return rc;
     const CwfWgPlan pl = cwf_wg_plan(g);
     const int bn = cwf_bn(g.cout);
     CwfWgParams q{};
@@ -1044,7 +1041,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     q.n_pairs = pl.n_pairs; q.chunks = pl.chunks; q.n_pad = pl.n_pad; q.cout = g.cout;
     q.x = xcopy; q.g = gcopy; q.NI = g.batch;
     q.idesc = cwf_idesc(bn, true);
-    q.partial = reinterpret_cast<float*>(rest + (x_is_copy ? 0 : xc.bytes()));
+    q.partial = reinterpret_cast<float*>(rest + xc.bytes());
     q.status = device_status_word();
     LB2_REQUIRE(q.status != nullptr, LB2_LAUNCH_FAIL, "conv_cw_f32: device status word unavailable");
     for (int t = 0; t < n_taps; ++t) {

@@ -1337,3 +1337,22 @@ def test_f32_attention_passes_infinities_on_as_fp32_sums_do(dims, planted):
         return (x, w) + tuple(pb(dev(a[3], "f32"))[:3])
     for name, got, want in zip(("x", "w", "dq", "dk", "dv"), outputs(0), outputs(L._cabi.FLAG_FORCE_SIMT)):
         _same_kind(got, want, name)
+
+
+def test_f32_conv_keeps_x_alone_for_its_pullback():
+    # a Float32 call keeps no copy of x and no scratch from the forward call to the pullback: it says so and refuses one
+    import ctypes as C
+    from luxlib_b200 import ops as _ops
+    x, w = torch.randn(8, 32, 40, 41, device="cuda").permute(3, 2, 1, 0), torch.randn(48, 32, 3, 3, device="cuda").permute(3, 2, 1, 0)
+    cd, lib = L.ConvDims.make(2, 2, 1), L._cabi.load()
+    d = _ops._conv_desc(w, x, cd)
+    assert lib.lb2_conv_fwd_workspace_bytes(C.byref(d), 0) > 4 * x.numel()
+    assert lib.lb2_conv_fwd_leaves_x_copy(C.byref(d), 0) == 0
+    L.rrule_fused_conv("identity", w, x, None, cd)
+    before = torch.cuda.memory_allocated()
+    y, pullback = L.rrule_fused_conv("identity", w, x, None, cd)
+    assert torch.cuda.memory_allocated() - before <= 4 * y.numel() + 512          # the allocator's granularity
+    ws = torch.empty(lib.lb2_conv_bwd_workspace_bytes(C.byref(d), 0, 0), dtype=torch.uint8, device="cuda")
+    dw = torch.empty_like(w)
+    assert lib.lb2_conv_bwd(dw.data_ptr(), None, None, y.data_ptr(), None, None, ws.data_ptr(), w.data_ptr(), C.byref(d), 0, 0,
+                            L._cabi.FLAG_X_COPY_GIVEN, ws.data_ptr(), ws.numel(), None) == -1                # LB2_BAD_ARG
