@@ -170,7 +170,11 @@ typedef struct {
 /* Fills out[0..ndim) with (in + pad_lo + pad_hi - dil*(k-1) - 1) / stride + 1 (src/layers/conv.jl:175-177). */
 LB2_API int32_t lb2_conv_output_size(const lb2_conv_desc* d, int32_t* out);
 /* y = act.(conv(x, w) .+ b); optional pre-activation store. Replaces conv_bias_act / conv!
- * for CUDADevice (lib/LuxLib/src/impl/conv.jl:42-60,157-166). */
+ * for CUDADevice (lib/LuxLib/src/impl/conv.jl:42-60,157-166).
+ * Float32 geometries that only the general tensor-core path takes (any stride, odd planes) are still served without its
+ * workspace, by the CUDA-core kernels: lb2_conv_fwd with less than this size (none at all, or one that is not 256-byte
+ * aligned), lb2_conv_fwd_sums with room for lb2_channel_sums alone, lb2_conv_bwd with room for its activation pass
+ * (dy's size where act is not the identity, rounded up to 1024, and lb2_bias_act_bwd_workspace_bytes, likewise). */
 LB2_API size_t lb2_conv_fwd_workspace_bytes(const lb2_conv_desc* d, int32_t dtype);
 LB2_API int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const void* b,
                      const lb2_conv_desc* d, int32_t dtype, int32_t act, uint32_t flags,

@@ -109,7 +109,7 @@ int32_t lb2_conv_fwd(void* y, void* preact, const void* x, const void* w, const 
   if (route != 0) {
     const size_t need = route_fwd_bytes(route, g, dtype);
     // without room for the Float32 copies the CUDA-core kernels, which need none, still serve the call
-    if (route == 3 && (workspace == nullptr || workspace_bytes < need))
+    if (route == 3 && (workspace == nullptr || workspace_bytes < need || !aligned_to(workspace, 256)))
       return conv_fwd_direct(y, preact, x, w, b, g, dtype, act, static_cast<cudaStream_t>(stream));
     LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", need);
     LB2_REQUIRE(aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");
@@ -157,8 +157,12 @@ int32_t lb2_conv_fwd_sums(void* y, float* sums, const void* x, const void* w, co
     cudaMemsetAsync(sums, 0, (size_t)g.cout * 2 * sizeof(float), st);
     return LB2_OK;
   }
-  LB2_REQUIRE(workspace_bytes >= lb2_conv_fwd_sums_workspace_bytes(d, dtype), LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed",
-              lb2_conv_fwd_sums_workspace_bytes(d, dtype));
+  size_t conv = align_up(lb2_conv_fwd_workspace_bytes(d, dtype), 1024), need = lb2_conv_fwd_sums_workspace_bytes(d, dtype);
+  if (conv_route(g, dtype) == 3 && ((flags & LB2_FLAG_FORCE_SIMT) || workspace_bytes < need)) {   // as in lb2_conv_fwd
+    need -= conv;
+    conv = 0;
+  }
+  LB2_REQUIRE(workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", need);
   const bool fused = !(flags & LB2_FLAG_FORCE_SIMT) && conv_route(g, dtype) == 2;
   if (fused) {
     LB2_REQUIRE(y && x && w, LB2_BAD_ARG, "null tensor pointer");
@@ -166,7 +170,6 @@ int32_t lb2_conv_fwd_sums(void* y, float* sums, const void* x, const void* w, co
     LB2_REQUIRE(aligned_to(y, 2) && aligned_to(x, 2) && aligned_to(w, 2), LB2_BAD_ALIGN, "pointer not aligned to the element size");
     return conv_cw_fwd(y, nullptr, x, w, nullptr, g, LB2_ACT_IDENTITY, workspace, st, sums);
   }
-  const size_t conv = align_up(lb2_conv_fwd_workspace_bytes(d, dtype), 1024);
   rc = lb2_conv_fwd(y, nullptr, x, w, nullptr, d, dtype, LB2_ACT_IDENTITY, flags, workspace, conv, stream);
   if (rc != LB2_OK) return rc;
   uint8_t* rest = static_cast<uint8_t*>(workspace) + conv;
@@ -206,11 +209,11 @@ int32_t lb2_conv_bwd(void* dw, void* dx, void* db, const void* dy, const void* o
   const ConvBwdLayout lay = conv_bwd_layout(g, dtype, act);
   int route = (flags & LB2_FLAG_FORCE_SIMT) ? 0 : (lay.tc_bytes > 0 ? conv_route(g, dtype) : 0);
   size_t need = lay.total();
-  if (route == 3 && workspace_bytes < need) {   // as in the forward call
+  if (conv_route(g, dtype) == 3 && (route == 0 || workspace_bytes < need)) {   // as in the forward call
     route = 0;
     need = lay.g_bytes + lay.red_bytes;
   }
-  LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", lay.total());
+  LB2_REQUIRE(workspace != nullptr && workspace_bytes >= need, LB2_WORKSPACE_TOO_SMALL, "workspace of %zu bytes needed", need);
   LB2_REQUIRE(aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   float* red = reinterpret_cast<float*>(ws + lay.g_bytes);

@@ -1356,3 +1356,44 @@ def test_f32_conv_keeps_x_alone_for_its_pullback():
     dw = torch.empty_like(w)
     assert lib.lb2_conv_bwd(dw.data_ptr(), None, None, y.data_ptr(), None, None, ws.data_ptr(), w.data_ptr(), C.byref(d), 0, 0,
                             L._cabi.FLAG_X_COPY_GIVEN, ws.data_ptr(), ws.numel(), None) == -1                # LB2_BAD_ARG
+
+
+@pytest.mark.parametrize("act", [0, 1])
+def test_f32_conv_scratch_the_cuda_core_kernels_need_is_enough(act):
+    # what these calls took before the general tensor-core path: forced onto the CUDA cores, sums, a base off 256 bytes
+    import ctypes as C
+    from luxlib_b200 import ops as _ops
+    rng = np.random.default_rng(70)
+    x, w = rng.standard_normal((9, 7, 6, 3)).astype(np.float32), rng.standard_normal((3, 3, 6, 5)).astype(np.float32)
+    name = ("identity", "relu")[act]
+    y_ref, pb_ref = O.fused_conv_rrule(name, w.astype(np.float64), x.astype(np.float64), None, O.ConvDims.make(2, 2, 1, 1, 1, False))
+    lib, simt = L._cabi.load(), L._cabi.FLAG_FORCE_SIMT
+    X, W = dev(x, "f32"), dev(w, "f32")
+    d = _ops._conv_desc(W, X, L.ConvDims.make(2, 2, 1))
+    S, Cc, B = int(np.prod(y_ref.shape[:2])), y_ref.shape[2], y_ref.shape[3]
+    up = lambda n: (n + 1023) // 1024 * 1024
+    y = L.jl_empty(y_ref.shape, X.dtype, X.device)
+    ws = torch.empty(lib.lb2_conv_fwd_workspace_bytes(C.byref(d), 0) + 512, dtype=torch.uint8, device="cuda")
+    assert lib.lb2_conv_fwd(y.data_ptr(), None, X.data_ptr(), W.data_ptr(), None, C.byref(d), 0, act, 0, ws.data_ptr() + 8, ws.numel() - 8, None) == 0
+    check(y, y_ref, "f32", "y")
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    dw_ref, dx_ref, _ = pb_ref(delta.astype(np.float64))
+    G, dw, dx = dev(delta, "f32"), L.jl_empty(w.shape, X.dtype, X.device), L.jl_empty(x.shape, X.dtype, X.device)
+    n = (up(4 * y.numel()) if act else 0) + up(lib.lb2_bias_act_bwd_workspace_bytes(S, Cc, B))
+    args = lambda flags, n: (dw.data_ptr(), dx.data_ptr(), None, G.data_ptr(), y.data_ptr(), None, X.data_ptr(), W.data_ptr(), C.byref(d), 0, act,
+                             flags, small.data_ptr(), n, None)
+    small = torch.empty(n, dtype=torch.uint8, device="cuda")
+    for flags in (simt, 0):
+        dw.zero_(), dx.zero_()
+        assert lib.lb2_conv_bwd(*args(flags, n)) == 0
+        check(dw, dw_ref, "f32", "dw")
+        check(dx, dx_ref, "f32", "dx")
+        assert lib.lb2_conv_bwd(*args(flags, n - 1)) == -7                       # LB2_WORKSPACE_TOO_SMALL
+    if act == 0:
+        sums = torch.empty(2 * Cc, device="cuda")
+        n = lib.lb2_channel_sums_workspace_bytes(S, Cc, B)
+        small = torch.empty(max(n, 1), dtype=torch.uint8, device="cuda")
+        for flags in (simt, 0):
+            assert lib.lb2_conv_fwd_sums(y.data_ptr(), sums.data_ptr(), X.data_ptr(), W.data_ptr(), C.byref(d), 0, flags, small.data_ptr(), n,
+                                         None) == 0
+            check(sums, np.stack([y_ref.sum((0, 1, 3)), (y_ref ** 2).sum((0, 1, 3))], 1).ravel(), "f32", "sums")
