@@ -135,7 +135,9 @@ LB2_API int32_t lb2_dense_fwd(void* y, void* preact, const void* W, const void* 
  * Any of dW, dx, db may be NULL (not computed). accumulate != 0 adds into dW, dx, db instead of
  * overwriting them — the Enzyme shadow contract (lib/LuxLib/src/impl/dense.jl:253-283:
  *   mul!(dW, g, x', true, true); mul!(dx, W', g, true, true); db .+= sum(g)). The last step of that rule,
- * zeroing the output shadow dy (impl/dense.jl:281), is left to the caller: dy is read-only here. */
+ * zeroing the output shadow dy (impl/dense.jl:281), is left to the caller: dy is read-only here.
+ * bf16: the part of the workspace behind the activation pass is for packed copies of odd widths; without room for them the
+ * CUDA-core kernels take the products (lb2_dense_fwd, lb2_matmul: likewise). */
 LB2_API size_t lb2_dense_bwd_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t dtype, int32_t act,
                                      uint32_t flags);
 LB2_API int32_t lb2_dense_bwd(void* dW, void* dx, void* db, const void* dy, const void* out,

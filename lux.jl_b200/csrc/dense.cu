@@ -97,7 +97,9 @@ int32_t lb2_dense_bwd(void* dW, void* dx, void* db, const void* dy, const void* 
   LB2_REQUIRE(aligned_to(dW, es) && aligned_to(dx, es) && aligned_to(db, es) && aligned_to(dy, es) && aligned_to(out, es) &&
                   aligned_to(preact, es) && aligned_to(W, es) && aligned_to(x, es),
               LB2_BAD_ALIGN, "pointer not aligned to the element size");
-  const BwdLayout lay = bwd_layout(M, N, K, dtype, act, flags);
+  BwdLayout lay = bwd_layout(M, N, K, dtype, act, flags);
+  // bf16: without room for the packed copies of odd widths the CUDA-core kernels, which need none, still serve the call
+  if (dtype == LB2_BF16 && workspace_bytes < lay.total()) lay.gemm_bytes = 0;
   LB2_REQUIRE(lay.total() == 0 || (workspace != nullptr && workspace_bytes >= lay.total()), LB2_WORKSPACE_TOO_SMALL,
               "workspace of %zu bytes needed", lay.total());
   LB2_REQUIRE(workspace == nullptr || aligned_to(workspace, 256), LB2_BAD_ALIGN, "workspace must be 256-byte aligned");

@@ -1397,3 +1397,24 @@ def test_f32_conv_scratch_the_cuda_core_kernels_need_is_enough(act):
             assert lib.lb2_conv_fwd_sums(y.data_ptr(), sums.data_ptr(), X.data_ptr(), W.data_ptr(), C.byref(d), 0, flags, small.data_ptr(), n,
                                          None) == 0
             check(sums, np.stack([y_ref.sum((0, 1, 3)), (y_ref ** 2).sum((0, 1, 3))], 1).ravel(), "f32", "sums")
+
+
+@pytest.mark.parametrize("act", [0, 1])
+def test_dense_pullback_of_odd_widths_without_room_for_packed_copies(act):
+    # bf16 widths that TMA cannot read are packed into scratch that the CUDA-core kernels did not need: without it they serve the call
+    M, N, K = 67, 129, 45
+    rng = np.random.default_rng(71)
+    W, x, b, d = (prep(a, "bf16") for a in (O.glorot_uniform(rng, (M, K)), rng.standard_normal((K, N)), rng.uniform(-1, 1, M), rng.standard_normal((M, N))))
+    y_ref, pb_ref = O.fused_dense_rrule(("identity", "relu")[act], *(a.astype(np.float64) for a in (W, x, b)))
+    lib = L._cabi.load()
+    Wd, xd, dd, y = dev(W, "bf16"), dev(x, "bf16"), dev(d, "bf16"), dev(y_ref, "bf16")
+    dW, dx, db = L.jl_empty((M, K), Wd.dtype, "cuda"), L.jl_empty((K, N), Wd.dtype, "cuda"), torch.empty(M, dtype=Wd.dtype, device="cuda")
+    n = ((2 * M * N + 255) // 256 * 256 if act else 0) + lib.lb2_bias_act_bwd_workspace_bytes(1, M, N)
+    assert lib.lb2_dense_bwd_workspace_bytes(M, N, K, 1, act, 0) > n
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    call = lambda n: lib.lb2_dense_bwd(dW.data_ptr(), dx.data_ptr(), db.data_ptr(), dd.data_ptr(), y.data_ptr(), None, Wd.data_ptr(), xd.data_ptr(),
+                                       M, N, K, M, K, M, 1, act, 0, 0, ws.data_ptr(), n, None)
+    assert call(n) == 0
+    for name, got, want in zip(("dW", "dx", "db"), (dW, dx, db), pb_ref(d.astype(np.float64))):
+        check(got, want, "bf16", name)
+    assert call(n - 1) == -7                       # LB2_WORKSPACE_TOO_SMALL
