@@ -93,6 +93,24 @@ def _ws(nbytes: int, device):
     return w, ptr(w), int(nbytes) if w is not None else 0
 
 
+def _with_scratch(nbytes: int, least: int, device, call):
+    """`call(pointer, bytes)` with `nbytes` of scratch, which is returned. Where the device has no room for that, with `least`:
+    what the CUDA-core kernels need, which then serve the call if the library lets them."""
+    try:
+        w, wsp, wsn = _ws(nbytes, device)
+    except torch.OutOfMemoryError:
+        if least >= nbytes:
+            raise
+        w, wsp, wsn = _ws(least, device)
+        status = call(wsp, wsn)
+        if status == _cabi.WORKSPACE_TOO_SMALL:
+            raise
+        _cabi.check(status)
+        return w
+    _cabi.check(call(wsp, wsn))
+    return w
+
+
 @functools.lru_cache(maxsize=4096)
 def _query(name: str, device_index, *args):
     """A pure query of the library (workspace sizes and the like): it depends on the extents and on the device's kind only,
@@ -445,6 +463,13 @@ class _ConvQuery:
         self.sums_fused = lib.lb2_conv_fwd_sums_is_fused(ref, dt) == 1
         self.bwd_bytes = functools.lru_cache(maxsize=8)(lambda code: lib.lb2_conv_bwd_workspace_bytes(ref, dt, code))
 
+    def least_bwd_bytes(self, code: int) -> int:
+        """Scratch of lb2_conv_bwd's activation pass alone."""
+        up = lambda n: (n + 1023) // 1024 * 1024
+        n = math.prod(self.yshape)
+        red = _cabi.load().lb2_bias_act_bwd_workspace_bytes(math.prod(self.yshape[:-2]), self.yshape[-2], self.yshape[-1])
+        return (0 if code == _cabi.ACT_IDENTITY else up(n * (4 if self.dt == 0 else 2))) + up(red)
+
 
 @functools.lru_cache(maxsize=1024)
 def _conv_query_of(device_index, dt, wshape, spatial, cin, batch, stride, padding, dilation, groups, flipkernel):
@@ -474,9 +499,8 @@ def _conv_fwd(act, weight, x, b, cd, want_preact, flags=0, want_ws=False):
     info = _conv_query(Wt, X, cd, dt)
     y = jl_empty(info.yshape, X.dtype, X.device)
     pre = jl_empty(info.yshape, X.dtype, X.device) if want_preact else None
-    ws, wsp, wsn = _ws(info.fwd_bytes, X.device)
-    _cabi.check(lib.lb2_conv_fwd(ptr(y), ptr(pre), ptr(X), ptr(Wt), ptr(b), C.byref(d), dt, act_code(act), flags, wsp, wsn,
-                                 current_stream(X.device)))
+    ws = _with_scratch(info.fwd_bytes, 0, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
+        ptr(y), ptr(pre), ptr(X), ptr(Wt), ptr(b), C.byref(d), dt, act_code(act), flags, wsp, wsn, current_stream(X.device)))
     # the general tensor-core path leaves its channel-innermost copy of x at the start of the workspace; a pullback
     # that keeps the workspace alive hands it back instead of having the copy made again
     keep = ws if (want_ws and ws is not None and not (flags & _cabi.FLAG_FORCE_SIMT) and X.data_ptr() % 16 == 0 and
@@ -503,10 +527,10 @@ def rrule_fused_conv(act: str, weight, x, b, cdims: ConvDims, *, flags: int = 0)
         dw = jl_empty(Wt.shape, X.dtype, X.device)
         dx = jl_empty(X.shape, X.dtype, X.device) if need_dx else None
         db = jl_empty((d.cout,), X.dtype, X.device) if bb is not None else None
-        _, wsp, wsn = _ws(info.bwd_bytes(code), X.device)
         xarg, xflag = (ptr(xcopy), _cabi.FLAG_X_COPY_GIVEN) if xcopy is not None else (ptr(X), 0)
-        _cabi.check(lib.lb2_conv_bwd(ptr(dw), ptr(dx), ptr(db), ptr(dl), None if keep_pre else ptr(y), ptr(pre), xarg,
-                                     ptr(Wt), C.byref(d), dt, code, flags | xflag, wsp, wsn, current_stream(X.device)))
+        _with_scratch(info.bwd_bytes(code), info.least_bwd_bytes(code), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+            ptr(dw), ptr(dx), ptr(db), ptr(dl), None if keep_pre else ptr(y), ptr(pre), xarg, ptr(Wt), C.byref(d), dt, code, flags | xflag,
+            wsp, wsn, current_stream(X.device)))
         return dw, dx, db
 
     return y, pullback
@@ -538,29 +562,26 @@ def rrule_conv_transpose(act: str, weight, x, b, cdims: ConvDims, outpad=0, *, f
     cu = Wt.shape[-2] * cdims.groups
     usz = conv_transpose_output_size(tuple(X.shape[:nd]), tuple(Wt.shape[:nd]), cdims, outpad)
     d = _conv_desc_from(tuple(Wt.shape), usz, cu, X.shape[-1], cdims)
-    osz = (C.c_int32 * 3)()
-    _cabi.check(lib.lb2_conv_output_size(C.byref(d), osz))
-    if tuple(osz[i] for i in range(nd)) != tuple(X.shape[:nd]):
+    dt = dtype_code(X.dtype)
+    info = _ConvQuery(d, dt)
+    if info.yshape[:nd] != tuple(X.shape[:nd]):
         raise DimensionMismatch("outpad does not fit the stride: the convolution of the result does not reproduce size(x)")
     if b is not None and b.shape[0] != cu:
         raise DimensionMismatch("length(bias) must equal the number of output channels")
-    dt = dtype_code(X.dtype)
     ident = act_code("identity")
     u = jl_empty(usz + (cu, X.shape[-1]), X.dtype, X.device)
-    _, wsp, wsn = _ws(lib.lb2_conv_bwd_workspace_bytes(C.byref(d), dt, ident), X.device)
-    _cabi.check(lib.lb2_conv_bwd(None, ptr(u), None, ptr(X), None, None, None, ptr(Wt), C.byref(d), dt, ident, flags, wsp, wsn,
-                                 current_stream(X.device)))
+    _with_scratch(info.bwd_bytes(ident), info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+        None, ptr(u), None, ptr(X), None, None, None, ptr(Wt), C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
     y, pb_act = rrule_bias_activation(act, u, b)
 
     def pullback(delta):
         g, db = pb_act(delta)
         dx = jl_empty(X.shape, X.dtype, X.device)
-        _, w1, n1 = _ws(lib.lb2_conv_fwd_workspace_bytes(C.byref(d), dt), X.device)
-        _cabi.check(lib.lb2_conv_fwd(ptr(dx), None, ptr(g), ptr(Wt), None, C.byref(d), dt, ident, flags, w1, n1, current_stream(X.device)))
+        _with_scratch(info.fwd_bytes, 0, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
+            ptr(dx), None, ptr(g), ptr(Wt), None, C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
         dw = jl_empty(Wt.shape, X.dtype, X.device)
-        _, w2, n2 = _ws(lib.lb2_conv_bwd_workspace_bytes(C.byref(d), dt, ident), X.device)
-        _cabi.check(lib.lb2_conv_bwd(ptr(dw), None, None, ptr(X), None, None, ptr(g), None, C.byref(d), dt, ident, flags, w2, n2,
-                                     current_stream(X.device)))
+        _with_scratch(info.bwd_bytes(ident), info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+            ptr(dw), None, None, ptr(X), None, None, ptr(g), None, C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
         return dw, dx, db
 
     return y, pullback
@@ -648,6 +669,15 @@ def rrule_batched_matmul(x, y, *, flags: int = 0):
         return dx, dy
 
     return z, pullback
+
+
+def _attention_scratch(nbytes: int, device):
+    """The tensor-core path's scratch (Float32: up to four copies of the weights), or None where the device has no room for it:
+    the products one by one, which need one, then take the call."""
+    try:
+        return workspace(nbytes, device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _attention_fwd_by_product(lib, out, w, Q, Kx, V, bias_c, bias_bs, mask_c, mask_bs, causal, sc, dims, dt, flags):
@@ -744,10 +774,10 @@ def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_cau
             mask_bs = S * Lq
         else:
             raise DimensionMismatch("mask must have the shape (S, L) or (S, L, H, B...)")
-    if fused:
-        _, wsp, wsn = _ws(lib.lb2_attention_fwd_workspace_bytes(C.byref(dims), dt), device)
+    scratch = _attention_scratch(lib.lb2_attention_fwd_workspace_bytes(C.byref(dims), dt), device) if fused else None
+    if scratch is not None:
         _cabi.check(lib.lb2_attention_fwd(ptr(out), ptr(w), ptr(Q), ptr(Kx), ptr(V), ptr(bias_c), bias_bs, ptr(mask_c), mask_bs, causal, sc,
-                                          C.byref(dims), dt, wsp, wsn, current_stream(device)))
+                                          C.byref(dims), dt, ptr(scratch), scratch.numel(), current_stream(device)))
     else:
         _attention_fwd_by_product(lib, out, w, Q, Kx, V, bias_c, bias_bs, mask_c, mask_bs, causal, sc, dims, dt, flags)
 
@@ -755,10 +785,12 @@ def rrule_scaled_dot_product_attention(q, k, v, *, scale=None, mask=None, is_cau
         G = as_colmajor(dx.to(Q.dtype))
         dq, dk, dv = (jl_empty(tuple(t.shape), Q.dtype, device) for t in (Q, Kx, V))
         db = jl_empty(tuple(w.shape), Q.dtype, device) if bias_c is not None else None
+        scratch = None
         if fused and G.data_ptr() % 16 == 0:
-            _, wsp, wsn = _ws(lib.lb2_attention_bwd_workspace_bytes(C.byref(dims), dt), device)
+            scratch = _attention_scratch(lib.lb2_attention_bwd_workspace_bytes(C.byref(dims), dt), device)
+        if scratch is not None:
             _cabi.check(lib.lb2_attention_bwd(ptr(dq), ptr(dk), ptr(dv), ptr(db), ptr(G), ptr(w), ptr(Q), ptr(Kx), ptr(V), causal, sc,
-                                              C.byref(dims), dt, wsp, wsn, current_stream(device)))
+                                              C.byref(dims), dt, ptr(scratch), scratch.numel(), current_stream(device)))
         else:
             _attention_bwd_by_product(lib, dq, dk, dv, db, G, w, Q, Kx, V, sc, dims, dt, flags)
         if db is not None and bias_bs == 0:

@@ -1418,3 +1418,38 @@ def test_dense_pullback_of_odd_widths_without_room_for_packed_copies(act):
     for name, got, want in zip(("dW", "dx", "db"), (dW, dx, db), pb_ref(d.astype(np.float64))):
         check(got, want, "bf16", name)
     assert call(n - 1) == -7                       # LB2_WORKSPACE_TOO_SMALL
+
+
+def test_float32_calls_run_where_the_device_has_no_room_for_tensor_core_copies(monkeypatch):
+    # what ran before those paths needed next to no scratch; an allocator that refuses more than 64 KB stands for a full device
+    from luxlib_b200 import ops as _ops
+    real = _ops.workspace
+
+    def small_only(nbytes, device):
+        if nbytes > 65536:
+            raise torch.OutOfMemoryError("no room")
+        return real(nbytes, device)
+    rng = np.random.default_rng(72)
+    x, w = rng.standard_normal((21, 17, 24, 5)).astype(np.float32), O.kaiming_normal(rng, (3, 3, 24, 20)).astype(np.float32)
+    cd, ocd = L.ConvDims.make(2, 2, 1), O.ConvDims.make(2, 2, 1, 1, 1, False)
+    y_ref, pb_ref = O.fused_conv_rrule("tanh", w.astype(np.float64), x.astype(np.float64), None, ocd)
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    q, k, v, dx = (rng.standard_normal((32, 2, n, 2)).astype(np.float32) for n in (150, 140, 140, 150))
+    (a_ref, w_ref), apb_ref = O.attention_rrule(*(t.astype(np.float64) for t in (q, k, v)))
+    ut = rng.standard_normal((11, 9, 20, 5)).astype(np.float32)
+    plain = L.rrule_conv_transpose("identity", dev(w, "f32"), dev(ut, "f32"), None, cd)
+    plain = (plain[0],) + tuple(plain[1](plain[0])[:2])
+    monkeypatch.setattr(_ops, "workspace", small_only)
+    y, pb = L.rrule_fused_conv("tanh", dev(w, "f32"), dev(x, "f32"), None, cd)
+    check(y, y_ref, "f32", "y")
+    for name, got, want in zip(("dw", "dx"), pb(dev(delta, "f32")), pb_ref(delta.astype(np.float64))):
+        check(got, want, "f32", name)
+    u, pbt = L.rrule_conv_transpose("identity", dev(w, "f32"), dev(ut, "f32"), None, cd)
+    for name, got, want in zip(("u", "dw", "dx"), (u,) + tuple(pbt(u)[:2]), plain):
+        check(got, L.to_numpy(want), "f32", "transpose " + name)
+    (a, aw), apb = L.rrule_scaled_dot_product_attention(dev(q, "f32"), dev(k, "f32"), dev(v, "f32"))
+    check(a, a_ref, "f32", "attention")
+    for name, got, want in zip(("dq", "dk", "dv"), apb(dev(dx, "f32")), apb_ref(dx.astype(np.float64))):
+        check(got, want, "f32", name)
+    with pytest.raises(torch.OutOfMemoryError):          # kernels that always needed their scratch say so, as before
+        L.fused_conv_bias_activation("identity", dev(w, "bf16"), dev(x, "bf16"), None, cd)
