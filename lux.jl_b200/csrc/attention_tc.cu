@@ -185,6 +185,7 @@ attn_gemm_kernel(const __grid_constant__ AtMaps tmA, const __grid_constant__ AtM
     uint32_t acc = 0, acc_phase = 0;
     bool ok = true;
     for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      __syncwarp();                        // rows past the last left the stores below early; the TMEM loads want whole warps
       Item t;
       if (!decode(item, &t)) continue;
       const int n_kb = (t.kb_hi - t.kb_lo) * p.rep;

@@ -365,6 +365,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   }
+  __syncwarp();                           // rows past the last took no part above; the barrier wants whole warps
   tc_fence_before();
   if (p.splits > 1) cluster_sync_all();   // nobody leaves while its partial may still be read
   else __syncthreads();
