@@ -883,6 +883,7 @@ int32_t cw_launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, CwFwdParams&
   const int fixed = resident ? p.num_kb * B_BYTES : 0, stage_bytes = resident ? A_BYTES : A_BYTES + B_BYTES;
   p.stages = (200 * 1024 - fixed) / stage_bytes > 8 ? 8 : (200 * 1024 - fixed) / stage_bytes;
   const int smem = fixed + p.stages * stage_bytes + 1024 + 256;
+  constexpr int most = 200 * 1024 + 1024 + 256;   // the limit is the kernel's, whoever launches it: the same for every filter and thread
   const int tiles = p.tiles_w * p.tiles_h * p.tiles_i * p.tiles_n;
   int grid = tiles < sm_count() ? tiles : sm_count();
   if (p.sums_partial != nullptr) {
@@ -892,8 +893,8 @@ int32_t cw_launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, CwFwdParams&
   }
   if (grid_out != nullptr) *grid_out = grid;
   auto launch = [&](auto kernel) -> int32_t {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
     kernel<<<grid, kCwThreads, smem, st>>>(mX, mW, p);
     LB2_CHECK_LAUNCH("conv_cw_fwd");
     return LB2_OK;

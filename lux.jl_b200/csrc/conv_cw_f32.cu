@@ -1074,9 +1074,9 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
       LB2_CHECK_LAUNCH("conv_cw_f32 filter-gradient split sum");
     }
     const CwfReduce rd{g.k[0], g.k[1], g.cin, g.cout, g.flip, fold, pl.chunks, pl.n_pad};
-    const int smem = 4 * g.k[0] * g.k[1] * 33 * 4;
-    cudaError_t e = cudaFuncSetAttribute(cwf_wgrad_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    const int smem = 4 * g.k[0] * g.k[1] * 33 * 4, most = 4 * kFMaxTaps * 33 * 4;   // the limit is the kernel's: the same for every thread
+    cudaError_t e = cudaFuncSetAttribute(cwf_wgrad_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
     cwf_wgrad_store_kernel<<<(unsigned)(((g.cin + 3) / 4) * ((g.cout + 31) / 32)), 256, smem, st>>>((float*)dw, q.partial, rd);
     LB2_CHECK_LAUNCH("conv_cw_f32 filter-gradient reduction");
   }

@@ -1453,3 +1453,33 @@ def test_float32_calls_run_where_the_device_has_no_room_for_tensor_core_copies(m
         check(got, want, "f32", name)
     with pytest.raises(torch.OutOfMemoryError):          # kernels that always needed their scratch say so, as before
         L.fused_conv_bias_activation("identity", dev(w, "bf16"), dev(x, "bf16"), None, cd)
+
+
+def test_convolutions_of_different_filters_from_several_threads():
+    # one kernel, two amounts of shared memory: each launch may use what its own filter needs, whatever another thread launches
+    import ctypes as C
+    import threading
+    from luxlib_b200 import ops as _ops
+    lib, failures, start = L._cabi.load(), [], threading.Barrier(4)
+
+    def calls(k):
+        x, w = torch.ones(1, 64, 8, 8, device="cuda", dtype=torch.bfloat16).permute(3, 2, 1, 0), \
+            torch.ones(64, 64, k, k, device="cuda", dtype=torch.bfloat16).permute(3, 2, 1, 0)
+        d = _ops._conv_desc(w, x, L.ConvDims.make(2, 2, k // 2))
+        y = torch.empty(4 * 4 * 64, device="cuda", dtype=torch.bfloat16)
+        ws = torch.empty(lib.lb2_conv_fwd_workspace_bytes(C.byref(d), 1), dtype=torch.uint8, device="cuda")
+        assert lib.lb2_conv_fwd_leaves_x_copy(C.byref(d), 1) == 1
+        stream = torch.cuda.Stream()
+        args = (y.data_ptr(), None, x.data_ptr(), w.data_ptr(), None, C.byref(d), 1, 0, 0, ws.data_ptr(), ws.numel(), stream.cuda_stream)
+        torch.cuda.synchronize()
+        start.wait()
+        for _ in range(8000):
+            if lib.lb2_conv_fwd(*args) != 0:
+                failures.append((k, lib.lb2_last_error_string()))
+        stream.synchronize()
+    threads = [threading.Thread(target=calls, args=(k,)) for k in (1, 3, 1, 3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
