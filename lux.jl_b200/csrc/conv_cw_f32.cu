@@ -972,6 +972,8 @@ bool conv_cwf_supported(const ConvGeom& g) {
   if (g.stride[0] > 4 || g.stride[1] > 4) return false;               // box extent = positions x stride must stay <= 256
   if (g.k[0] * g.k[1] > kFMaxTaps) return false;
   if (g.k[0] * g.dil[0] > 120 || g.k[1] * g.dil[1] > 120) return false;
+  if (g.pad_lo[0] > 30000 || g.pad_lo[1] > 30000) return false;        // tap offsets are 16 bits wide
+  if ((int64_t)g.in[0] * g.in[1] >= (1 << 30) || (int64_t)g.out[0] * g.out[1] >= (1 << 30)) return false;   // positions of a plane: int
   if (x_numel(g) >= ((int64_t)1 << 40)) return false;
   const CwfGrid t = cwf_grid(g.out[0], g.out[1], g.batch, g.cout);
   if (t.BW * g.stride[0] > 256 || t.BH * g.stride[1] > 256) return false;

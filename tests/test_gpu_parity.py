@@ -1483,3 +1483,15 @@ def test_convolutions_of_different_filters_from_several_threads():
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+def test_f32_conv_with_padding_beyond_16_bits():
+    rng = np.random.default_rng(73)
+    x, w, pad = rng.standard_normal((5, 3, 4, 1)).astype(np.float32), rng.standard_normal((3, 3, 4, 6)).astype(np.float32), (40000, 2, 1, 1)
+    ocd, cd = O.ConvDims.make(2, 1, pad, 1, 1, False), L.ConvDims.make(2, 1, pad)
+    y_ref, pb_ref = O.fused_conv_rrule("identity", w.astype(np.float64), x.astype(np.float64), None, ocd)
+    y, pb = L.rrule_fused_conv("identity", dev(w, "f32"), dev(x, "f32"), None, cd)
+    check(y, y_ref, "f32", "y")
+    delta = rng.standard_normal(y_ref.shape).astype(np.float32)
+    for name, got, want in zip(("dw", "dx"), pb(dev(delta, "f32")), pb_ref(delta.astype(np.float64))):
+        check(got, want, "f32", name)
