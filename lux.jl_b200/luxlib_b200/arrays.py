@@ -24,7 +24,8 @@ def colmajor_strides(shape: Sequence[int]):
 
 def jl_empty(shape: Sequence[int], dtype: torch.dtype, device) -> torch.Tensor:
     """similar(x, T, shape...): uninitialised column-major array."""
-    return torch.empty_strided(tuple(shape), colmajor_strides(shape), dtype=dtype, device=device)
+    shape = tuple(int(d) for d in shape)
+    return torch.empty_strided(shape, colmajor_strides(shape), dtype=dtype, device=device)
 
 
 def jl_zeros(shape, dtype, device) -> torch.Tensor:

@@ -153,6 +153,13 @@ def test_host_mirror_argument_errors_need_no_gpu():
     assert L.is_colmajor(j) and (L.to_numpy(j) == a).all()
 
 
+@pytest.mark.parametrize("shape", [(3.0, 4), (3, 4.0)])
+def test_array_extents_are_whatever_int_takes(shape):
+    import torch
+    t = L.jl_empty(shape, torch.float32, "cpu")
+    assert tuple(t.shape) == (3, 4) and t.stride() == (1, 3)
+
+
 def test_the_library_reads_no_environment_variable():
     # a drop-in library must not change its arithmetic on an inherited environment: every switch is an argument
     import glob
