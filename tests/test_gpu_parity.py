@@ -1495,3 +1495,21 @@ def test_f32_conv_with_padding_beyond_16_bits():
     delta = rng.standard_normal(y_ref.shape).astype(np.float32)
     for name, got, want in zip(("dw", "dx"), pb(dev(delta, "f32")), pb_ref(delta.astype(np.float64))):
         check(got, want, "f32", name)
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("variant", ["plain", "causal", "mask+bias"])
+@pytest.mark.parametrize("dims", [
+    (32, 2, 1, 70, 771, 32, 1),        # rows of eight quads per lane, the last ones partly filled; no multiple of 8 or 4
+    (16, 1, 1, 1024, 1024, 24, 1),     # rows that fill the registers
+    (136, 2, 2, 130, 60, 200, 1),      # more than one column tile of features, with remainders
+])
+def test_attention_tensor_core_path_long_rows_and_wide_features(dt, variant, dims):
+    test_attention_tensor_core_path(dt, variant, dims)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dims", [(20, 2, 1, 33, 47, 12, 2), (4, 1, 1, 129, 9, 36, 1)])
+def test_f32_attention_features_that_are_not_whole_vectors_of_parts(dims, causal):
+    # four floats are the 16-byte rule of Float32; the parts' rows are padded to eight
+    test_attention_tensor_core_path("f32", "causal" if causal else "plain", dims)
