@@ -24,8 +24,11 @@ def colmajor_strides(shape: Sequence[int]):
 
 def jl_empty(shape: Sequence[int], dtype: torch.dtype, device) -> torch.Tensor:
     """similar(x, T, shape...): uninitialised column-major array."""
-    shape = tuple(int(d) for d in shape)
-    return torch.empty_strided(shape, colmajor_strides(shape), dtype=dtype, device=device)
+    try:
+        return torch.empty_strided(tuple(shape), colmajor_strides(shape), dtype=dtype, device=device)
+    except TypeError:                                    # extents that are no integers yet
+        shape = tuple(int(d) for d in shape)
+        return torch.empty_strided(shape, colmajor_strides(shape), dtype=dtype, device=device)
 
 
 def jl_zeros(shape, dtype, device) -> torch.Tensor:
