@@ -6,7 +6,7 @@
 //   logits[l][s] = q . k      dw[l][s] = dx . v        M = queries, N = keys
 //   x[l][e] = w . v           dq[l][d] = dl . k        M = queries, contraction over the keys
 //   dk[s][d] = dl' . q        dv[s][e] = w' . dx       M = keys, contraction over the queries of all heads that share the key
-// The arrays are read in place through 4-D TMA maps (feature, head, token, sample); either index of an operand may be the
+// The arrays are read through TMA maps (feature, head, token, sample; Float32: part), bf16 in place; either index of an operand may be the
 // contiguous one (K-major / MN-major shared-memory descriptors), so nothing is transposed. A causal mask skips the tiles
 // and the k-blocks that are zero.
 // bf16: one accumulator per tile, two in flight. Float32: operands in three bf16 parts (parts.cuh), six products per k-block,
@@ -27,8 +27,8 @@ constexpr int kAtThreads = 384;    // warps 0-2: TMA / MMA / TMEM, warps 4-11: e
 constexpr int kAtBM = 128;
 
 struct AtOperand {
-  int32_t boxes, box_bytes, mn_step, mn_major, head_first, head_div;
-  uint32_t desc_hi, lbo, k_adv;
+  int32_t boxes, box_bytes, mn_step, mn_major, head_first, head_div;   // Float32: a box holds all parts
+  uint32_t desc_hi, lbo, k_adv, part;
 };
 enum { kCausalNone = 0, kCausalTiles = 1, kCausalKeys = 2, kCausalQueries = 3 };
 struct AtParams {
@@ -47,18 +47,18 @@ template <int BN, bool F32> struct AtCfg {
   static constexpr int ROW = F32 ? 64 : 128;                                // bytes of a k-block's row: 32 / 64 elements
   static constexpr int A_BYTES = kAtBM * ROW, B_BYTES = BN * ROW;           // one part
   static constexpr int PARTS = F32 ? 3 : 1;
-  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES) * PARTS;           // F32: [A1 | A2 | A3 | B1 | B2 | B3]
+  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES) * PARTS;           // F32: [A1 | A2 | A3 | B1 | B2 | B3]; MN-major: boxes of all parts
   static constexpr int STAGES = (200 * 1024) / STAGE_BYTES < 6 ? (200 * 1024) / STAGE_BYTES : 6;
   static constexpr int ACC_COLS = F32 ? 2 * BN : BN;                        // F32: [A1*B1 | the small products] of one k-block
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 };
-struct AtMaps { CUtensorMap m[3]; };   // the parts; bf16: the first only
 
-__device__ __forceinline__ void at_load(uint32_t dst, const CUtensorMap* map, const AtOperand& o, int mn, int k, int head, int img,
-                                        uint64_t* bar) {
+template <bool F32>
+__device__ __forceinline__ void at_load(uint32_t dst, const CUtensorMap* map, const AtOperand& o, int mn, int k, int head, int img, uint64_t* bar) {
   const int inner = o.mn_major ? mn : k, outer = o.mn_major ? k : mn;
-  if (o.head_first) tma_load_4d(dst, map, inner, head, outer, img, bar);
-  else tma_load_4d(dst, map, inner, outer, head, img, bar);
+  const int c1 = o.head_first ? head : outer, c2 = o.head_first ? outer : head;
+  if constexpr (F32) tma_load_5d(dst, map, inner, c1, c2, img, 0, bar);
+  else tma_load_4d(dst, map, inner, c1, c2, img, bar);
 }
 
 __device__ __forceinline__ void at_store32(void* p, const uint32_t (&w)[8]) {
@@ -69,7 +69,7 @@ __device__ __forceinline__ void at_store32(void* p, const uint32_t (&w)[8]) {
 
 template <int BN, bool F32>
 __global__ void __launch_bounds__(kAtThreads, 1)
-attn_gemm_kernel(const __grid_constant__ AtMaps tmA, const __grid_constant__ AtMaps tmB, const __grid_constant__ AtParams p) {
+attn_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ AtParams p) {
   using Cfg = AtCfg<BN, F32>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -128,13 +128,10 @@ attn_gemm_kernel(const __grid_constant__ AtMaps tmA, const __grid_constant__ AtM
             mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
             const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + Cfg::A_BYTES * Cfg::PARTS;
             const int k0 = kb * p.bk;
-#pragma unroll
-            for (int part = 0; part < Cfg::PARTS; ++part) {
-              for (int bx = 0; bx < p.a.boxes; ++bx)
-                at_load(sA + part * Cfg::A_BYTES + bx * p.a.box_bytes, &tmA.m[part], p.a, t.m0 + bx * p.a.mn_step, k0, ha, t.img, &full[stage]);
-              for (int bx = 0; bx < p.b.boxes; ++bx)
-                at_load(sB + part * Cfg::B_BYTES + bx * p.b.box_bytes, &tmB.m[part], p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
-            }
+            for (int bx = 0; bx < p.a.boxes; ++bx)
+              at_load<F32>(sA + bx * p.a.box_bytes, &tmA, p.a, t.m0 + bx * p.a.mn_step, k0, ha, t.img, &full[stage]);
+            for (int bx = 0; bx < p.b.boxes; ++bx)
+              at_load<F32>(sB + bx * p.b.box_bytes, &tmB, p.b, t.n0 + bx * p.b.mn_step, k0, hb, t.img, &full[stage]);
           }
           __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -160,7 +157,7 @@ attn_gemm_kernel(const __grid_constant__ AtMaps tmA, const __grid_constant__ AtM
         const uint64_t bd = ((uint64_t)p.b.desc_hi << 32) | (uint64_t)(((sB >> 4) & 0x3FFFu) | p.b.lbo);
         if (elect_one()) {
           if constexpr (F32) {
-            parts_issue(d_tmem, d_tmem + BN, ad, bd, Cfg::A_BYTES >> 4, Cfg::B_BYTES >> 4, p.a.k_adv, p.b.k_adv, p.idesc, true, nullptr);
+            parts_issue(d_tmem, d_tmem + BN, ad, bd, p.a.part, p.b.part, p.a.k_adv, p.b.k_adv, p.idesc, true, nullptr);
           } else {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) umma<false>(d_tmem, ad + ks * p.a.k_adv, bd + ks * p.b.k_adv, p.idesc, (kb | ks) != 0 ? 1u : 0u);
@@ -488,36 +485,36 @@ struct AtArray {
   bool head_first;
 };
 
-bool at_encode(CUtensorMap* map, const void* ptr, const AtArray& t, int64_t batch, bool f32, int box_outer) {
+bool at_encode(CUtensorMap* map, const AtArray& t, int64_t batch, bool f32, int box_outer) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
   const int o = t.head_first ? 2 : 1, h = t.head_first ? 1 : 2;
-  cuuint64_t dims[4], strides[3];
-  cuuint32_t box[4] = {f32 ? 32u : 64u, 1, 1, 1}, estr[4] = {1, 1, 1, 1};
-  dims[0] = (cuuint64_t)t.inner; dims[o] = (cuuint64_t)t.outer; dims[h] = (cuuint64_t)t.heads; dims[3] = (cuuint64_t)batch;
+  cuuint64_t dims[5], strides[4];                     // Float32: the parts are a fifth dimension
+  cuuint32_t box[5] = {f32 ? 32u : 64u, 1, 1, 1, 3}, estr[5] = {1, 1, 1, 1, 1};
+  dims[0] = (cuuint64_t)t.inner; dims[o] = (cuuint64_t)t.outer; dims[h] = (cuuint64_t)t.heads; dims[3] = (cuuint64_t)batch; dims[4] = 3;
   strides[o - 1] = (cuuint64_t)(t.ld * 2); strides[h - 1] = (cuuint64_t)(t.head_stride * 2); strides[2] = (cuuint64_t)(t.batch_stride * 2);
+  strides[3] = (cuuint64_t)(t.part_stride * 2);
   box[o] = (cuuint32_t)box_outer;
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, f32 ? 5 : 4, const_cast<void*>(t.ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              f32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-bool at_operand(AtMaps* maps, const AtArray& t, bool mn_major, int head_div, int64_t batch, bool f32, int tile_mn, AtOperand* o) {
-  const int row = f32 ? 32 : 64, row_bytes = row * 2;   // a k-block's row: its depth, or the elements of the other index in a box
+bool at_operand(CUtensorMap* map, const AtArray& t, bool mn_major, int head_div, int64_t batch, bool f32, int tile_mn, AtOperand* o) {
+  const int row = f32 ? 32 : 64, row_bytes = row * 2, parts = f32 ? 3 : 1;   // a k-block's row: its depth, or the elements of the other index in a box
   o->mn_major = mn_major; o->head_first = t.head_first; o->head_div = head_div;
   if (mn_major) {
-    o->boxes = tile_mn / row; o->box_bytes = row * row_bytes; o->mn_step = row;
+    o->boxes = tile_mn / row; o->box_bytes = row * row_bytes * parts; o->mn_step = row;
     o->lbo = ((uint32_t)(o->box_bytes >> 4) & 0x3FFFu) << 16;
     o->k_adv = (uint32_t)((16 * row_bytes) >> 4);
   } else {
-    o->boxes = 1; o->box_bytes = tile_mn * row_bytes; o->mn_step = 0;
+    o->boxes = 1; o->box_bytes = tile_mn * row_bytes * parts; o->mn_step = 0;
     o->lbo = 1u << 16;
     o->k_adv = 2u;
   }
+  o->part = (uint32_t)((o->box_bytes / parts) >> 4);
   // eight-row swizzle atoms of 128-byte (2) or 64-byte (4) rows
   o->desc_hi = ((uint32_t)((8 * row_bytes) >> 4) & 0x3FFFu) | (1u << 14) | ((f32 ? 4u : 2u) << 29);
-  for (int i = 0; i < (f32 ? 3 : 1); ++i)
-    if (!at_encode(&maps->m[i], static_cast<const uint16_t*>(t.ptr) + i * t.part_stride, t, batch, f32, mn_major ? row : tile_mn)) return false;
-  return true;
+  return at_encode(map, t, batch, f32, mn_major ? row : tile_mn);
 }
 
 struct AtProduct {
@@ -534,7 +531,7 @@ int32_t at_gemm(const AtProduct& g, int64_t batch, int32_t dtype, cudaStream_t s
   const bool f32 = dtype == LB2_F32;
   const int bn = g.N <= 64 ? 64 : 128;
   AtParams p{};
-  AtMaps mA{}, mB{};
+  CUtensorMap mA, mB;
   if (!at_operand(&mA, g.A, g.a_mn, g.a_div, batch, f32, kAtBM, &p.a) || !at_operand(&mB, g.B, g.b_mn, g.b_div, batch, f32, bn, &p.b))
     return fail(LB2_LAUNCH_FAIL, "attention: cuTensorMapEncodeTiled failed");
   p.bk = f32 ? 32 : 64;

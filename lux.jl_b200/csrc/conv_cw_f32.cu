@@ -11,7 +11,7 @@
 // gets there.
 //
 //   layout       x (and dy) are rewritten channel-innermost, three parts (one pass: read 4 bytes, write 6 per element); a tap
-//                shift, the padding and the stride are then start coordinates / box parameters of a 4-D TMA map
+//                shift, the padding and the stride are then start coordinates / box parameters of a TMA map
 //   forward      M = 128 output positions (a w x h x image box), N = 64 / 128 output channels, both operands K-major
 //   data grad.   the same kernel on the copy of dy with the filter transposed; stride s: s*s classes of input positions
 //   filter grad. rows = four (tap, 32-channel chunk) boxes of x, columns = 64 / 128 output channels of dy, contraction over
@@ -162,23 +162,33 @@ __global__ void __launch_bounds__(256) cwf_pack_tile_kernel(uint16_t* __restrict
     cwf_tile[(r * 32 + c) * taps + t] = v;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < 256 * taps; e += 256) {
-    const int c = e & 31, r = (e >> 5) & 7, tap = e >> 8;
+  for (int e = threadIdx.x; e < 128 * taps; e += 256) {   // two channels: 4-byte stores
+    const int c = (e & 15) * 2, r = (e >> 4) & 7, tap = e >> 7;
     const int tw = tap % g.kW, th = tap / g.kW;
     const int kw = g.flip ? tw : g.kW - 1 - tw, kh = g.flip ? th : g.kH - 1 - th;
     const int64_t o = (int64_t)(row0 + r) * g.k_total + (tap * g.chunks + chunk) * 32 + c;
-    const Parts q = split_parts(cwf_tile[(r * 32 + c) * taps + kh * g.kW + kw]);
-    out[o] = q.a; out[o + part_stride] = q.b; out[o + 2 * part_stride] = q.c;
+    const float* v = cwf_tile + (r * 32 + c) * taps + kh * g.kW + kw;
+    const Parts l = split_parts(v[0]), h = split_parts(v[taps]);
+    *reinterpret_cast<uint32_t*>(out + o) = l.a | ((uint32_t)h.a << 16);
+    *reinterpret_cast<uint32_t*>(out + o + part_stride) = l.b | ((uint32_t)h.b << 16);
+    *reinterpret_cast<uint32_t*>(out + o + 2 * part_stride) = l.c | ((uint32_t)h.c << 16);
   }
 }
 
 // ----------------------------------------------------------------------------------------------
 // kernels
 // ----------------------------------------------------------------------------------------------
+// K-major operands: 64-byte swizzle, 8-row atoms of 512 bytes, 32 bytes of K per MMA step
+constexpr uint32_t kDescHi = (uint32_t)((512u >> 4) & 0x3FFFu) | (1u << 14) | (4u << 29);
+constexpr uint32_t kLboK = 1u << 16, kAdvK = 2u;
+// MN-major operands: the same swizzle, atoms of 32 elements x 8 rows; a box is the three parts of 32 elements, 2048 bytes each, 16
+// rows of 64 bytes per MMA step
+constexpr uint32_t kPartMN = 2048u >> 4, kLboMN = ((3u * 2048u) >> 4) << 16, kAdvMN = (16u * 64u) >> 4;
+
 template <int BN> struct CwfCfg {
   static constexpr int A_BYTES = kFBM * 64;                     // 128 rows x 32 bf16, one part
   static constexpr int B_BYTES = BN * 64;
-  static constexpr int STAGE_BYTES = 3 * (A_BYTES + B_BYTES);   // [A1 | A2 | A3 | B1 | B2 | B3]
+  static constexpr int STAGE_BYTES = 3 * (A_BYTES + B_BYTES);   // [A1 | A2 | A3 | B1 | B2 | B3]; MN-major: boxes of all parts
   static constexpr int SLOTS = 512 / BN - 1;                    // TMEM: a ring of BN-column accumulators and one for the small products
   static constexpr int STAGES = (200 * 1024) / STAGE_BYTES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
@@ -195,22 +205,23 @@ template <int SLOTS> struct CwfRing {
   }
 };
 // k-block i of `n` of an item
-template <int BN>
-__device__ __forceinline__ bool cwf_issue_kblock(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_base, uint32_t sA, uint32_t sB, uint32_t desc_hi,
-                                                 uint32_t lbo, uint32_t k_adv, uint32_t idesc, int i, int n, uint64_t* stage_empty,
-                                                 unsigned int* status, unsigned int code) {
+template <int BN, bool MN>
+__device__ __forceinline__ bool cwf_issue_kblock(CwfRing<CwfCfg<BN>::SLOTS>& ring, uint32_t tmem_base, uint32_t sA, uint32_t sB, uint32_t idesc,
+                                                 int i, int n, uint64_t* stage_empty, unsigned int* status, unsigned int code) {
   constexpr int SLOTS = CwfCfg<BN>::SLOTS;
   const bool first = i % kSegment == 0, last = i % kSegment == kSegment - 1 || i == n - 1;   // of its segment
-  const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | lbo, b32 = ((sB >> 4) & 0x3FFFu) | lbo;
-  const uint64_t top = (uint64_t)desc_hi << 32;
+  constexpr uint32_t LBO = MN ? kLboMN : kLboK, K_ADV = MN ? kAdvMN : kAdvK;
+  constexpr uint32_t A_PART = MN ? kPartMN : CwfCfg<BN>::A_BYTES >> 4, B_PART = MN ? kPartMN : CwfCfg<BN>::B_BYTES >> 4;
+  const uint32_t a32 = ((sA >> 4) & 0x3FFFu) | LBO, b32 = ((sB >> 4) & 0x3FFFu) | LBO;
+  constexpr uint64_t top = (uint64_t)kDescHi << 32;
   if (!mbar_wait_uniform(&ring.empty[ring.slot], ring.phase ^ 1u, status, code)) return false;
   if (first) {
     if (!mbar_wait_uniform(&ring.empty[SLOTS], ring.small_phase ^ 1u, status, code)) return false;
   }
   tc_fence_after();
   if (elect_one()) {
-    parts_issue(tmem_base + ring.slot * BN, tmem_base + SLOTS * BN, top | (uint64_t)a32, top | (uint64_t)b32, CwfCfg<BN>::A_BYTES >> 4,
-                CwfCfg<BN>::B_BYTES >> 4, k_adv, k_adv, idesc, first, &ring.full[ring.slot]);
+    parts_issue(tmem_base + ring.slot * BN, tmem_base + SLOTS * BN, top | (uint64_t)a32, top | (uint64_t)b32, A_PART, B_PART, K_ADV, K_ADV, idesc,
+                first, &ring.full[ring.slot]);
     umma_commit(stage_empty);
     if (last) umma_commit(&ring.full[SLOTS]);
   }
@@ -265,13 +276,6 @@ __device__ __forceinline__ bool cwf_accumulate(CwfRing<CwfCfg<BN>::SLOTS>& ring,
   }
   return true;
 }
-
-// K-major operands: 64-byte swizzle, 8-row atoms of 512 bytes, 32 bytes of K per MMA step
-constexpr uint32_t kDescHi = (uint32_t)((512u >> 4) & 0x3FFFu) | (1u << 14) | (4u << 29);
-constexpr uint32_t kLboK = 1u << 16, kAdvK = 2u;
-// MN-major operands: the same swizzle, atoms of 32 elements x 8 rows, the next 32 elements one 2048-byte box further, 16 rows of
-// 64 bytes per MMA step
-constexpr uint32_t kLboMN = ((2048u >> 4) & 0x3FFFu) << 16, kAdvMN = (16u * 64u) >> 4;
 
 // A channel-innermost array of parts and what of it exists; the taps a folded copy (fold = cin) holds beside one another
 struct CwfSource {
@@ -373,9 +377,7 @@ __device__ __noinline__ void cwf_redo_fwd(const CwfFwdParams& p, int q, int half
 
 template <int BN, int ACT>
 __global__ void __launch_bounds__(kFThreads, 1)
-conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
-                    const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmW3,
-                    const __grid_constant__ CwfFwdParams p) {
+conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CwfFwdParams p) {
   using Cfg = CwfCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -407,8 +409,7 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmX3);
-    tma_prefetch_desc(&tmW1); tma_prefetch_desc(&tmW2); tma_prefetch_desc(&tmW3);
+    tma_prefetch_desc(&tmX); tma_prefetch_desc(&tmW);
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
@@ -423,12 +424,9 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
           mbar_expect_tx(&full[stage], tx);
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
           const int w = w0 + p.tap_dw[tap], h = h0 + p.tap_dh[tap], k0 = (p.tap_index[tap] * p.chunks + ch) * 32;
-          tma_load_4d(sA, &tmX1, ch * 32, w, h, i0, &full[stage]);
-          tma_load_2d(sB, &tmW1, k0, n0, &full[stage]);
-          tma_load_4d(sA + Cfg::A_BYTES, &tmX2, ch * 32, w, h, i0, &full[stage]);
-          tma_load_2d(sB + Cfg::B_BYTES, &tmW2, k0, n0, &full[stage]);
-          tma_load_4d(sA + 2 * Cfg::A_BYTES, &tmX3, ch * 32, w, h, i0, &full[stage]);
-          tma_load_2d(sB + 2 * Cfg::B_BYTES, &tmW3, k0, n0, &full[stage]);
+          tma_load_3d(sB, &tmW, k0, n0, 0, &full[stage]);
+#pragma unroll
+          for (int part = 0; part < 3; ++part) tma_load_5d(sA + part * Cfg::A_BYTES, &tmX, ch * 32, w, h, i0, part, &full[stage]);
         }
         __syncwarp();
         if (++ch == p.chunks) { ch = 0; ++tap; }
@@ -445,7 +443,7 @@ conv_cwf_fwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_const
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x4000u)) { ok = false; break; }
         const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
-        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHi, kLboK, kAdvK, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x2000u)) { ok = false; break; }
+        if (!cwf_issue_kblock<BN, false>(ring, tmem_base, sA, sB, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x2000u)) { ok = false; break; }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
@@ -566,9 +564,7 @@ __device__ __noinline__ void cwf_redo_wgrad(const CwfWgParams& p, int q, int hal
 
 template <int BN>
 __global__ void __launch_bounds__(kFThreads, 1)
-conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
-                      const __grid_constant__ CUtensorMap tmG1, const __grid_constant__ CUtensorMap tmG2, const __grid_constant__ CUtensorMap tmG3,
-                      const __grid_constant__ CwfWgParams p) {
+conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CwfWgParams p) {
   using Cfg = CwfCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -600,8 +596,7 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 
   // item -> (m tile fastest, n tile, split)
   if (warp == 0) {
-    tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmX3);
-    tma_prefetch_desc(&tmG1); tma_prefetch_desc(&tmG2); tma_prefetch_desc(&tmG3);
+    tma_prefetch_desc(&tmX); tma_prefetch_desc(&tmG);
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
@@ -623,19 +618,10 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
           mbar_expect_tx(&full[stage], (uint32_t)Cfg::STAGE_BYTES);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int w = a0 * p.sw + dw[j], h = b0 * p.sh + dh[j];
-            tma_load_4d(sA + j * 2048, &tmX1, c0[j], w, h, i0, &full[stage]);
-            tma_load_4d(sA + Cfg::A_BYTES + j * 2048, &tmX2, c0[j], w, h, i0, &full[stage]);
-            tma_load_4d(sA + 2 * Cfg::A_BYTES + j * 2048, &tmX3, c0[j], w, h, i0, &full[stage]);
-          }
+          for (int j = 0; j < 4; ++j) tma_load_5d(sA + j * 6144, &tmX, c0[j], a0 * p.sw + dw[j], b0 * p.sh + dh[j], i0, 0, &full[stage]);
 #pragma unroll
-          for (int j = 0; j < BN / 32; ++j) {            // channels past the last and positions past the ends are zero-filled
-            const int c = nt * BN + j * 32;
-            tma_load_4d(sB + j * 2048, &tmG1, c, a0, b0, i0, &full[stage]);
-            tma_load_4d(sB + Cfg::B_BYTES + j * 2048, &tmG2, c, a0, b0, i0, &full[stage]);
-            tma_load_4d(sB + 2 * Cfg::B_BYTES + j * 2048, &tmG3, c, a0, b0, i0, &full[stage]);
-          }
+          for (int j = 0; j < BN / 32; ++j)              // channels past the last and positions past the ends are zero-filled
+            tma_load_5d(sB + j * 6144, &tmG, nt * BN + j * 32, a0, b0, i0, 0, &full[stage]);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -650,7 +636,7 @@ conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         if (!mbar_wait_uniform(&full[stage], phase, p.status, 0x80000u)) { ok = false; break; }
         const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES, sB = sA + 3 * Cfg::A_BYTES;
-        if (!cwf_issue_kblock<BN>(ring, tmem_base, sA, sB, kDescHi, kLboMN, kAdvMN, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x40000u)) { ok = false; break; }
+        if (!cwf_issue_kblock<BN, true>(ring, tmem_base, sA, sB, p.idesc, kb - kb_lo, kb_hi - kb_lo, &empty[stage], p.status, 0x40000u)) { ok = false; break; }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
@@ -741,26 +727,26 @@ __global__ void __launch_bounds__(256) cwf_wgrad_store_kernel(float* __restrict_
 // ----------------------------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------------------------
-// 4-D map over one part of a channel-innermost array (Cp, W, H, N): box = 32 channels x bw x bh x bi positions
-bool cwf_map(CUtensorMap* map, const void* ptr, int Cp, int W, int H, int N, int bw, int bh, int bi, int sw, int sh) {
+// 5-D map over a channel-innermost array (Cp, W, H, N, part): box = 32 channels x bw x bh x bi positions of one part or all three
+bool cwf_map(CUtensorMap* map, const CwfSource& s, int N, int bw, int bh, int bi, int sw, int sh, int parts) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
-  cuuint64_t dims[4] = {(cuuint64_t)Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-  cuuint64_t strides[3] = {(cuuint64_t)Cp * 2, (cuuint64_t)Cp * W * 2, (cuuint64_t)Cp * W * H * 2};
-  cuuint32_t box[4] = {32, (cuuint32_t)(bw * sw), (cuuint32_t)(bh * sh), (cuuint32_t)bi};
-  cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t dims[5] = {(cuuint64_t)s.Cp, (cuuint64_t)s.W, (cuuint64_t)s.H, (cuuint64_t)N, 3};
+  cuuint64_t strides[4] = {(cuuint64_t)s.Cp * 2, (cuuint64_t)s.Cp * s.W * 2, (cuuint64_t)s.Cp * s.W * s.H * 2, (cuuint64_t)s.part_stride * 2};
+  cuuint32_t box[5] = {32, (cuuint32_t)(bw * sw), (cuuint32_t)(bh * sh), (cuuint32_t)bi, (cuuint32_t)parts};
+  cuuint32_t estr[5] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<uint16_t*>(s.ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-bool cwf_map_2d(CUtensorMap* map, const void* ptr, int64_t d0, int64_t d1, int box1) {
+bool cwf_map_filter(CUtensorMap* map, const void* ptr, int64_t cols, int64_t rows, size_t packed_one, int box_rows) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)d0, (cuuint64_t)d1};
-  cuuint64_t strides[1] = {(cuuint64_t)d0 * 2};
-  cuuint32_t box[2] = {32, (cuuint32_t)box1};
-  cuuint32_t estr[2] = {1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 3};
+  cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)packed_one};
+  cuuint32_t box[3] = {32, (cuuint32_t)box_rows, 3};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -899,12 +885,9 @@ int32_t cwf_run(const CwfOut& o, const CwfSource& src, int NI, int chunks, const
     p.tap_dw[i] = (int16_t)taps[i].dw; p.tap_dh[i] = (int16_t)taps[i].dh; p.tap_index[i] = (int16_t)taps[i].index;
   }
   p.src = src; p.wp = wp; p.wp_part_stride = (int64_t)(packed_one / 2); p.wp_cols = wp_cols;
-  CUtensorMap mX[3], mW[3];
-  bool encoded = true;
-  for (int i = 0; i < 3; ++i)
-    encoded = encoded && cwf_map(&mX[i], src.ptr + i * src.part_stride, src.Cp, src.W, src.H, NI, t.BW, t.BH, t.BI, sw, sh) &&
-              cwf_map_2d(&mW[i], wp + i * p.wp_part_stride, wp_cols, wp_rows, bn);
-  if (!encoded)
+  CUtensorMap mX, mW;
+  // the parts of a position box that is no multiple of 8 positions would start inside a swizzle atom: one load each
+  if (!cwf_map(&mX, src, NI, t.BW, t.BH, t.BI, sw, sh, 1) || !cwf_map_filter(&mW, wp, wp_cols, wp_rows, packed_one, bn))
     return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cuTensorMapEncodeTiled failed");
   const int64_t items = t.tiles() * o.splits;
   LB2_REQUIRE(items <= 0x7FFFFFFF, LB2_BAD_SHAPE, "conv_cw_f32: too many tiles");
@@ -912,7 +895,7 @@ int32_t cwf_run(const CwfOut& o, const CwfSource& src, int NI, int chunks, const
   auto launch = [&](auto kernel, int smem) -> int32_t {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    kernel<<<grid, kFThreads, smem, st>>>(mX[0], mX[1], mX[2], mW[0], mW[1], mW[2], p);
+    kernel<<<grid, kFThreads, smem, st>>>(mX, mW, p);
     LB2_CHECK_LAUNCH("conv_cw_f32");
     return LB2_OK;
   };
@@ -1050,13 +1033,8 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
       q.tap_dw[t] = (int16_t)(fold ? 0 : (t % g.k[0]) * g.dil[0] - g.pad_lo[0]);
       q.tap_dh[t] = (int16_t)((fold ? t : t / g.k[0]) * g.dil[1] - g.pad_lo[1]);
     }
-    CUtensorMap mX[3], mG[3];
-    bool encoded = true;
-    for (int i = 0; i < 3; ++i)
-      encoded = encoded &&
-                cwf_map(&mX[i], xcopy.ptr + i * xcopy.part_stride, xc.Cp, xc.W, xc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, q.sw, q.sh) &&
-                cwf_map(&mG[i], gcopy.ptr + i * gcopy.part_stride, yc.Cp, yc.W, yc.H, g.batch, pl.KW_, pl.KH_, pl.KI_, 1, 1);
-    if (!encoded)
+    CUtensorMap mX, mG;
+    if (!cwf_map(&mX, xcopy, g.batch, pl.KW_, pl.KH_, pl.KI_, q.sw, q.sh, 3) || !cwf_map(&mG, gcopy, g.batch, pl.KW_, pl.KH_, pl.KI_, 1, 1, 3))
       return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cuTensorMapEncodeTiled failed");
     const int64_t items = (int64_t)pl.m_tiles * pl.tiles_n * pl.splits;
     LB2_REQUIRE(items <= 0x7FFFFFFF, LB2_BAD_SHAPE, "conv_cw_f32: too many tiles");
@@ -1064,7 +1042,7 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
     auto launch = [&](auto kernel, int smem) -> int32_t {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_cw_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      kernel<<<grid, kFThreads, smem, st>>>(mX[0], mX[1], mX[2], mG[0], mG[1], mG[2], q);
+      kernel<<<grid, kFThreads, smem, st>>>(mX, mG, q);
       LB2_CHECK_LAUNCH("conv_cw_f32 filter gradient");
       return LB2_OK;
     };
