@@ -57,14 +57,14 @@ int32_t conv_cwf_bwd(void* dw, void* dx, const void* x, const void* gy, const vo
 // the whole planes are 4 % faster.
 inline void conv_position_box(int OW, int OH, int NI, int most, int64_t per_box, int64_t wave, int* BW, int* BH, int* BI) {
   int64_t best = 0;
-  for (int k = 1; k <= OW; ++k) {
-    const int bw = (OW + k - 1) / k;
-    if (bw > most) continue;
+  for (int bw = OW < most ? OW : most; bw >= 1; --bw) {   // widths, not counts of pieces: at most `most` of them for rows of any length
+    const int pieces = (OW + bw - 1) / bw;
+    if ((OW + pieces - 1) / pieces != bw) continue;       // no width of equal pieces
     if (best != 0 && bw < 8) break;
     const int rows = most / bw;
     for (int bh = rows < OH ? rows : OH; bh >= 1; --bh) {
       const int bi = rows / bh < NI ? rows / bh : NI;
-      const int64_t n = (int64_t)((OW + bw - 1) / bw) * ((OH + bh - 1) / bh) * ((NI + bi - 1) / bi);
+      const int64_t n = (int64_t)pieces * ((OH + bh - 1) / bh) * ((NI + bi - 1) / bi);
       const int64_t waves = (n * per_box + wave - 1) / wave;
       if (best == 0 || waves < best) { best = waves; *BW = bw; *BH = bh; *BI = bi; }
     }

@@ -1513,3 +1513,21 @@ def test_attention_tensor_core_path_long_rows_and_wide_features(dt, variant, dim
 def test_f32_attention_features_that_are_not_whole_vectors_of_parts(dims, causal):
     # four floats are the 16-byte rule of Float32; the parts' rows are padded to eight
     test_attention_tensor_core_path("f32", "causal" if causal else "plain", dims)
+
+
+def test_conv_queries_of_long_rows_take_no_time_that_grows_with_them():
+    # the tile search runs in every call: 4000 samples a row or four million, it looks at the same number of widths. A million
+    # of them took 10 ms and more
+    import ctypes as C
+    import time
+    from luxlib_b200 import ops as _ops
+    lib = L._cabi.load()
+    for dt in (0, 1):
+        d = _ops._conv_desc_from((3, 1, 16, 16), (4_000_000, 1), 16, 1, L.ConvDims.make(2, 1, (1, 1, 0, 0)))
+        assert lib.lb2_conv_fwd_workspace_bytes(C.byref(d), dt) > 0
+        took = []
+        for _ in range(5):
+            t = time.perf_counter()
+            lib.lb2_conv_fwd_workspace_bytes(C.byref(d), dt)
+            took.append(time.perf_counter() - t)
+        assert min(took) < 2e-3, took
