@@ -70,7 +70,7 @@ typedef enum {
                                 once the problem occupies an eighth of the SM pairs (default: only for two MN-major operands) */
 #define LB2_FLAG_NO_CTA_PAIR 8u /* tensor-core GEMM: never take the CTA-pair kernel */
 /* lb2_conv_bwd only: the `x` argument is not x but the start of the workspace that lb2_conv_fwd was given for the same
- * descriptor and x (and that the caller has kept untouched since): the general tensor-core path leaves its
+ * descriptor and x (and that the caller has kept untouched since): the general bf16 tensor-core path leaves its
  * channel-innermost copy of x there and the filter gradient then reads that copy instead of making it again. Valid
  * only where lb2_conv_fwd_leaves_x_copy() returns 1; refused (LB2_BAD_ARG) elsewhere. */
 #define LB2_FLAG_X_COPY_GIVEN 16u
@@ -173,7 +173,7 @@ typedef struct {
 LB2_API int32_t lb2_conv_output_size(const lb2_conv_desc* d, int32_t* out);
 /* y = act.(conv(x, w) .+ b); optional pre-activation store. Replaces conv_bias_act / conv!
  * for CUDADevice (lib/LuxLib/src/impl/conv.jl:42-60,157-166).
- * Float32 geometries that only the general tensor-core path takes (any stride, odd planes) are still served without its
+ * Float32 geometries that only the general tensor-core path takes (strided ones, odd planes) are still served without its
  * workspace, by the CUDA-core kernels: lb2_conv_fwd with less than this size (none at all, or one that is not 256-byte
  * aligned), lb2_conv_fwd_sums with room for lb2_channel_sums alone, lb2_conv_bwd with room for its activation pass
  * (dy's size where act is not the identity, rounded up to 1024, and lb2_bias_act_bwd_workspace_bytes, likewise). */

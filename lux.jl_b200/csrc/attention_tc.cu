@@ -6,14 +6,15 @@
 //   logits[l][s] = q . k      dw[l][s] = dx . v        M = queries, N = keys
 //   x[l][e] = w . v           dq[l][d] = dl . k        M = queries, contraction over the keys
 //   dk[s][d] = dl' . q        dv[s][e] = w' . dx       M = keys, contraction over the queries of all heads that share the key
-// The arrays are read through TMA maps (feature, head, token, sample; Float32: part), bf16 in place; either index of an operand may be the
-// contiguous one (K-major / MN-major shared-memory descriptors), so nothing is transposed. A causal mask skips the tiles
-// and the k-blocks that are zero.
+// The arrays are read through TMA maps (feature, head, token, sample; Float32: part), bf16 in place; either index of an
+// operand may be the contiguous one (K-major / MN-major shared-memory descriptors), so nothing is transposed. A causal mask
+// skips the tiles and the k-blocks that are zero.
 // bf16: one accumulator per tile, two in flight. Float32: operands in three bf16 parts (parts.cuh), six products per k-block,
 // k-blocks added in fp32 registers.
 //
-// Measured, forward + pullback through the operator, 8 heads x 8 samples, 512 x 512, 64 features, causal, bf16: 130 us (one
-// tensor-core GEMM launch per head, sample and product before: 4.1 ms); Float32 4 x 4, 771 x 771: 300 us (3.07 ms).
+// Measured, forward + pullback through the operator, 8 heads x 8 samples, 512 x 512, 64 features, causal, bf16: 122 us (one
+// tensor-core GEMM launch per head, sample and product before: 4.1 ms); Float32 4 x 4, 771 x 771: 285 us (3.07 ms;
+// 270 us with two tf32 parts, whose results were further from 64 bits than fp32 sums).
 // What bounds it: a contraction over a head's 64 features is one k-block, so the products move the S x L weights and little
 // else; the passes over the weights (in L2 for the usual sizes) are the cost.
 #include "common.cuh"

@@ -1,5 +1,6 @@
 // General tensor-core convolution for sm_100a (bf16 storage, fp32 accumulation in TMEM): implicit GEMM for any
-// 2-D ConvDims with groups == 1 — any stride, padding, dilation, kernel size and channel counts — which is what
+// 2-D ConvDims with groups == 1 — any padding, dilation, kernel size and channel counts, strides up to 4 whose position
+// boxes fit a TMA box (positions x stride at most 256: conv_cw_supported) — which is what
 // the layers of a ResNet need beyond the stride-1 64-channel case served by conv_tc.cu (strided 3x3 and 1x1
 // convolutions, the 7x7 stem, 128/256/512-channel stages whose filters do not fit in shared memory).
 //
@@ -873,8 +874,6 @@ int32_t cw_copy_x(void* xc, const void* x, const ConvGeom& g, const CwCopy& c, c
 
 template <int BN>
 int32_t cw_launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, CwFwdParams& p, int32_t act, cudaStream_t st, int* grid_out) {
-  // A filter of one column tile that fits 96 KB stays in shared memory: its tiles would otherwise be fetched again for every
-  // 128 positions (the folded stem's four: a third of what the kernel takes in, 506 us per 256 images of 224 x 224).
   constexpr int A_BYTES = kCwBM * 128, B_BYTES = BN * 128;
   // A filter of one column tile that fits 96 KB stays in shared memory; in the ring its tiles are fetched again for every 128
   // positions, a third of what a folded stem's kernel takes in (256 images of 224 x 224: 506 us, resident 449 us). Above

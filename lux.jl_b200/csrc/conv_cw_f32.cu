@@ -19,11 +19,11 @@
 // A problem with too few tiles for the SMs is split along the contraction as well: fp32 partials in the layout of the
 // output and one elementwise pass that adds them in order (deterministic) and applies bias and activation.
 //
-// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 84 / 155 us (89 /
-// 95 TFLOP/s); 3x3 512 -> 512 on 7x7: 95 / 171 us. Two tf32 parts took 90 / 154 and 99 / 168 us and were less accurate than
-// fp32 sums in the filter gradient. The CUDA-core kernels of conv_direct.cu, which took these geometries before, made a
-// ResNet-18 training step at batch 32 last 333 ms; it now takes 6.2 ms. Error against 64 bits (2-norm, normal data): 5e-8 to
-// 1.6e-7, the CUDA-core kernels' 6e-8 to 1.1e-6.
+// Measured (forward / both gradients, fp32 TFLOP/s of the convolution): 3x3 256 -> 256 on 14x14, batch 32: 81 / 158 us (92 /
+// 94 TFLOP/s); 3x3 512 -> 512 on 7x7: 91 / 172 us. Two tf32 parts took 90 / 154 and 99 / 168 us, the gradients with the forward
+// call's copy of x, and were less accurate than fp32 sums in the filter gradient. The CUDA-core kernels of conv_direct.cu, which
+// took these geometries before, made a ResNet-18 training step at batch 32 last 333 ms; it now takes 6.3 ms. Error against 64
+// bits (2-norm, normal data): 5e-8 to 1.6e-7, the CUDA-core kernels' 6e-8 to 1.1e-6.
 // What bounds it: a 128 x 128 x 32 k-block is 768 tensor-pipe cycles (12 MMAs) against about 1150 cycles of shared-memory
 // traffic (48 KB written by TMA, 96 KB read by the MMAs at 128 B/cycle).
 #include "conv.cuh"

@@ -1,5 +1,6 @@
 // Direct (CUDA-core) convolution: the catch-all for every ConvDims the implicit-GEMM tensor-core
-// paths do not take (1-D / 3-D, groups, strides above 4, very large kernels). Forward, data
+// paths do not take (1-D / 3-D, groups, strides above 4 or too large for a TMA box, very large
+// kernels and paddings, Float32 calls without workspace). Forward, data
 // gradient and filter gradient, each with fp32 accumulation in a fixed order (deterministic).
 // Layout: x (in..., Cin, N), w (k..., Cin/groups, Cout), y (out..., Cout, N), column-major;
 // true convolution (kernel flipped) unless flipkernel is set — NNlib semantics as used by

@@ -8,7 +8,8 @@
 // bf16: operands through TMA as in gemm_tc.cu. Float32: sixteen worker warps read the operands with plain loads (any leading
 // dimension, any alignment), split them into tf32 hi / lo on the way and write both as K-major swizzled tiles, so the
 // separate split passes and their copies are not needed; the same warps take the partial products out of TMEM (two k-steps of
-// hi*hi per accumulator, the small products in one accumulator) and add them in fp32 registers, as conv_cw_f32.cu does.
+// hi*hi per accumulator, the small products in one accumulator) and add them in fp32 registers. Error against 64 bits 0.9e-7 to
+// 1.6e-7 (gemm_tc_f32acc_kernel, which took these products before: 0.9e-7 to 3.2e-7); an infinite operand gives NaN, as there.
 //
 // Measured against the kernels of gemm_tc.cu (which the larger shapes keep), forward with bias and activation: bf16 4096 x 8 x
 // 4096 14.5 us (28.8; 33.5 MB of weights at 2.3 TB/s), 256 x 8 x 8192 12.5 us (49); Float32 4096 x 8 x 4096 47 us (169),

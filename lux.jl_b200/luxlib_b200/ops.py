@@ -501,7 +501,7 @@ def _conv_fwd(act, weight, x, b, cd, want_preact, flags=0, want_ws=False):
     pre = jl_empty(info.yshape, X.dtype, X.device) if want_preact else None
     ws = _with_scratch(info.fwd_bytes, 0, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
         ptr(y), ptr(pre), ptr(X), ptr(Wt), ptr(b), C.byref(d), dt, act_code(act), flags, wsp, wsn, current_stream(X.device)))
-    # the general tensor-core path leaves its channel-innermost copy of x at the start of the workspace; a pullback
+    # the general bf16 path leaves its channel-innermost copy of x at the start of the workspace; a pullback
     # that keeps the workspace alive hands it back instead of having the copy made again
     keep = ws if (want_ws and ws is not None and not (flags & _cabi.FLAG_FORCE_SIMT) and X.data_ptr() % 16 == 0 and
                   info.leaves_x_copy) else None
