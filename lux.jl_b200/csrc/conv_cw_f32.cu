@@ -331,7 +331,9 @@ struct CwfFwdParams {
 };
 
 // A warp's elements that came out as NaN once more, as the sum of their terms (positions outside the arrays are none). The lanes
-// share an element's channels. A NaN among the terms stays NaN and ends the sum early.
+// share an element's channels. A NaN among the terms stays NaN and ends the sum early; a NaN among a position's inputs settles
+// all its channels, and where everything is NaN the first term of each element settles it, a lane per element. (3x3 256 -> 256 on
+// 14x14, batch 32, one NaN in x: 0.28 ms; all of x: 0.47 ms; the CUDA-core kernel takes 4.5 ms whatever the values.)
 template <int BN>
 __device__ __noinline__ void cwf_redo_fwd(const CwfFwdParams& p, int q, int half) {
   constexpr int COLS = BN / 2;
@@ -344,32 +346,59 @@ __device__ __noinline__ void cwf_redo_fwd(const CwfFwdParams& p, int q, int half
     const int kb_lo = z * p.kb_per_split, kb_hi = min(p.num_kb, kb_lo + p.kb_per_split);
     const int a = tw * p.BW + iw, b = th * p.BH + ih, img = ti * p.BI + ii;
     const bool live = ii < p.BI && a < p.OW && b < p.OH && img < p.NI;
+    uint32_t seen = 0, nan_rows = 0;                     // lanes whose position's inputs were looked through / hold a NaN
     for (int j = 0; j < COLS; ++j) {
       const int col = tn * BN + half * COLS + j;
       if (col >= p.n_out) break;
       const int64_t out = p.out_index(a, b, img, col);
       float* const dst = p.splits > 1 ? p.partial + z * p.split_stride + out : p.y + out;
+      const uint16_t* const wrow = p.wp + (int64_t)col * p.wp_cols;
       const float old = live ? *dst : 0.f;
-      for (uint32_t todo = __ballot_sync(0xffffffffu, old != old); todo != 0; todo &= todo - 1) {
-        const int who = __ffs(todo) - 1;
+      const uint32_t todo = __ballot_sync(0xffffffffu, old != old);
+      if (todo == 0) continue;
+      bool settled = false;
+      if (old != old) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
+          const int tap = kb / p.chunks, c = (kb - tap * p.chunks) * 32, w = a * p.sw + p.tap_dw[tap], h = b * p.sh + p.tap_dh[tap];
+          if (!p.src.has(c, w, h)) continue;
+          const float v = p.src.at(c, w, h, img) * join_parts(wrow + p.tap_index[tap] * p.chunks * 32 + c, p.wp_part_stride);
+          settled = v != v;
+          break;
+        }
+      }
+      float result = old;
+      for (uint32_t rest = todo & ~__ballot_sync(0xffffffffu, settled); rest != 0; rest &= rest - 1) {
+        const int who = __ffs(rest) - 1;
         const int wa = __shfl_sync(0xffffffffu, a, who) * p.sw, wb = __shfl_sync(0xffffffffu, b, who) * p.sh, wi = __shfl_sync(0xffffffffu, img, who);
-        float sum = 0.f;
-        for (int kb = kb_lo; kb < kb_hi && !__any_sync(0xffffffffu, sum != sum); ++kb) {
-          const int tap = kb / p.chunks, c = (kb - tap * p.chunks) * 32 + lane;
-          const int w = wa + p.tap_dw[tap], h = wb + p.tap_dh[tap];
-          if (p.src.has(c, w, h))
-            sum = fmaf(p.src.at(c, w, h, wi),
-                       join_parts(p.wp + (int64_t)col * p.wp_cols + p.tap_index[tap] * p.chunks * 32 + c, p.wp_part_stride), sum);
-        }
-        sum = warp_sum(sum);
-        if (lane == who) {
-          if (p.splits == 1) {
-            if (p.bias != nullptr) sum += __ldg(p.bias + col);
-            if (p.preact != nullptr) p.preact[out] = sum;
-            sum = act_apply_any<-1, false>(p.act, sum);
+        auto walk = [&](auto term) {                     // term(x, filter offset) until it says stop
+          for (int kb = kb_lo; kb < kb_hi; ++kb) {
+            const int tap = kb / p.chunks, c = (kb - tap * p.chunks) * 32 + lane, w = wa + p.tap_dw[tap], h = wb + p.tap_dh[tap];
+            bool stop = false;
+            if (p.src.has(c, w, h)) stop = term(p.src.at(c, w, h, wi), p.tap_index[tap] * p.chunks * 32 + c);
+            if (__any_sync(0xffffffffu, stop)) return true;
           }
-          *dst = sum;
+          return false;
+        };
+        if ((seen >> who & 1u) == 0) {
+          seen |= 1u << who;
+          if (walk([](float x, int) { return x != x; })) nan_rows |= 1u << who;
         }
+        if ((nan_rows >> who & 1u) != 0) continue;
+        float sum = 0.f;
+        walk([&](float x, int at) {
+          sum = fmaf(x, join_parts(wrow + at, p.wp_part_stride), sum);
+          return sum != sum;
+        });
+        sum = warp_sum(sum);
+        if (lane == who) result = sum;
+      }
+      if (old != old) {
+        if (p.splits == 1) {
+          if (p.bias != nullptr) result += __ldg(p.bias + col);
+          if (p.preact != nullptr) p.preact[out] = result;
+          result = act_apply_any<-1, false>(p.act, result);
+        }
+        *dst = result;
       }
     }
   }
@@ -543,25 +572,35 @@ __device__ __noinline__ void cwf_redo_wgrad(const CwfWgParams& p, int q, int hal
     if (pr >= p.n_pairs) continue;
     const int tap = pr / p.chunks, c = (pr - tap * p.chunks) * 32 + lane;
     float* const row = p.partial + ((int64_t)z * p.m_tiles * 128 + mt * 128 + q * 32 + lane) * p.n_pad;
-    for (int j = 0; j < COLS; ++j) {
-      const int col = nt * BN + half * COLS + j;
-      if (col >= p.cout) break;
-      const bool todo = row[col] != row[col];
-      if (!__any_sync(0xffffffffu, todo)) continue;
-      float sum = 0.f;
-      for (int kb = kb_lo; kb < kb_hi && __any_sync(0xffffffffu, todo && sum == sum); ++kb) {
+    // body(x, position of dy) for every position of the item that is a term of the lane's elements, until done()
+    auto walk = [&](auto body, auto done) {
+      for (int kb = kb_lo; kb < kb_hi && !done(); ++kb) {
         const int a0 = (kb % p.kbw) * p.KW_, b0 = (kb / p.kbw) % p.kbh * p.KH_, i0 = kb / (p.kbw * p.kbh) * p.KI_;
         for (int t = 0; t < 32; ++t) {
           const int a = a0 + t % p.KW_, b = b0 + t / p.KW_ % p.KH_, img = i0 + t / (p.KW_ * p.KH_);
           const int w = a * p.sw + p.tap_dw[tap], h = b * p.sh + p.tap_dh[tap];
-          if (a < p.g.W && b < p.g.H && img < p.NI && p.x.has(c, w, h)) sum = fmaf(p.x.at(c, w, h, img), p.g.at(col, a, b, img), sum);
+          if (a < p.g.W && b < p.g.H && img < p.NI && p.x.has(c, w, h)) body(p.x.at(c, w, h, img), a, b, img);
         }
       }
+    };
+    bool seen = false, x_nan = false;                    // a NaN among the channel's inputs settles all its filter elements
+    for (int j = 0; j < COLS; ++j) {
+      const int col = nt * BN + half * COLS + j;
+      if (col >= p.cout) break;
+      const bool nan = row[col] != row[col];
+      if (!__any_sync(0xffffffffu, nan)) continue;
+      if (!seen) {
+        seen = true;
+        walk([&](float x, int, int, int) { x_nan |= x != x; }, [&]() { return __all_sync(0xffffffffu, x_nan) != 0; });
+      }
+      const bool todo = nan && !x_nan;
+      float sum = 0.f;
+      walk([&](float x, int a, int b, int img) { sum = fmaf(x, p.g.at(col, a, b, img), sum); },
+           [&]() { return !__any_sync(0xffffffffu, todo && sum == sum); });
       if (todo) row[col] = sum;
     }
   }
 }
-
 template <int BN>
 __global__ void __launch_bounds__(kFThreads, 1)
 conv_cwf_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CwfWgParams p) {

@@ -1,6 +1,7 @@
 // A Float32 operand of the tensor-core kernels as three bf16 parts.
 //
-// x = x1 + x2 + x3, 8 significant bits each; the sum is exact down to 2^-110. Of the nine products of two operands the six
+// x = x1 + x2 + x3, 8 significant bits each; the sum is exact for |x| >= 2^-110 (8e-34; below, the third part falls under the
+// smallest bf16 and x is off by up to 2^-134). Of the nine products of two operands the six
 // x1*y1, x1*y2, x2*y1, x1*y3, x3*y1, x2*y2 are formed; the three left out are below 2^-25 of x*y. (Two tf32 parts leave a bit
 // of x over in every fourth value, 4e-8 of it, and their 22-bit products lose bits where the tensor core aligns them; an 8-bit
 // product loses next to nothing. Six bf16 products take the tensor core as long as three tf32 products.)

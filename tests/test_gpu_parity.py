@@ -1322,6 +1322,12 @@ def test_f32_conv_passes_infinities_and_nan_on_as_fp32_sums_do(case, planted, ac
     assert L._cabi.load().lb2_poll_device_status(None) == 0
 
 
+@pytest.mark.parametrize("planted", ["x", "w", "dy"])
+def test_f32_conv_passes_infinities_and_nan_on_over_several_tiles(planted):
+    # several tiles per CTA, two column tiles; no relu, whose cotangent comes or goes whole for a pre-activation within rounding of 0
+    test_f32_conv_passes_infinities_and_nan_on_as_fp32_sums_do(((61, 59), (3, 3), 8, 130, 1, 1, 12), planted, "identity")
+
+
 @pytest.mark.parametrize("planted", range(4))      # q, k, v, dx
 @pytest.mark.parametrize("dims", [(64, 2, 2, 40, 60, 2), (20, 2, 1, 130, 130, 1)])
 def test_f32_attention_passes_infinities_on_as_fp32_sums_do(dims, planted):
