@@ -13,6 +13,10 @@ namespace lb2 {
 // ---- host-side error plumbing ---------------------------------------------------------------
 void set_error(const char* fmt, ...);  // thread-local message, defined in api.cu
 int32_t fail(int32_t status, const char* fmt, ...);
+// Shared memory a block may have on this device. cudaFuncAttributeMaxDynamicSharedMemorySize is a limit of the kernel, not of a
+// launch: kernels whose launches need different amounts set it to all there is (less their static shared memory), or a thread
+// could lower it between another thread's setting and launch.
+constexpr int kMaxBlockSmem = 227 * 1024;
 int sm_count();                        // cached per device
 unsigned int* device_status_word();    // per-device status word written by bounded waits
 

@@ -1055,7 +1055,7 @@ static int32_t run_conv_gemm(void* out, void* preact, const void* bias, int32_t 
     if (per_n2 < 1) per_n2 = 1;
     const int grid2 = per_n2 * q.tiles_n;
     auto launch2 = [&](auto kernel) -> int32_t {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem - 256);   // 256: the bias tile
       if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_tc: cannot reserve %d bytes of shared memory: %s", smem2, cudaGetErrorString(e));
       kernel<<<grid2, kConv2Threads, smem2, st>>>(mX2, mW2, mY2, mP2, q);
       LB2_CHECK_LAUNCH("conv_tc_fwd2");
@@ -1225,7 +1225,7 @@ int32_t conv_tc_wgrad(void* dw, const void* x, const void* gy, const ConvGeom& g
     const int items3 = w3.chunks * w3.splits;
     const int grid3 = items3 < sm_count() ? items3 : sm_count();
     auto launch3 = [&](auto kernel) -> int32_t {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem3);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
       if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_tc: cannot reserve %d bytes of shared memory: %s", smem3, cudaGetErrorString(e));
       kernel<<<grid3, kConvThreads, smem3, st>>>(mX3, mXh3, mG3, q, w3.stages, w3.stage_bytes, w3.tmem_cols);
       LB2_CHECK_LAUNCH("conv_tc_wgrad_rows");
@@ -1283,7 +1283,7 @@ int32_t conv_tc_wgrad(void* dw, const void* x, const void* gy, const ConvGeom& g
     const int items2 = w2.groups * w2.splits;
     const int grid2 = items2 < sm_count() ? items2 : sm_count();
     auto launch2 = [&](auto kernel) -> int32_t {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
       if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "conv_tc: cannot reserve %d bytes of shared memory: %s", smem2, cudaGetErrorString(e));
       kernel<<<grid2, kConvThreads, smem2, st>>>(mX2, mX0, mG2, q);
       LB2_CHECK_LAUNCH("conv_tc_wgrad2");

@@ -663,7 +663,7 @@ static int32_t gn_bwd_launch(T* dx, T* dg, T* db, const T* dy, const T* x, const
     const int resident = nchunks <= 4 ? 1 : 0;
     const int stages = resident ? (int)nchunks : 6;
     const int smem = kGnHeaderBytes + (int)aux + stages * 2 * (int)kGnChunkBytes;
-    cudaError_t e = cudaFuncSetAttribute(gn_bwd_stream_kernel<T, ACT, AFFINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gn_bwd_stream_kernel<T, ACT, AFFINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
     LB2_REQUIRE(e == cudaSuccess, LB2_LAUNCH_FAIL, "groupnorm: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const int per_sm = smem <= 112 * 1024 ? 2 : 1;
     grid = (int)(rows < (int64_t)sms * per_sm ? rows : (int64_t)sms * per_sm);

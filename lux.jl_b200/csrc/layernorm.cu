@@ -703,7 +703,7 @@ template <typename T> static LnPlan ln_plan(int64_t D, int64_t R, bool aligned, 
 
 template <typename K>
 static int32_t ring_smem_attr(K kernel, int smem) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
   if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "layernorm: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
   return LB2_OK;
 }

@@ -600,7 +600,7 @@ int32_t lb2_pool_fwd(void* y, const void* x, const lb2_pool_desc* d, int32_t kin
       const int st2 = same && g.stride[0] <= 2 ? g.stride[0] : 0;
       auto launch = [&](auto kernel) -> int32_t {
         if (sp.bytes > 48 * 1024) {
-          cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes);
+          cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
           if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "pool2d_fwd: cannot reserve %d bytes of shared memory: %s", sp.bytes, cudaGetErrorString(e));
         }
         kernel<<<plane_grid(g.planes), 256, sp.bytes, st>>>((decltype(pool_arg_y(kernel)))y, (decltype(pool_arg_x(kernel)))x, g, sp.lw_out, vec);
@@ -680,7 +680,7 @@ int32_t lb2_pool_bwd(void* dx, const void* dy, const void* y, const void* x, con
       const int st2 = same && g.stride[0] <= 2 ? g.stride[0] : 0;
       auto reserve = [&](auto kernel) -> int32_t {
         if (sp.bytes > 48 * 1024) {
-          cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes);
+          cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
           if (e != cudaSuccess) return fail(LB2_LAUNCH_FAIL, "pool2d_bwd: cannot reserve %d bytes of shared memory: %s", sp.bytes, cudaGetErrorString(e));
         }
         return LB2_OK;

@@ -1537,3 +1537,46 @@ def test_conv_queries_of_long_rows_take_no_time_that_grows_with_them():
             lib.lb2_conv_fwd_workspace_bytes(C.byref(d), dt)
             took.append(time.perf_counter() - t)
         assert min(took) < 2e-3, took
+
+
+@pytest.mark.parametrize("op", ["layernorm", "maxpool", "conv"])
+def test_calls_of_different_extents_from_several_threads(op):
+    # as above, for the other kernels whose shared memory follows the extents
+    import ctypes as C
+    import threading
+    from luxlib_b200 import ops as _ops
+    lib, failures, start = L._cabi.load(), [], threading.Barrier(4)
+
+    def calls(big):
+        stream = torch.cuda.Stream()
+        buf = lambda n, dt=torch.float32: torch.ones(n, device="cuda", dtype=dt)
+        if op == "layernorm":
+            D = 8192 if big else 7168
+            x, y, mean, inv = buf(4 * D), buf(4 * D), buf(4), buf(4)
+            call = lambda: lib.lb2_layernorm_fwd(y.data_ptr(), mean.data_ptr(), inv.data_ptr(), x.data_ptr(), None, None, D, 4, 1e-5, 0, 0,
+                                                 stream.cuda_stream)
+        elif op == "maxpool":
+            n = 160 if big else 120
+            x, y = buf(2 * n * n).reshape(1, 2, n, n).permute(3, 2, 1, 0), buf(2 * n * n)
+            d = _ops._pool_desc(x, L.PoolDims.make((3, 3), 2, 1))
+            call = lambda: lib.lb2_pool_fwd(y.data_ptr(), x.data_ptr(), C.byref(d), 0, 0, stream.cuda_stream)
+        else:
+            ci = 128 if big else 64
+            x, w = buf(ci * 256, torch.bfloat16).reshape(1, ci, 16, 16).permute(3, 2, 1, 0), \
+                buf(64 * ci * 9, torch.bfloat16).reshape(64, ci, 3, 3).permute(3, 2, 1, 0)
+            d = _ops._conv_desc(w, x, L.ConvDims.make(2, 1, 1))
+            y, ws = buf(64 * 256, torch.bfloat16), buf(max(lib.lb2_conv_fwd_workspace_bytes(C.byref(d), 1), 1), torch.uint8)
+            call = lambda: lib.lb2_conv_fwd(y.data_ptr(), None, x.data_ptr(), w.data_ptr(), None, C.byref(d), 1, 0, 0, ws.data_ptr(), ws.numel(),
+                                            stream.cuda_stream)
+        torch.cuda.synchronize()
+        start.wait()
+        for _ in range(8000):
+            if call() != 0:
+                failures.append((big, lib.lb2_last_error_string()))
+        stream.synchronize()
+    threads = [threading.Thread(target=calls, args=(big,)) for big in (False, True, False, True)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:3]
