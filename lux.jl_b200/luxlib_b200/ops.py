@@ -93,15 +93,16 @@ def _ws(nbytes: int, device):
     return w, ptr(w), int(nbytes) if w is not None else 0
 
 
-def _with_scratch(nbytes: int, least: int, device, call):
-    """`call(pointer, bytes)` with `nbytes` of scratch, which is returned. Where the device has no room for that, with `least`:
-    what the CUDA-core kernels need, which then serve the call if the library lets them."""
+def _with_scratch(nbytes: int, least, device, call):
+    """`call(pointer, bytes)` with `nbytes` of scratch, which is returned. Where the device has no room for that, with `least()`
+    (None: nothing): what the CUDA-core kernels need, which then serve the call if the library lets them."""
     try:
         w, wsp, wsn = _ws(nbytes, device)
     except torch.OutOfMemoryError:
-        if least >= nbytes:
+        n = least() if least is not None else 0
+        if n >= nbytes:
             raise
-        w, wsp, wsn = _ws(least, device)
+        w, wsp, wsn = _ws(n, device)
         status = call(wsp, wsn)
         if status == _cabi.WORKSPACE_TOO_SMALL:
             raise
@@ -499,7 +500,7 @@ def _conv_fwd(act, weight, x, b, cd, want_preact, flags=0, want_ws=False):
     info = _conv_query(Wt, X, cd, dt)
     y = jl_empty(info.yshape, X.dtype, X.device)
     pre = jl_empty(info.yshape, X.dtype, X.device) if want_preact else None
-    ws = _with_scratch(info.fwd_bytes, 0, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
+    ws = _with_scratch(info.fwd_bytes, None, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
         ptr(y), ptr(pre), ptr(X), ptr(Wt), ptr(b), C.byref(d), dt, act_code(act), flags, wsp, wsn, current_stream(X.device)))
     # the general bf16 path leaves its channel-innermost copy of x at the start of the workspace; a pullback
     # that keeps the workspace alive hands it back instead of having the copy made again
@@ -528,7 +529,7 @@ def rrule_fused_conv(act: str, weight, x, b, cdims: ConvDims, *, flags: int = 0)
         dx = jl_empty(X.shape, X.dtype, X.device) if need_dx else None
         db = jl_empty((d.cout,), X.dtype, X.device) if bb is not None else None
         xarg, xflag = (ptr(xcopy), _cabi.FLAG_X_COPY_GIVEN) if xcopy is not None else (ptr(X), 0)
-        _with_scratch(info.bwd_bytes(code), info.least_bwd_bytes(code), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+        _with_scratch(info.bwd_bytes(code), lambda: info.least_bwd_bytes(code), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
             ptr(dw), ptr(dx), ptr(db), ptr(dl), None if keep_pre else ptr(y), ptr(pre), xarg, ptr(Wt), C.byref(d), dt, code, flags | xflag,
             wsp, wsn, current_stream(X.device)))
         return dw, dx, db
@@ -570,17 +571,17 @@ def rrule_conv_transpose(act: str, weight, x, b, cdims: ConvDims, outpad=0, *, f
         raise DimensionMismatch("length(bias) must equal the number of output channels")
     ident = act_code("identity")
     u = jl_empty(usz + (cu, X.shape[-1]), X.dtype, X.device)
-    _with_scratch(info.bwd_bytes(ident), info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+    _with_scratch(info.bwd_bytes(ident), lambda: info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
         None, ptr(u), None, ptr(X), None, None, None, ptr(Wt), C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
     y, pb_act = rrule_bias_activation(act, u, b)
 
     def pullback(delta):
         g, db = pb_act(delta)
         dx = jl_empty(X.shape, X.dtype, X.device)
-        _with_scratch(info.fwd_bytes, 0, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
+        _with_scratch(info.fwd_bytes, None, X.device, lambda wsp, wsn: lib.lb2_conv_fwd(
             ptr(dx), None, ptr(g), ptr(Wt), None, C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
         dw = jl_empty(Wt.shape, X.dtype, X.device)
-        _with_scratch(info.bwd_bytes(ident), info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
+        _with_scratch(info.bwd_bytes(ident), lambda: info.least_bwd_bytes(ident), X.device, lambda wsp, wsn: lib.lb2_conv_bwd(
             ptr(dw), None, None, ptr(X), None, None, ptr(g), None, C.byref(d), dt, ident, flags, wsp, wsn, current_stream(X.device)))
         return dw, dx, db
 
